@@ -1,5 +1,6 @@
 // Empirical scores on the GPU: the pose-selection / affinity score kernel (one warp per
 // pose) and the FP64 generalised-Born / surface-area term, with their C ABI.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -365,100 +366,305 @@ __global__ void __launch_bounds__(kScoreWarps * kWarp) empirical_score_kernel(co
     }
 }
 
-// GB/SA (gbsa_total_energy::calculate, scorer.cpp:798-866) in FP64.
+// GB/SA (gbsa_total_energy::calculate, scorer.cpp:798-866) in FP64, for a batch of poses of
+// one ligand: the complex, the ligand alone and the receptor alone. What bounds it is the
+// FP64 pipe (about 1.7 operations a clock and SM), so the work is what is cut:
+//   - the receptor-receptor Born sums are formed once per receptor conformation (once per
+//     call without rotors) and serve the receptor alone and every complex;
+//   - the pair energies run over i < j (the sum over ordered pairs is symmetric);
+//   - r, 1/r and f, 1/f come from one rsqrt each.
+// Every sum has a fixed order, so the energies repeat bit for bit. The work is split over
+// warps (Born sums) and 64 x 64 tiles of atom pairs (energies), which fills the chip at one
+// pose: 8 poses of 42 atoms in a pocket of 1,866 take 2.3 ms of kernel time; with one thread
+// per atom and three systems per pose they took 186 ms.
+constexpr double kGbOffset = 0.09;
+constexpr int kGbTile = 64;
+constexpr int kGbThreads = 128;
+constexpr int kGbLanes = 8;       // lanes that share a receptor atom's sum over the ligand
+constexpr int kGbPoses = 512;     // poses per batch of launches (bounds the workspace)
+
 struct GbArgs {
-    int n;
-    const double* x;       // [n][3]
-    const double* q;
-    const double* radius;
-    const double* screen;
-    double* born;          // [n] out
-    double* partial;       // [n] out: per-atom egb row + esa
+    int n_lig, n_rec, n_poses, n_conf;  // n_conf: receptor conformations, 1 or n_poses
+    const double4* rec;      // [n_conf][n_rec] position, charge
+    const double4* lig;      // [n_poses][n_lig]
+    const double4* rec_p;    // [n_rec] radius, rho = radius - offset, rho * screen
+    const double4* lig_p;    // [n_lig]
+    double* sum_rr;          // [n_conf][n_rec] receptor-receptor Born sums
+    double* ib_rec;          // [n_conf][n_rec] inverse Born radii, receptor alone
+    double* ib_lig;          // [n_poses][n_lig] ligand alone
+    double* ib_com;          // [n_poses][n_lig + n_rec] complex
+    double* partial;         // [systems][n_tiles]
+    int n_tiles;             // of the complex
+    double* energy;          // [systems]: n_poses complexes, n_conf receptors, n_poses ligands
 };
 
-__global__ void gb_born_kernel(const GbArgs a) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= a.n) return;
-    const double offset = 0.09, alpha = 1.0, beta = 0.8, gamma = 4.85;
-    const double orj = a.radius[j] - offset;
-    const double xj = a.x[3 * j], yj = a.x[3 * j + 1], zj = a.x[3 * j + 2];
+// One pair term of atom j's Born sum (scorer.cpp:806-821).
+__device__ __forceinline__ double gb_born_term(double4 xi, double sr, double4 xj, double rho) {
+    const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double ri = rsqrt(r2);
+    const double r = r2 > 0.0 ? r2 * ri : 0.0;
+    const double U = r + sr;
+    if (U < rho) return 0.0;
+    const double L = fmax(rho, fabs(r - sr));
+    const double Ui = 1.0 / U, Li = 1.0 / L;
+    const double D = 0.25 * (r - sr * sr * ri) * (Ui * Ui - Li * Li);
+    return 0.5 * (D + (Li - Ui + 0.5 * log(L * Ui + 1e-20) * ri));
+}
+
+__device__ __forceinline__ double gb_inverse_born(double sum, double4 p) {
+    const double psi = sum * p.y;
+    const double t = tanh(psi - 0.8 * psi * psi + 4.85 * psi * psi * psi);
+    return 1.0 / p.y - t / p.x;
+}
+
+template <int kLanes>
+__device__ __forceinline__ double gb_lane_sum(double v) {
+#pragma unroll
+    for (int off = kLanes / 2; off > 0; off >>= 1) v += __shfl_xor_sync(kFull, v, off);
+    return v;
+}
+
+// Receptor alone: one warp per atom, the lanes over the other atoms.
+__global__ void __launch_bounds__(kGbThreads) gb_receptor_kernel(const __grid_constant__ GbArgs a) {
+    const int lane = threadIdx.x & (kWarp - 1);
+    const int j = blockIdx.x * (kGbThreads / kWarp) + threadIdx.x / kWarp;
+    if (j >= a.n_rec) return;
+    const double4* x = a.rec + static_cast<size_t>(blockIdx.y) * a.n_rec;
+    const double4 xj = x[j], pj = a.rec_p[j];
     double sum = 0.0;
-    for (int i = 0; i < a.n; ++i) {
-        if (i == j) continue;
-        const double sr = (a.radius[i] - offset) * a.screen[i];
-        const double dx = a.x[3 * i] - xj, dy = a.x[3 * i + 1] - yj, dz = a.x[3 * i + 2] - zj;
-        const double r12 = sqrt(dx * dx + dy * dy + dz * dz);
-        const double U = r12 + sr;
-        if (U < orj) continue;
-        const double r12i = 1.0 / r12;
-        double D = fabs(r12 - sr);
-        const double L = orj > D ? orj : D;
-        const double Ui = 1.0 / U, Li = 1.0 / L;
-        D = 0.25 * (r12 - sr * sr * r12i) * (Ui * Ui - Li * Li);
-        D += (Li - Ui + 0.5 * log(L * Ui + 1e-20) * r12i);
-        sum += 0.5 * D;
+    for (int i = lane; i < a.n_rec; i += kWarp)
+        if (i != j) sum += gb_born_term(x[i], a.rec_p[i].z, xj, pj.y);
+    sum = gb_lane_sum<kWarp>(sum);
+    if (lane == 0) {
+        const size_t o = static_cast<size_t>(blockIdx.y) * a.n_rec + j;
+        a.sum_rr[o] = sum;
+        a.ib_rec[o] = gb_inverse_born(sum, pj);
     }
-    const double psi = sum * orj;
-    const double t = tanh(alpha * psi - beta * psi * psi + gamma * psi * psi * psi);
-    a.born[j] = 1.0 / (1.0 / orj - t / a.radius[j]);
 }
 
-__global__ void gb_energy_kernel(const GbArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const double kC = 332.0637141491396, solute = 1.0, solvent = 78.5;
-    const double kappa = 0.09293963686178248, probe = 1.4, surface = 0.0678584012906;
-    const double xi = a.x[3 * i], yi = a.x[3 * i + 1], zi = a.x[3 * i + 2];
-    double egb = 0.0;
-    for (int j = 0; j < a.n; ++j) {
-        double f;
-        if (i == j) {
-            f = a.born[i];
-        } else {
-            const double dx = xi - a.x[3 * j], dy = yi - a.x[3 * j + 1], dz = zi - a.x[3 * j + 2];
-            const double r2 = dx * dx + dy * dy + dz * dz;
-            const double bp = a.born[i] * a.born[j];
-            f = sqrt(r2 + bp * exp(-0.25 * r2 / bp) + 1e-20);
+// Complex and ligand alone: a warp per ligand atom (lanes over the receptor, then the
+// ligand), then kGbLanes lanes per receptor atom (over the ligand, added to its receptor sum).
+__global__ void __launch_bounds__(kGbThreads) gb_complex_kernel(const __grid_constant__ GbArgs a) {
+    const int lane = threadIdx.x & (kWarp - 1);
+    const int task = blockIdx.x * (kGbThreads / kWarp) + threadIdx.x / kWarp;
+    const int p = blockIdx.y, c = a.n_conf > 1 ? p : 0;
+    const double4* xl = a.lig + static_cast<size_t>(p) * a.n_lig;
+    const double4* xr = a.rec + static_cast<size_t>(c) * a.n_rec;
+    double* ib = a.ib_com + static_cast<size_t>(p) * (a.n_lig + a.n_rec);
+    if (task < a.n_lig) {
+        const double4 xj = xl[task], pj = a.lig_p[task];
+        double own = 0.0, rec = 0.0;
+        for (int i = lane; i < a.n_lig; i += kWarp)
+            if (i != task) own += gb_born_term(xl[i], a.lig_p[i].z, xj, pj.y);
+        for (int i = lane; i < a.n_rec; i += kWarp) rec += gb_born_term(xr[i], a.rec_p[i].z, xj, pj.y);
+        own = gb_lane_sum<kWarp>(own);
+        rec = gb_lane_sum<kWarp>(rec);
+        if (lane == 0) {
+            a.ib_lig[static_cast<size_t>(p) * a.n_lig + task] = gb_inverse_born(own, pj);
+            ib[task] = gb_inverse_born(own + rec, pj);
         }
-        const double pref = 0.5 * kC * (1.0 / solute - exp(-kappa * f) / solvent);
-        egb -= a.q[i] * a.q[j] / f * pref;
+        return;
     }
-    const double rr = a.radius[i] + probe;
-    a.partial[i] = egb + rr * rr * pow(a.radius[i] / a.born[i], 6.0) * surface;
+    const int j = (task - a.n_lig) * (kWarp / kGbLanes) + lane / kGbLanes;
+    const int jc = min(j, a.n_rec - 1);  // every lane of a warp that has an atom meets the shuffles
+    if (jc < 0) return;
+    const double4 xj = xr[jc], pj = a.rec_p[jc];
+    double sum = 0.0;
+    for (int i = lane % kGbLanes; i < a.n_lig; i += kGbLanes) sum += gb_born_term(xl[i], a.lig_p[i].z, xj, pj.y);
+    sum = gb_lane_sum<kGbLanes>(sum);
+    if (lane % kGbLanes == 0 && j < a.n_rec)
+        ib[a.n_lig + j] = gb_inverse_born(a.sum_rr[static_cast<size_t>(c) * a.n_rec + j] + sum, pj);
 }
 
-static int gbsa_system(pxd_context* ctx, int n, const std::vector<double>& x, const std::vector<double>& q,
-                       const std::vector<double>& radius, const std::vector<double>& screen, double* out) {
-    if (n == 0) {
-        *out = 0.0;
-        return PXD_OK;
+// A system of the batch: its atoms and their inverse Born radii.
+struct GbSystem {
+    const double4 *lig, *rec;
+    const double* ib;
+    int n_lig, n;
+    __device__ __forceinline__ double4 atom(int i) const { return i < n_lig ? lig[i] : rec[i - n_lig]; }
+};
+
+__device__ __forceinline__ GbSystem gb_system(const GbArgs& a, int s) {
+    if (s < a.n_poses)
+        return {a.lig + static_cast<size_t>(s) * a.n_lig, a.rec + (a.n_conf > 1 ? static_cast<size_t>(s) * a.n_rec : 0),
+                a.ib_com + static_cast<size_t>(s) * (a.n_lig + a.n_rec), a.n_lig, a.n_lig + a.n_rec};
+    s -= a.n_poses;
+    if (s < a.n_conf)
+        return {nullptr, a.rec + static_cast<size_t>(s) * a.n_rec, a.ib_rec + static_cast<size_t>(s) * a.n_rec, 0, a.n_rec};
+    s -= a.n_conf;
+    return {a.lig + static_cast<size_t>(s) * a.n_lig, nullptr, a.ib_lig + static_cast<size_t>(s) * a.n_lig, a.n_lig, a.n_lig};
+}
+
+constexpr double kGbKappa = 0.09293963686178248, kGbSolvent = 78.5, kGbProbe = 1.4, kGbSurface = 0.0678584012906;
+constexpr double kGbCoulomb = 332.0637141491396;
+
+__device__ __forceinline__ double gb_prefactor(double f) {
+    return 0.5 * kGbCoulomb * (1.0 - exp(-kGbKappa * f) / kGbSolvent);
+}
+
+// Pair energies of one 64 x 64 tile (rows bi <= columns bj of the triangle i < j).
+__global__ void __launch_bounds__(kGbThreads) gb_pair_kernel(const __grid_constant__ GbArgs a) {
+    __shared__ double4 s_x[kGbTile];
+    __shared__ double s_ib[kGbTile], s_b[kGbTile];
+    __shared__ double s_sum[kGbThreads / kWarp];
+    const GbSystem y = gb_system(a, blockIdx.y);
+    const int nb = (y.n + kGbTile - 1) / kGbTile;
+    int bi = 0, t = blockIdx.x;
+    if (t >= nb * (nb + 1) / 2) return;
+    while (t >= nb - bi) t -= nb - bi++;
+    const int i0 = bi * kGbTile, j = (bi + t) * kGbTile + (threadIdx.x & (kGbTile - 1));
+    const int ni = min(kGbTile, y.n - i0);
+    for (int u = threadIdx.x; u < ni; u += kGbThreads) {
+        s_x[u] = y.atom(i0 + u);
+        s_ib[u] = y.ib[i0 + u];
+        s_b[u] = 1.0 / s_ib[u];
     }
+    __syncthreads();
+    double e = 0.0;
+    if (j < y.n) {
+        const double4 xj = y.atom(j);
+        const double ibj = y.ib[j], bj = 1.0 / ibj;
+        const int last = min(ni, j - i0);  // i < j
+        for (int u = threadIdx.x / kGbTile; u < last; u += kGbThreads / kGbTile) {
+            const double4 xi = s_x[u];
+            const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            const double s = r2 + s_b[u] * bj * exp(-0.25 * r2 * (s_ib[u] * ibj)) + 1e-20;
+            const double fi = rsqrt(s);
+            e += xi.w * fi * gb_prefactor(s * fi);
+        }
+        e *= xj.w;
+    }
+    e = gb_lane_sum<kWarp>(e);
+    if ((threadIdx.x & (kWarp - 1)) == 0) s_sum[threadIdx.x / kWarp] = e;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double v = 0.0;
+        for (int w = 0; w < kGbThreads / kWarp; ++w) v += s_sum[w];
+        a.partial[static_cast<size_t>(blockIdx.y) * a.n_tiles + blockIdx.x] = -2.0 * v;
+    }
+}
+
+// A system's total: its tiles' pair energies, and per atom the self energy and the surface term.
+__global__ void __launch_bounds__(kGbThreads) gb_total_kernel(const __grid_constant__ GbArgs a) {
+    __shared__ double s_sum[kGbThreads / kWarp];
+    const GbSystem y = gb_system(a, blockIdx.x);
+    const int nb = (y.n + kGbTile - 1) / kGbTile;
+    double e = 0.0;
+    for (int t = threadIdx.x; t < nb * (nb + 1) / 2; t += kGbThreads)
+        e += a.partial[static_cast<size_t>(blockIdx.x) * a.n_tiles + t];
+    for (int i = threadIdx.x; i < y.n; i += kGbThreads) {
+        const double q = y.atom(i).w, ib = y.ib[i];
+        const double radius = i < y.n_lig ? a.lig_p[i].x : a.rec_p[i - y.n_lig].x;
+        const double rr = radius + kGbProbe, x2 = radius * ib * (radius * ib);
+        e += rr * rr * (x2 * x2 * x2) * kGbSurface - q * q * ib * gb_prefactor(1.0 / ib);
+    }
+    e = gb_lane_sum<kWarp>(e);
+    if ((threadIdx.x & (kWarp - 1)) == 0) s_sum[threadIdx.x / kWarp] = e;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double v = 0.0;
+        for (int w = 0; w < kGbThreads / kWarp; ++w) v += s_sum[w];
+        a.energy[blockIdx.x] = v;
+    }
+}
+
+static std::vector<double4> gb_properties4(const std::vector<double>& radius, const std::vector<double>& screen) {
+    std::vector<double4> v;
+    for (size_t i = 0; i < radius.size(); ++i) {
+        const double rho = radius[i] - kGbOffset;
+        v.push_back(make_double4(radius[i], rho, rho * screen[i], 0.0));
+    }
+    return v;
+}
+
+// Receptor coordinates for torsions t in FP64 (torsional_receptor::apply_parameters).
+static std::vector<double> receptor_coords(pxd_context* ctx, const double* t) {
+    std::vector<double> x = ctx->rec_xyz;
+    for (int r = 0; r < ctx->rec.n_rotors; ++r) {
+        const double* k = &ctx->rotor_axis[3 * r];
+        const double* o = &ctx->rotor_origin[3 * r];
+        const double st = std::sin(t[r]), ct = std::cos(t[r]), omc = 1 - ct;
+        const double m[9] = {ct + k[0] * k[0] * omc,        k[0] * k[1] * omc - k[2] * st,
+                             k[1] * st + k[0] * k[2] * omc, k[2] * st + k[0] * k[1] * omc,
+                             ct + k[1] * k[1] * omc,        k[1] * k[2] * omc - k[0] * st,
+                             k[0] * k[2] * omc - k[1] * st, k[0] * st + k[1] * k[2] * omc,
+                             ct + k[2] * k[2] * omc};
+        for (int u = ctx->rotor_mov_off[r]; u < ctx->rotor_mov_off[r + 1]; ++u) {
+            double* p = &x[3 * static_cast<size_t>(ctx->mov_atoms[u])];
+            const double v[3] = {p[0] - o[0], p[1] - o[1], p[2] - o[2]};
+            for (int d = 0; d < 3; ++d) p[d] = m[3 * d] * v[0] + m[3 * d + 1] * v[1] + m[3 * d + 2] * v[2] + o[d];
+        }
+    }
+    return x;
+}
+
+// GB/SA energies of n poses of one ligand (lig_xyz [n][N][3], rec_tors [n][R]):
+// complex, ligand and receptor energies of pose k in parts[3 k .. 3 k + 2].
+static int gbsa_batch(pxd_context* ctx, const LigandEntry& e, int n, const double* lig_xyz, const double* rec_tors,
+                      double* parts) {
+    const int nl = e.n_atoms, nr = ctx->n_rec, R = ctx->rec.n_rotors;
+    const int nc = R > 0 ? n : 1;
+    std::vector<double4> rec, lig;
+    for (int c = 0; c < nc; ++c) {
+        const std::vector<double> x = receptor_coords(ctx, R > 0 ? rec_tors + static_cast<size_t>(c) * R : nullptr);
+        for (int i = 0; i < nr; ++i) rec.push_back(make_double4(x[3 * i], x[3 * i + 1], x[3 * i + 2], ctx->rec_charge[i]));
+    }
+    for (int p = 0; p < n; ++p)
+        for (int i = 0; i < nl; ++i) {
+            const double* x = lig_xyz + 3 * (static_cast<size_t>(p) * nl + i);
+            lig.push_back(make_double4(x[0], x[1], x[2], e.charge[i]));
+        }
+    Pack pk;
+    const size_t o_rec = pk.put(rec), o_lig = pk.put(lig);
+    const size_t o_rp = pk.put(gb_properties4(ctx->rec_gb_radius, ctx->rec_gb_screen));
+    const size_t o_lp = pk.put(gb_properties4(e.gb_radius, e.gb_screen));
+    const int nb = (nl + nr + kGbTile - 1) / kGbTile, systems = 2 * n + nc;
+    GbArgs a{};
+    a.n_lig = nl;
+    a.n_rec = nr;
+    a.n_poses = n;
+    a.n_conf = nc;
+    a.n_tiles = nb * (nb + 1) / 2;
+    const size_t in_bytes = (pk.bytes.size() + 15) / 16 * 16;
+    const size_t rec_n = static_cast<size_t>(nc) * nr, lig_n = static_cast<size_t>(n) * nl;
+    const size_t doubles = 2 * rec_n + lig_n + lig_n + static_cast<size_t>(n) * nr +
+                           static_cast<size_t>(systems) * a.n_tiles + systems;
     void* mem = nullptr;
-    const size_t bytes = sizeof(double) * (3 * n + 5 * static_cast<size_t>(n));
-    int rc = cuda_check(ctx, cudaMallocAsync(&mem, bytes, ctx->stream), "gbsa buffers");
+    int rc = cuda_check(ctx, cudaMallocAsync(&mem, in_bytes + sizeof(double) * doubles, ctx->stream), "gbsa buffers");
     if (rc) return rc;
-    double* d = static_cast<double*>(mem);
-    GbArgs a{n, d, d + 3 * n, d + 4 * n, d + 5 * n, d + 6 * n, d + 7 * n};
-    queue_copy(ctx, &rc, d, x.data(), sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream, "gbsa coordinates");
-    queue_copy(ctx, &rc, d + 3 * n, q.data(), sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream, "gbsa charges");
-    queue_copy(ctx, &rc, d + 4 * n, radius.data(), sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream,
-               "gbsa radii");
-    queue_copy(ctx, &rc, d + 5 * n, screen.data(), sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream,
-               "gbsa screening");
-    const int threads = 128, blocks = (n + threads - 1) / threads;
+    a.rec = at<double4>(mem, o_rec);
+    a.lig = at<double4>(mem, o_lig);
+    a.rec_p = at<double4>(mem, o_rp);
+    a.lig_p = at<double4>(mem, o_lp);
+    a.sum_rr = reinterpret_cast<double*>(static_cast<char*>(mem) + in_bytes);
+    a.ib_rec = a.sum_rr + rec_n;
+    a.ib_lig = a.ib_rec + rec_n;
+    a.ib_com = a.ib_lig + lig_n;
+    a.partial = a.ib_com + lig_n + static_cast<size_t>(n) * nr;
+    a.energy = a.partial + static_cast<size_t>(systems) * a.n_tiles;
+    queue_copy(ctx, &rc, mem, pk.bytes.data(), pk.bytes.size(), cudaMemcpyHostToDevice, ctx->stream, "gbsa inputs");
     if (!rc) {
-        gb_born_kernel<<<blocks, threads, 0, ctx->stream>>>(a);
-        gb_energy_kernel<<<blocks, threads, 0, ctx->stream>>>(a);
+        constexpr int warps = kGbThreads / kWarp;
+        if (nr > 0) gb_receptor_kernel<<<dim3((nr + warps - 1) / warps, nc), kGbThreads, 0, ctx->stream>>>(a);
+        constexpr int per = kWarp / kGbLanes;
+        const int tasks = nl + (nr + per - 1) / per;
+        gb_complex_kernel<<<dim3((tasks + warps - 1) / warps, n), kGbThreads, 0, ctx->stream>>>(a);
+        gb_pair_kernel<<<dim3(a.n_tiles, systems), kGbThreads, 0, ctx->stream>>>(a);
+        gb_total_kernel<<<systems, kGbThreads, 0, ctx->stream>>>(a);
         rc = cuda_check(ctx, cudaGetLastError(), "gbsa kernels launch");
     }
-    std::vector<double> part(n);
-    queue_copy(ctx, &rc, part.data(), a.partial, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream, "gbsa sums");
+    std::vector<double> out(systems);
+    queue_copy(ctx, &rc, out.data(), a.energy, sizeof(double) * systems, cudaMemcpyDeviceToHost, ctx->stream, "gbsa sums");
     cudaFreeAsync(mem, ctx->stream);
     rc = sync_copies(ctx, rc, ctx->stream, "gbsa");
     if (rc) return rc;
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += part[i];
-    *out = s;
+    for (int p = 0; p < n; ++p) {
+        parts[3 * p] = out[p];
+        parts[3 * p + 1] = out[n + nc + p];
+        parts[3 * p + 2] = out[n + (nc > 1 ? p : 0)];
+    }
     return PXD_OK;
 }
 
@@ -553,27 +759,6 @@ int pxd_score_dev(pxd_context* ctx, int32_t which, int32_t n_poses, int32_t max_
     return cuda_check(ctx, cudaGetLastError(), "empirical_score_kernel launch");
 }
 
-// Receptor coordinates for torsions t in FP64 (torsional_receptor::apply_parameters).
-static std::vector<double> receptor_coords(pxd_context* ctx, const double* t) {
-    std::vector<double> x = ctx->rec_xyz;
-    for (int r = 0; r < ctx->rec.n_rotors; ++r) {
-        const double* k = &ctx->rotor_axis[3 * r];
-        const double* o = &ctx->rotor_origin[3 * r];
-        const double st = std::sin(t[r]), ct = std::cos(t[r]), omc = 1 - ct;
-        const double m[9] = {ct + k[0] * k[0] * omc,        k[0] * k[1] * omc - k[2] * st,
-                             k[1] * st + k[0] * k[2] * omc, k[2] * st + k[0] * k[1] * omc,
-                             ct + k[1] * k[1] * omc,        k[1] * k[2] * omc - k[0] * st,
-                             k[0] * k[2] * omc - k[1] * st, k[0] * st + k[1] * k[2] * omc,
-                             ct + k[2] * k[2] * omc};
-        for (int u = ctx->rotor_mov_off[r]; u < ctx->rotor_mov_off[r + 1]; ++u) {
-            double* p = &x[3 * static_cast<size_t>(ctx->mov_atoms[u])];
-            const double v[3] = {p[0] - o[0], p[1] - o[1], p[2] - o[2]};
-            for (int d = 0; d < 3; ++d) p[d] = m[3 * d] * v[0] + m[3 * d + 1] * v[1] + m[3 * d + 2] * v[2] + o[d];
-        }
-    }
-    return x;
-}
-
 int pxd_score_gbsa(pxd_context* ctx, int32_t lig, const double* lig_xyz, const double* rec_tors, double* delta,
                    double* parts) {
     if (!ctx || !lig_xyz || !delta) return PXD_ERR_INVALID;
@@ -581,29 +766,12 @@ int pxd_score_gbsa(pxd_context* ctx, int32_t lig, const double* lig_xyz, const d
     if (lig < 0 || lig >= static_cast<int>(ctx->ligands.size())) return set_error(ctx, PXD_ERR_INVALID, "ligand id");
     if (ctx->rec.n_rotors > 0 && !rec_tors) return set_error(ctx, PXD_ERR_INVALID, "receptor torsions required");
     cudaSetDevice(ctx->device);
-    const LigandEntry& e = ctx->ligands[lig];
-    const int nl = e.n_atoms, nr = ctx->n_rec;
-    std::vector<double> rx = receptor_coords(ctx, rec_tors);
-    std::vector<double> lx(lig_xyz, lig_xyz + 3 * static_cast<size_t>(nl));
-    double e_pro = 0, e_lig = 0, e_com = 0;
-    int rc = gbsa_system(ctx, nr, rx, ctx->rec_charge, ctx->rec_gb_radius, ctx->rec_gb_screen, &e_pro);
+    double out[3];
+    const int rc = gbsa_batch(ctx, ctx->ligands[lig], 1, lig_xyz, rec_tors, out);
     if (rc) return rc;
-    rc = gbsa_system(ctx, nl, lx, e.charge, e.gb_radius, e.gb_screen, &e_lig);
-    if (rc) return rc;
-    // complex: ligand atoms first, then the receptor (scorer.cpp:770-780)
-    std::vector<double> cx = lx, cq = e.charge, cr = e.gb_radius, cs = e.gb_screen;
-    cx.insert(cx.end(), rx.begin(), rx.end());
-    cq.insert(cq.end(), ctx->rec_charge.begin(), ctx->rec_charge.end());
-    cr.insert(cr.end(), ctx->rec_gb_radius.begin(), ctx->rec_gb_radius.end());
-    cs.insert(cs.end(), ctx->rec_gb_screen.begin(), ctx->rec_gb_screen.end());
-    rc = gbsa_system(ctx, nl + nr, cx, cq, cr, cs, &e_com);
-    if (rc) return rc;
-    *delta = e_com - e_lig - e_pro;
-    if (parts) {
-        parts[0] = e_com;
-        parts[1] = e_lig;
-        parts[2] = e_pro;
-    }
+    *delta = out[0] - out[1] - out[2];
+    if (parts)
+        for (int k = 0; k < 3; ++k) parts[k] = out[k];
     return PXD_OK;
 }
 
@@ -642,15 +810,22 @@ int pxd_score(pxd_context* ctx, int32_t which, int32_t lig, int32_t n_poses, con
     rc = sync_copies(ctx, rc, ctx->stream, "score");
     if (rc) return rc;
     const double gcoef = ctx->sf_host[which].coef[PXD_TERM_GBSA];
-    for (int p = 0; p < n_poses; ++p) {
-        if (gcoef > 1e-5 || gcoef < -1e-5) {
-            double g = 0.0;
-            rc = pxd_score_gbsa(ctx, lig, xyz + 3 * static_cast<size_t>(N) * p, tors + static_cast<size_t>(R) * p, &g,
-                                nullptr);
+    if (gcoef > 1e-5 || gcoef < -1e-5) {
+        if (R > 0 && !tors) return set_error(ctx, PXD_ERR_INVALID, "receptor torsions required");
+        std::vector<double> parts(3 * static_cast<size_t>(std::min(n_poses, kGbPoses)));
+        for (int p0 = 0; p0 < n_poses; p0 += kGbPoses) {
+            const int n = std::min(kGbPoses, n_poses - p0);
+            rc = gbsa_batch(ctx, ctx->ligands[lig], n, xyz + 3 * static_cast<size_t>(N) * p0,
+                            R > 0 ? tors + static_cast<size_t>(R) * p0 : nullptr, parts.data());
             if (rc) return rc;
-            ht2[static_cast<size_t>(p) * PXD_NUM_TERMS + PXD_TERM_GBSA] = g;
-            score[p] += gcoef * g;
+            for (int p = 0; p < n; ++p) {
+                const double g = parts[3 * p] - parts[3 * p + 1] - parts[3 * p + 2];
+                ht2[static_cast<size_t>(p0 + p) * PXD_NUM_TERMS + PXD_TERM_GBSA] = g;
+                score[p0 + p] += gcoef * g;
+            }
         }
+    }
+    for (int p = 0; p < n_poses; ++p) {
         if (terms)
             for (int k = 0; k < PXD_NUM_TERMS; ++k)
                 terms[static_cast<size_t>(p) * PXD_NUM_TERMS + k] = ht2[static_cast<size_t>(p) * PXD_NUM_TERMS + k];

@@ -821,35 +821,7 @@ int pxd_grid_build(pxd_context* ctx, const pxd_box* box, const int32_t* types, i
     if (rc) return set_error(ctx, rc, "vdW type out of range");
     rc = alloc_maps(ctx, box, tl);
     if (rc) return rc;
-    // non-rotor receptor atoms (grid.cpp:119-123, 173)
-    std::vector<float4> xq, xl;
-    std::vector<float2> se;
-    std::vector<double2> se64;
-    for (int a = 0; a < ctx->n_rec; ++a) {
-        if (ctx->is_mov[a]) continue;
-        se64.push_back(make_double2(ctx->rec_sigma[a], ctx->rec_epsilon[a]));
-        const double* x = &ctx->rec_xyz[3 * a];
-        const float4 hi = make_float4(static_cast<float>(x[0]), static_cast<float>(x[1]), static_cast<float>(x[2]),
-                                      static_cast<float>(ctx->rec_charge[a]));
-        xq.push_back(hi);
-        xl.push_back(make_float4(static_cast<float>(x[0] - hi.x), static_cast<float>(x[1] - hi.y),
-                                 static_cast<float>(x[2] - hi.z), static_cast<float>(ctx->rec_charge[a] - hi.w)));
-        se.push_back(make_float2(static_cast<float>(ctx->rec_sigma[a]), static_cast<float>(ctx->rec_epsilon[a])));
-    }
-    std::vector<int> slot_type(ctx->n_slots, -1);
-    for (size_t k = 0; k < tl.size(); ++k) slot_type[1 + k] = tl[k];
-    Packer pk;
-    const size_t o_xq = pk.put(xq), o_xl = pk.put(xl), o_se = pk.put(se), o_st = pk.put(slot_type);
-    const size_t o_se64 = pk.put(se64);
-    void* mem = nullptr;
-    rc = cuda_check(ctx, cudaMalloc(&mem, pk.bytes.size()), "grid atom upload");
-    if (rc) return rc;
-    rc = cuda_check(ctx, cudaMemcpy(mem, pk.bytes.data(), pk.bytes.size(), cudaMemcpyHostToDevice), "grid atom copy");
-    if (!rc)
-        rc = launch_grid_build(ctx, at<float4>(mem, o_xq), at<float4>(mem, o_xl), at<float2>(mem, o_se),
-                               at<double2>(mem, o_se64), static_cast<int>(xq.size()), at<int>(mem, o_st),
-                               ctx->n_slots, ctx->maps, const_cast<float*>(ctx->grid.e_lo));
-    cudaFree(mem);
+    rc = launch_grid_build(ctx, tl);
     if (rc) {
         pxd_grid_drop(ctx);
         return rc;

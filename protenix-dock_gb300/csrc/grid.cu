@@ -1,208 +1,504 @@
 // Receptor map build on the GPU: replaces receptor_cache::populate and
 // partial_worker::populate (grid.cpp:115-195).
 //
-// One thread per (grid point, map); a block covers 128 consecutive points (k fastest)
-// of one map, so all its threads read the same receptor-atom tile from shared memory
-// (broadcast). Pair terms are FP32; each 256-atom tile's partial sums are folded into
-// FP64 accumulators, which keeps the Coulomb sum over ~2k atoms of mixed sign accurate.
-// Atom and point coordinates travel as FP32 hi + lo pairs, so each difference
-// atom - point is formed to FP32 relative precision: a plain FP32 coordinate carries
-// ~1e-6 A of rounding, which the 12th power of the LJ term would amplify 12-fold.
-// The Coulomb map is summed in FP64 (see the loop).
-// The squared distance is floored at 1e-4 A^2 so that a grid point sitting on an atom
-// cannot overflow FP32, and records are clamped to +-1e30 before the FP32 store.
+// The Lennard-Jones energy of every ligand type is a combination of the same sums over the
+// receptor: with the receptor atoms grouped by (sigma, epsilon) into classes c,
+//   E_t(p) = sum_c C_tc (s_tc^12 m12_c - s_tc^6 m6_c),     m_n = sum_i r_i^-n
+// (s_tc the mean sigma, C_tc = 4 sqrt(eps_t eps_c)). grid_moment_kernel walks the receptor
+// once per point for the Coulomb map and the sums of every class, so the exact part of the
+// work no longer grows with the number of types; grid_lj_kernel forms the LJ gradients of a
+// few types per walk and combines the sums into their energies.
 //
-// The energy channel is also kept in FP64 for the final FP64 energy of a pose: every LJ
-// pair term above kFp64Term kcal/mol in magnitude is recomputed in FP64 from FP64 sigma,
-// epsilon and coordinates (an FP32 term carries ~1e-6 of its size, 100 kcal/mol on a
-// 1e8 clash), the smaller ones stay FP32 (each under ~1e-8 kcal/mol of rounding, ~1e-6
-// over a point's atoms), and the record's energy is the FP64 sum rounded to FP32 with the
-// remainder stored in e_lo. The FP64 terms (atoms within ~6.5 A of the point) bound the
-// build by the FP64 pipe.
+// Precision. FP64 runs at 1/64 of FP32 here and bounded the build (84 % of the FP64 pipe busy)
+// when the Coulomb terms and the LJ terms near a point were FP64 per (point, map). The pair
+// terms of grid_moment_kernel are FP32 pairs (hi + lo, ~47 bits, products by fma, sums by
+// two-sum) instead:
+//   - atom and point coordinates are split into a hi part on a common power-of-two grid, so
+//     that the difference of two hi parts is exact, and an FP32 remainder (~2^-44 A);
+//   - 1/r comes from the FP32 rsqrt with a third-order correction in pairs;
+//   - r^-6 and r^-12 of atoms closer than 2 A are formed and summed in FP64 from the FP64
+//     coordinates (the 12th power of a clash amplifies the coordinates' rounding most);
+//   - the classes' energies are combined in FP64, and kept as the FP32 record and the FP32
+//     remainder below it.
+// The Coulomb map needs the pairs throughout: its q/r terms of both signs cancel to a small
+// part of their size. Against FP64 sums over the same points the LJ energies are off by
+// 3e-15 of themselves in the median (4e-13 before) and 1e-11 kcal/mol where |E| < 10 (1e-7
+// before, when the terms under 1e-2 kcal/mol were plain FP32); the Coulomb energies of a unit
+// charge by 2e-11 kcal/mol (3e-13 before; 1e-15 of the sum of the terms' sizes).
+// The LJ gradients are FP32 per pair from hi + lo coordinate differences, folded into FP64
+// every kGridTile atoms. Squared distances are floored at 1e-4 A^2 (a point that sits on an
+// atom cannot overflow FP32) and records clamped to +-1e30 before the FP32 store.
+//
+// Measured, 81^3 points x 1,866 atoms: 12 maps in 11.1 ms (104 ms with FP64 terms per point and
+// map): 5.0 ms for grid_moment_kernel and 3.0 ms for each walk of grid_lj_kernel over 6 types,
+// both near the FP32 issue rate; all 99 types over 55 x 49 x 53 points in 15.9 ms (240 ms).
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <map>
+#include <vector>
+
 #include "device_eval.cuh"
 #include "../../include/pxdock_gb300_vdw.h"
 
 namespace pxd {
 
 constexpr int kGridThreads = 128;
-constexpr int kGridTile = 256;
+constexpr int kMomentTile = 128;
+constexpr int kGridTile = 256;  // atoms per FP32 partial sum of the LJ gradients
 constexpr float kR2Floor = 1e-4f;
+constexpr float kNearR2 = 4.f;  // A^2: closer atoms' LJ powers are FP64
+// Systems that reach further than this from an atom to a point (A) give up the common hi
+// grid, whose step would grow with them (an outlying atom would cost every point precision),
+// for two-sum differences: 15 operations a pair more.
+constexpr double kGridReach = 256.0;
 constexpr double kRecordCeil = 1e30;
 constexpr double kCoulombD = 332.0637141491396;  // kCoulombFactor, system.h:83
-constexpr float kFp64Term = 1e-2f;
+constexpr size_t kMomentBytes = 2 * sizeof(double);  // per point and class
+constexpr size_t kMomentLimit = size_t(96) << 20;  // workspace of the sums; larger boxes run in chunks
+
+struct GridClass {
+    int first, count;  // atoms [first, first + count) of the class-ordered list
+    int slot;          // index of its sums, -1: epsilon 0, Coulomb only
+};
+
+struct FoldCoef {
+    double a12, a6;  // C s^12, C s^6
+};
+
+// The atoms with LJ terms in receptor order, in tiles of kGridTile receptor atoms.
+struct LjAtoms {
+    const float4* hi;     // x, y, z rounded to FP32; class slot (int bits)
+    const float4* lo;     // x, y, z remainders
+    const int2* tiles;    // [n_tiles] first, count
+    int n_tiles;
+    const float2* kind;   // [n_slots] sigma, epsilon of a class
+    const float2* types;  // [n_types] sigma, epsilon of a ligand type
+};
 
 struct GridArgs {
-    const float4* atoms;   // x, y, z, charge of every non-rotor receptor atom (FP32 hi part)
-    const float4* atoms_lo;// x, y, z, charge residuals: value - hi, in FP32
-    const float2* se;      // sigma, epsilon
-    const double2* se64;   // sigma, epsilon in FP64
-    int n_atoms;
+    const float4* hi;        // class order: coordinates on the hi grid relative to `origin`, charge
+    const float4* lo;        // remainders
+    const double4* x64;      // FP64 coordinates
+    const GridClass* classes;
+    int n_classes, n_slots;  // n_slots: classes with sums
     int3 npts;
     double3 init;
     double spacing;
-    const int* slot_type;  // [n_slots] ligand type, or -1 for the Coulomb map
-    const float2* type_se; // [99] sigma, epsilon of the ligand types
-    const double2* type_se64;
-    float4* maps;
-    float* e_lo;           // [n_slots][P] FP64 energy - FP32 record energy
+    double3 origin;
+    double step, step_inv;   // hi grid
+    int p0, n_points;        // points [p0, p0 + n_points) of the box in this launch
     int P;
+    double* m6;              // [n_slots][n_points]
+    double* m12;
+    LjAtoms lj;
+    const FoldCoef* coef;    // [n_types][n_slots]
+    int n_types;
+    float4* maps;            // [1 + n_types][P]
+    float* e_lo;
 };
 
 __device__ __forceinline__ float clampf_rec(double v) {
     return static_cast<float>(fmin(fmax(v, -kRecordCeil), kRecordCeil));
 }
 
-__global__ void __launch_bounds__(kGridThreads) grid_build_kernel(const GridArgs a) {
-    __shared__ float4 s_xyzq[kGridTile];
-    __shared__ float4 s_lo[kGridTile];
-    __shared__ float2 s_se[kGridTile];
-    __shared__ double2 s_se64[kGridTile];
-    const int p = blockIdx.x * kGridThreads + threadIdx.x;
-    const int slot = blockIdx.y;
-    const int type = a.slot_type[slot];
-    const bool coul = type < 0;
-    const float2 tse = coul ? make_float2(0.f, 0.f) : a.type_se[type];
-    const double2 tse64 = coul ? make_double2(0.0, 0.0) : a.type_se64[type];
+__device__ __forceinline__ void store_record(const GridArgs& a, int slot, int p, double E, float gx, float gy, float gz) {
+    const float hi = clampf_rec(E);
+    a.maps[static_cast<size_t>(slot) * a.P + p] = make_float4(hi, gx, gy, gz);
+    a.e_lo[static_cast<size_t>(slot) * a.P + p] =
+        fabs(E) < kRecordCeil ? static_cast<float>(E - static_cast<double>(hi)) : 0.f;
+}
+
+// acc += v + e with the rounding of hi + v kept (two-sum); the intrinsics keep the compiler
+// from contracting the pieces.
+__device__ __forceinline__ void pair_acc(float& hi, float& lo, float v, float e) {
+    const float s = __fadd_rn(hi, v);
+    const float b = __fsub_rn(s, hi);
+    const float err = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(v, b));
+    hi = s;
+    lo = __fadd_rn(lo, __fadd_rn(err, e));
+}
+
+struct PointSums {
+    float eh, el, xh, xl, yh, yl, zh, zl;  // Coulomb energy and gradient
+    float m6h, m6l, m12h, m12l;            // LJ sums of the current class
+    double m6d, m12d;                      // its atoms within 2 A
+};
+
+// a.hi - p.hi and the remainder of the difference. kWide: the hi parts are not on a common
+// grid, so the difference's rounding is formed too (two-sum).
+template <bool kWide>
+__device__ __forceinline__ void coord_diff(float ah, float al, float ph, float pl, float& d, float& e) {
+    d = __fsub_rn(ah, ph);
+    e = __fsub_rn(al, pl);
+    if (kWide) {
+        const float b = __fsub_rn(d, ah);
+        e = __fadd_rn(e, __fsub_rn(__fsub_rn(ah, __fsub_rn(d, b)), __fadd_rn(ph, b)));
+    }
+}
+
+// Adds one receptor atom to the sums of the point (ph + pl, FP64 p64).
+template <bool kLj, bool kWide>
+__device__ __forceinline__ void grid_pair(const float4 ah, const float4 al, const double4* x64, float3 ph, float3 pl,
+                                          double3 p64, PointSums& s) {
+    float dx, dy, dz, ex, ey, ez;
+    coord_diff<kWide>(ah.x, al.x, ph.x, pl.x, dx, ex);
+    coord_diff<kWide>(ah.y, al.y, ph.y, pl.y, dy, ey);
+    coord_diff<kWide>(ah.z, al.z, ph.z, pl.z, dz, ez);
+    // r^2 as r2 + r2l
+    const float sx = __fmul_rn(dx, dx), sy = __fmul_rn(dy, dy), sz = __fmul_rn(dz, dz);
+    float r2l = __fadd_rn(__fmaf_rn(dx, dx, -sx), __fadd_rn(__fmaf_rn(dy, dy, -sy), __fmaf_rn(dz, dz, -sz)));
+    const float cross = __fmaf_rn(dx, ex, __fmaf_rn(dy, ey, __fmul_rn(dz, ez)));
+    r2l = __fmaf_rn(2.f, cross, r2l);
+    float r2 = sx;
+    pair_acc(r2, r2l, sy, 0.f);
+    pair_acc(r2, r2l, sz, 0.f);
+    const bool near = r2 < kNearR2;
+    double n6 = 0.0;
+    if (near) {
+        if (r2 < kR2Floor) {
+            r2 = kR2Floor;
+            r2l = 0.f;
+        }
+        if (kLj) {
+            const double4 x = *x64;
+            const double ux = x.x - p64.x, uy = x.y - p64.y, uz = x.z - p64.z;
+            const double inv = 1.0 / fmax(ux * ux + uy * uy + uz * uz, static_cast<double>(kR2Floor));
+            n6 = inv * inv * inv;
+            s.m6d += n6;
+            s.m12d += n6 * n6;
+        }
+    }
+    // 1/r = y + c and 1/r^2 = ih + il from y ~ 1/r and h = 1 - r^2 y^2
+    const float y = rsqrtf(r2);
+    const float ih = __fmul_rn(y, y);
+    const float yl = __fmaf_rn(y, y, -ih);
+    float h = __fmaf_rn(-r2, ih, 1.f);
+    h = __fmaf_rn(-r2, yl, h);
+    h = __fmaf_rn(-r2l, ih, h);
+    const float c = __fmul_rn(y, __fmul_rn(h, __fmaf_rn(h, 0.375f, 0.5f)));
+    const float il = __fmaf_rn(ih, __fmaf_rn(h, h, h), yl);
+    // Coulomb: q/r and q (x - p)/r^3
+    const float q = __fmul_rn(ah.w, y);
+    float ql = __fmaf_rn(ah.w, y, -q);
+    ql = __fmaf_rn(ah.w, c, ql);
+    ql = __fmaf_rn(al.w, y, ql);
+    pair_acc(s.eh, s.el, q, ql);
+    const float w = __fmul_rn(q, ih);
+    float wl = __fmaf_rn(q, ih, -w);
+    wl = __fmaf_rn(q, il, wl);
+    wl = __fmaf_rn(ql, ih, wl);
+    const float gx = __fmul_rn(w, dx), gy = __fmul_rn(w, dy), gz = __fmul_rn(w, dz);
+    pair_acc(s.xh, s.xl, gx, __fmaf_rn(wl, dx, __fmaf_rn(w, ex, __fmaf_rn(w, dx, -gx))));
+    pair_acc(s.yh, s.yl, gy, __fmaf_rn(wl, dy, __fmaf_rn(w, ey, __fmaf_rn(w, dy, -gy))));
+    pair_acc(s.zh, s.zl, gz, __fmaf_rn(wl, dz, __fmaf_rn(w, ez, __fmaf_rn(w, dz, -gz))));
+    if (kLj) {
+        const float i4 = __fmul_rn(ih, ih);
+        const float i4l = __fmaf_rn(__fadd_rn(ih, ih), il, __fmaf_rn(ih, ih, -i4));
+        float i6 = __fmul_rn(i4, ih);
+        float i6l = __fmaf_rn(i4l, ih, __fmaf_rn(i4, il, __fmaf_rn(i4, ih, -i6)));
+        float i12 = __fmul_rn(i6, i6);
+        float i12l = __fmaf_rn(__fadd_rn(i6, i6), i6l, __fmaf_rn(i6, i6, -i12));
+        if (near) i6 = i6l = i12 = i12l = 0.f;  // summed in FP64 above
+        pair_acc(s.m6h, s.m6l, i6, i6l);
+        pair_acc(s.m12h, s.m12l, i12, i12l);
+    }
+}
+
+// One thread per point, 128 consecutive points (k fastest) per block, so that every thread
+// reads the same atom of a shared-memory tile (broadcast). About 150 FP32 operations a pair:
+// bound by FP32 issue.
+template <bool kWide>
+__global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_constant__ GridArgs a) {
+    __shared__ float4 s_hi[kMomentTile];
+    __shared__ float4 s_lo[kMomentTile];
+    const int t = blockIdx.x * kGridThreads + threadIdx.x;
+    const int p = a.p0 + t;
     const int nz = a.npts.z, ny = a.npts.y;
     const int k = p % nz;
     const int j = (p / nz) % ny;
     const int i = p / (nz * ny);
     // grid.cpp:159-163: point = init + spacing * index, formed in FP64
+    const double3 p64 = make_double3(a.init.x + a.spacing * i, a.init.y + a.spacing * j, a.init.z + a.spacing * k);
+    const double rx = p64.x - a.origin.x, ry = p64.y - a.origin.y, rz = p64.z - a.origin.z;
+    auto hi_part = [&a](double r) { return kWide ? static_cast<double>(static_cast<float>(r)) : rint(r * a.step_inv) * a.step; };
+    const double hx = hi_part(rx), hy = hi_part(ry), hz = hi_part(rz);
+    const float3 ph = make_float3(static_cast<float>(hx), static_cast<float>(hy), static_cast<float>(hz));
+    const float3 pl = make_float3(static_cast<float>(rx - hx), static_cast<float>(ry - hy), static_cast<float>(rz - hz));
+    PointSums s{};
+    double E = 0.0;
+    for (int c = 0; c < a.n_classes; ++c) {
+        const GridClass gc = a.classes[c];
+        for (int t0 = 0; t0 < gc.count; t0 += kMomentTile) {
+            const int n = min(kMomentTile, gc.count - t0);
+            const int base = gc.first + t0;
+            __syncthreads();
+            for (int u = threadIdx.x; u < n; u += kGridThreads) {
+                s_hi[u] = a.hi[base + u];
+                s_lo[u] = a.lo[base + u];
+            }
+            __syncthreads();
+            if (gc.slot >= 0) {
+                for (int u = 0; u < n; ++u) grid_pair<true, kWide>(s_hi[u], s_lo[u], a.x64 + base + u, ph, pl, p64, s);
+            } else {
+                for (int u = 0; u < n; ++u) grid_pair<false, kWide>(s_hi[u], s_lo[u], nullptr, ph, pl, p64, s);
+            }
+            // the low part of a long sum would round at ~1e-11 kcal/mol
+            E += static_cast<double>(s.eh) + static_cast<double>(s.el);
+            s.eh = s.el = 0.f;
+        }
+        if (gc.slot >= 0) {
+            if (t < a.n_points) {
+                const size_t o = static_cast<size_t>(gc.slot) * a.n_points + t;
+                a.m6[o] = s.m6d + (static_cast<double>(s.m6h) + static_cast<double>(s.m6l));
+                a.m12[o] = s.m12d + (static_cast<double>(s.m12h) + static_cast<double>(s.m12l));
+            }
+            s.m6h = s.m6l = s.m12h = s.m12l = 0.f;
+            s.m6d = s.m12d = 0.0;
+        }
+    }
+    if (t < a.n_points) {
+        auto total = [](float h, float l) { return (static_cast<double>(h) + static_cast<double>(l)) * kCoulombD; };
+        store_record(a, 0, p, E * kCoulombD, clampf_rec(total(s.xh, s.xl)), clampf_rec(total(s.yh, s.yl)),
+                     clampf_rec(total(s.zh, s.zl)));
+    }
+}
+
+// LJ records of kTypes ligand types per thread: the FP32 gradients from one walk over the
+// receptor (~38 operations a pair that the types share, 11 a type), the energies from the
+// classes' sums (two FP64 operations a type and class). Bound by FP32 issue.
+template <int kTypes>
+__global__ void __launch_bounds__(kGridThreads) grid_lj_kernel(const __grid_constant__ GridArgs a) {
+    __shared__ float4 s_x[kGridTile];
+    __shared__ float4 s_lo[kGridTile];
+    __shared__ float2 s_p[kGridTile][kTypes];  // (mean sigma)^2, 4 sqrt(eps eps) of an atom and a type
+    const int t = blockIdx.x * kGridThreads + threadIdx.x;
+    const int t0 = blockIdx.y * kTypes;
+    const int p = a.p0 + t;
+    const int nz = a.npts.z, ny = a.npts.y;
+    const int k = p % nz;
+    const int j = (p / nz) % ny;
+    const int i = p / (nz * ny);
     const double px = a.init.x + a.spacing * i, py = a.init.y + a.spacing * j, pz = a.init.z + a.spacing * k;
     const float3 pt = make_float3(static_cast<float>(px), static_cast<float>(py), static_cast<float>(pz));
     const float3 pl = make_float3(static_cast<float>(px - pt.x), static_cast<float>(py - pt.y),
                                   static_cast<float>(pz - pt.z));
-    double E = 0.0, GX = 0.0, GY = 0.0, GZ = 0.0;
-    double E64 = 0.0;  // LJ terms recomputed in FP64
-    for (int t0 = 0; t0 < a.n_atoms; t0 += kGridTile) {
-        const int n = min(kGridTile, a.n_atoms - t0);
+    double GX[kTypes], GY[kTypes], GZ[kTypes];
+#pragma unroll
+    for (int g = 0; g < kTypes; ++g) GX[g] = GY[g] = GZ[g] = 0.0;
+    for (int b = 0; b < a.lj.n_tiles; ++b) {
+        const int2 tile = a.lj.tiles[b];
         __syncthreads();
-        for (int u = threadIdx.x; u < n; u += kGridThreads) {
-            s_xyzq[u] = a.atoms[t0 + u];
-            s_lo[u] = a.atoms_lo[t0 + u];
-            s_se[u] = a.se[t0 + u];
-            s_se64[u] = a.se64[t0 + u];
+        for (int u = threadIdx.x; u < tile.y; u += kGridThreads) {
+            s_x[u] = a.lj.hi[tile.x + u];
+            s_lo[u] = a.lj.lo[tile.x + u];
+            const float2 se = a.lj.kind[__float_as_int(s_x[u].w)];
+            for (int g = 0; g < kTypes; ++g) {
+                const float2 tse = a.lj.types[min(t0 + g, a.n_types - 1)];
+                const float s = (tse.x + se.x) * 0.5f;
+                s_p[u][g] = make_float2(s * s, sqrtf(tse.y * se.y) * 4.f);
+            }
         }
         __syncthreads();
-        float e = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
-        if (coul) {
-            // FP64 per pair: the map is a sum of ~M terms q/r of both signs that cancel
-            // to a small fraction of their magnitudes, so FP32 rounding of each term
-            // (~1e-7 relative) would leave ~1e-3 kcal/mol in the records
-            double ce = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
-            for (int u = 0; u < n; ++u) {
-                const float4 at = s_xyzq[u];
-                const float4 lo = s_lo[u];
-                const double vx = (static_cast<double>(at.x) - px) + static_cast<double>(lo.x);
-                const double vy = (static_cast<double>(at.y) - py) + static_cast<double>(lo.y);
-                const double vz = (static_cast<double>(at.z) - pz) + static_cast<double>(lo.z);
-                const double r2 = fmax(vx * vx + vy * vy + vz * vz, static_cast<double>(kR2Floor));
-                const double rinv = rsqrt(r2);
-                const double qr = (static_cast<double>(at.w) + static_cast<double>(lo.w)) * rinv;
-                ce += qr;
-                // dE/dpoint = q (atom - point) / r^3 (pair.h:25-40 with grad_i -= ...)
-                const double w = qr * rinv * rinv;
-                cx = fma(vx, w, cx);
-                cy = fma(vy, w, cy);
-                cz = fma(vz, w, cz);
-            }
-            E += ce * kCoulombD;
-            GX += cx * kCoulombD;
-            GY += cy * kCoulombD;
-            GZ += cz * kCoulombD;
-        } else {
-            for (int u = 0; u < n; ++u) {
-                const float4 at = s_xyzq[u];
-                const float4 lo = s_lo[u];
-                const float2 se = s_se[u];
-                const float vx = (at.x - pt.x) + (lo.x - pl.x), vy = (at.y - pt.y) + (lo.y - pl.y),
-                            vz = (at.z - pt.z) + (lo.z - pl.z);
-                const float r2 = fmaxf(vx * vx + vy * vy + vz * vz, kR2Floor);
-                const float rinv2 = 1.f / r2;
-                const float s = (tse.x + se.x) * 0.5f;
-                const float x = s * s * rinv2;
+        float gx[kTypes], gy[kTypes], gz[kTypes];
+#pragma unroll
+        for (int g = 0; g < kTypes; ++g) gx[g] = gy[g] = gz[g] = 0.f;
+        for (int u = 0; u < tile.y; ++u) {
+            const float4 at = s_x[u];
+            const float4 lo = s_lo[u];
+            const float vx = (at.x - pt.x) + (lo.x - pl.x), vy = (at.y - pt.y) + (lo.y - pl.y),
+                        vz = (at.z - pt.z) + (lo.z - pl.z);
+            const float r2 = fmaxf(vx * vx + vy * vy + vz * vz, kR2Floor);
+            const float rinv2 = 1.f / r2;
+#pragma unroll
+            for (int g = 0; g < kTypes; ++g) {
+                const float2 sc = s_p[u][g];
+                const float x = sc.x * rinv2;
                 const float u6 = x * x * x;
                 const float u12 = u6 * u6;
-                const float C = sqrtf(tse.y * se.y) * 4.f;
-                const float ep = C * (u12 - u6);
-                if (fabsf(ep) > kFp64Term) {
-                    const double2 se64 = s_se64[u];
-                    const double dx = (static_cast<double>(at.x) - px) + static_cast<double>(lo.x);
-                    const double dy = (static_cast<double>(at.y) - py) + static_cast<double>(lo.y);
-                    const double dz = (static_cast<double>(at.z) - pz) + static_cast<double>(lo.z);
-                    const double r2d = fmax(dx * dx + dy * dy + dz * dz, static_cast<double>(kR2Floor));
-                    const double sd = (tse64.x + se64.x) * 0.5;
-                    const double xd = sd * sd / r2d;
-                    const double u6d = xd * xd * xd;
-                    E64 += sqrt(tse64.y * se64.y) * 4.0 * (u6d * u6d - u6d);
-                } else {
-                    e += ep;
-                }
                 // grad_point -= vec * de_dr_r, de_dr_r = C(-12 u12 + 6 u6) / r^2 (pair.h:42-60)
-                const float w = C * (12.f * u12 - 6.f * u6) * rinv2;
-                gx = fmaf(vx, w, gx);
-                gy = fmaf(vy, w, gy);
-                gz = fmaf(vz, w, gz);
+                const float w = sc.y * (12.f * u12 - 6.f * u6) * rinv2;
+                gx[g] = fmaf(vx, w, gx[g]);
+                gy[g] = fmaf(vy, w, gy[g]);
+                gz[g] = fmaf(vz, w, gz[g]);
             }
-            E += e;
-            GX += gx;
-            GY += gy;
-            GZ += gz;
+        }
+#pragma unroll
+        for (int g = 0; g < kTypes; ++g) {
+            GX[g] += gx[g];
+            GY[g] += gy[g];
+            GZ[g] += gz[g];
         }
     }
-    if (p < a.P) {
-        const double Ef = E + E64;
-        const float hi = clampf_rec(Ef);
-        a.maps[static_cast<size_t>(slot) * a.P + p] = make_float4(hi, clampf_rec(GX), clampf_rec(GY), clampf_rec(GZ));
-        const double rest = Ef - static_cast<double>(hi);
-        a.e_lo[static_cast<size_t>(slot) * a.P + p] =
-            fabs(Ef) < kRecordCeil ? static_cast<float>(rest) : 0.f;
+    if (t >= a.n_points) return;
+    double E[kTypes];
+#pragma unroll
+    for (int g = 0; g < kTypes; ++g) E[g] = 0.0;
+    for (int c = 0; c < a.n_slots; ++c) {
+        const size_t o = static_cast<size_t>(c) * a.n_points + t;
+        const double m6 = a.m6[o], m12 = a.m12[o];
+#pragma unroll
+        for (int g = 0; g < kTypes; ++g) {
+            const FoldCoef f = a.coef[static_cast<size_t>(min(t0 + g, a.n_types - 1)) * a.n_slots + c];
+            E[g] += f.a12 * m12 - f.a6 * m6;
+        }
     }
+#pragma unroll
+    for (int g = 0; g < kTypes; ++g)
+        if (t0 + g < a.n_types)
+            store_record(a, 1 + t0 + g, p, E[g], clampf_rec(GX[g]), clampf_rec(GY[g]), clampf_rec(GZ[g]));
 }
 
-int launch_grid_build(pxd_context* ctx, const float4* atoms, const float4* atoms_lo, const float2* se,
-                      const double2* se64, int n_atoms, const int* slot_type, int n_slots, float4* maps,
-                      float* e_lo) {
+// Types per thread: as even as groups of at most 8 allow (a smaller group repeats the walk's
+// shared part more often, a larger one no longer fits the registers).
+static void launch_lj(const GridArgs& a, int blocks, cudaStream_t s) {
+    const int groups = (a.n_types + 7) / 8;
+    const int per = (a.n_types + groups - 1) / groups;
+    const dim3 grid(blocks, groups);
+    if (per > 6)
+        grid_lj_kernel<8><<<grid, kGridThreads, 0, s>>>(a);
+    else if (per > 4)
+        grid_lj_kernel<6><<<grid, kGridThreads, 0, s>>>(a);
+    else if (per > 2)
+        grid_lj_kernel<4><<<grid, kGridThreads, 0, s>>>(a);
+    else
+        grid_lj_kernel<2><<<grid, kGridThreads, 0, s>>>(a);
+}
+
+// Builds the Coulomb map (slot 0) and the maps of `types` (slots 1..) over the context's
+// box from every non-rotor receptor atom (grid.cpp:119-123, 173). Synchronous.
+int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
+    std::map<std::pair<double, double>, std::vector<int>> by_kind;  // (epsilon, sigma) -> atoms
+    for (int i = 0; i < ctx->n_rec; ++i)
+        if (!ctx->is_mov[i]) by_kind[{ctx->rec_epsilon[i], ctx->rec_sigma[i]}].push_back(i);
     GridArgs a{};
-    a.atoms = atoms;
-    a.atoms_lo = atoms_lo;
-    a.se = se;
-    a.se64 = se64;
-    a.e_lo = e_lo;
-    a.n_atoms = n_atoms;
     a.npts = make_int3(ctx->box.npoints[0], ctx->box.npoints[1], ctx->box.npoints[2]);
     a.init = make_double3(ctx->box.init_xyz[0], ctx->box.init_xyz[1], ctx->box.init_xyz[2]);
     a.spacing = ctx->box.spacing;
-    a.slot_type = slot_type;
-    a.maps = maps;
     a.P = ctx->grid.P;
-    // ligand type table on the device (sigma, epsilon)
-    struct Tables {
-        float2 f32[PXD_NUM_VDW_TYPES];
-        double2 f64[PXD_NUM_VDW_TYPES];
-    } table;
-    for (int t = 0; t < PXD_NUM_VDW_TYPES; ++t) {
-        table.f32[t] = make_float2(static_cast<float>(PXD_VDW_SIGMA[t]), static_cast<float>(PXD_VDW_EPSILON[t]));
-        table.f64[t] = make_double2(PXD_VDW_SIGMA[t], PXD_VDW_EPSILON[t]);
+    a.maps = ctx->maps;
+    a.e_lo = const_cast<float*>(ctx->grid.e_lo);
+    a.n_types = static_cast<int>(types.size());
+    // the hi grid: 2^24 steps span the largest coordinate difference of an atom and a point
+    double half[3], reach = 0.0;
+    for (int d = 0; d < 3; ++d) {
+        half[d] = 0.5 * (ctx->box.npoints[d] - 1) * ctx->box.spacing;
+        (&a.origin.x)[d] = ctx->box.init_xyz[d] + half[d];
+        reach = std::max(reach, half[d]);
     }
-    Tables* d_table = nullptr;
-    int rc = cuda_check(ctx, cudaMallocAsync(&d_table, sizeof(table), ctx->stream), "type table");
-    if (rc) return rc;
-    rc = cuda_check(ctx, cudaMemcpyAsync(d_table, &table, sizeof(table), cudaMemcpyHostToDevice,
-                                         ctx->stream),
-                    "type table copy");
-    if (rc) {
-        cudaFreeAsync(d_table, ctx->stream);
-        return rc;
+    for (const auto& [kind, atoms] : by_kind)
+        for (int i : atoms)
+            for (int d = 0; d < 3; ++d) {
+                const double r = std::fabs(ctx->rec_xyz[3 * i + d] - (&a.origin.x)[d]) + half[d];
+                if (std::isfinite(r)) reach = std::max(reach, r);
+            }
+    const bool wide = reach >= kGridReach;
+    a.step = std::ldexp(1.0, std::ilogb(std::max(reach, 1.0)) + 1 - 24);
+    a.step_inv = 1.0 / a.step;
+    std::vector<float4> hi, lo;
+    std::vector<double4> x64;
+    std::vector<GridClass> classes;
+    std::vector<int> order;  // receptor atoms in class order
+    std::vector<std::pair<double, double>> kinds;  // of the classes with sums
+    for (const auto& [kind, atoms] : by_kind) {
+        const bool lj = kind.first != 0.0;
+        classes.push_back({static_cast<int>(hi.size()), static_cast<int>(atoms.size()),
+                           lj ? static_cast<int>(kinds.size()) : -1});
+        if (lj) kinds.push_back(kind);
+        for (int i : atoms) {
+            order.push_back(i);
+            float h[4], l[4];
+            for (int d = 0; d < 3; ++d) {
+                const double r = ctx->rec_xyz[3 * i + d] - (&a.origin.x)[d];
+                const double g = wide ? static_cast<double>(static_cast<float>(r)) : std::rint(r * a.step_inv) * a.step;
+                h[d] = static_cast<float>(g);
+                l[d] = static_cast<float>(r - g);
+            }
+            h[3] = static_cast<float>(ctx->rec_charge[i]);
+            l[3] = static_cast<float>(ctx->rec_charge[i] - h[3]);
+            hi.push_back(make_float4(h[0], h[1], h[2], h[3]));
+            lo.push_back(make_float4(l[0], l[1], l[2], l[3]));
+            x64.push_back(make_double4(ctx->rec_xyz[3 * i], ctx->rec_xyz[3 * i + 1], ctx->rec_xyz[3 * i + 2], 0.0));
+        }
     }
-    a.type_se = d_table->f32;
-    a.type_se64 = d_table->f64;
-    dim3 grid((a.P + kGridThreads - 1) / kGridThreads, n_slots);
-    grid_build_kernel<<<grid, kGridThreads, 0, ctx->stream>>>(a);
-    rc = cuda_check(ctx, cudaGetLastError(), "grid_build_kernel launch");
-    cudaFreeAsync(d_table, ctx->stream);
+    a.n_classes = static_cast<int>(classes.size());
+    a.n_slots = static_cast<int>(kinds.size());
+    std::vector<FoldCoef> coef;
+    for (int t : types)
+        for (const auto& [eps, sigma] : kinds) {
+            const double s = (PXD_VDW_SIGMA[t] + sigma) * 0.5, s6 = std::pow(s, 6.0);
+            const double C = std::sqrt(PXD_VDW_EPSILON[t] * eps) * 4.0;
+            coef.push_back({C * s6 * s6, C * s6});
+        }
+    // the LJ atoms in receptor order, cut at every kGridTile receptor atoms
+    std::vector<float4> lj_hi, lj_lo;
+    std::vector<int2> tiles;
+    std::vector<float2> kind_se, type_se;
+    for (const auto& [eps, sigma] : kinds)
+        kind_se.push_back(make_float2(static_cast<float>(sigma), static_cast<float>(eps)));
+    for (int t : types)
+        type_se.push_back(make_float2(static_cast<float>(PXD_VDW_SIGMA[t]), static_cast<float>(PXD_VDW_EPSILON[t])));
+    std::vector<int> slot_of(ctx->n_rec, -1);
+    for (const GridClass& c : classes)
+        for (int u = 0; u < c.count; ++u) slot_of[order[c.first + u]] = c.slot;
+    for (int i = 0, seen = 0; i < ctx->n_rec; ++i) {
+        if (ctx->is_mov[i]) continue;
+        if (seen++ % kGridTile == 0) tiles.push_back(make_int2(static_cast<int>(lj_hi.size()), 0));
+        if (slot_of[i] < 0) continue;
+        const double* x = &ctx->rec_xyz[3 * i];
+        const float3 h = make_float3(static_cast<float>(x[0]), static_cast<float>(x[1]), static_cast<float>(x[2]));
+        float bits;
+        std::memcpy(&bits, &slot_of[i], sizeof(bits));
+        lj_hi.push_back(make_float4(h.x, h.y, h.z, bits));
+        lj_lo.push_back(make_float4(static_cast<float>(x[0] - h.x), static_cast<float>(x[1] - h.y),
+                                    static_cast<float>(x[2] - h.z), 0.f));
+        ++tiles.back().y;
+    }
+    a.lj.n_tiles = static_cast<int>(tiles.size());
+    // one allocation: inputs, then the sums of a chunk of points
+    const size_t n_slots = std::max(1, a.n_slots);
+    const size_t fit = kMomentLimit / (kMomentBytes * n_slots) / kGridThreads * kGridThreads;
+    const int chunk = static_cast<int>(std::min<size_t>(a.P, std::max<size_t>(fit, kGridThreads)));
+    std::vector<unsigned char> in;
+    auto put = [&in](const auto& v) {
+        const size_t off = in.size(), bytes = v.size() * sizeof(v[0]);
+        in.resize(off + (bytes + 31) / 32 * 32 + 32);
+        if (bytes) std::memcpy(in.data() + off, v.data(), bytes);
+        return off;
+    };
+    const size_t o_hi = put(hi), o_lo = put(lo), o_x = put(x64), o_cls = put(classes), o_coef = put(coef);
+    const size_t o_lh = put(lj_hi), o_ll = put(lj_lo), o_tile = put(tiles), o_kind = put(kind_se), o_type = put(type_se);
+    cudaStream_t s = ctx->stream;
+    char* mem = nullptr;
+    int rc = cuda_check(ctx, cudaMallocAsync(reinterpret_cast<void**>(&mem), in.size() + kMomentBytes * n_slots * chunk, s),
+                        "map build workspace");
     if (rc) return rc;
-    return cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "grid build");
+    queue_copy(ctx, &rc, mem, in.data(), in.size(), cudaMemcpyHostToDevice, s, "map build inputs");
+    a.hi = reinterpret_cast<const float4*>(mem + o_hi);
+    a.lo = reinterpret_cast<const float4*>(mem + o_lo);
+    a.x64 = reinterpret_cast<const double4*>(mem + o_x);
+    a.classes = reinterpret_cast<const GridClass*>(mem + o_cls);
+    a.coef = reinterpret_cast<const FoldCoef*>(mem + o_coef);
+    a.lj.hi = reinterpret_cast<const float4*>(mem + o_lh);
+    a.lj.lo = reinterpret_cast<const float4*>(mem + o_ll);
+    a.lj.tiles = reinterpret_cast<const int2*>(mem + o_tile);
+    a.lj.kind = reinterpret_cast<const float2*>(mem + o_kind);
+    a.lj.types = reinterpret_cast<const float2*>(mem + o_type);
+    a.m6 = reinterpret_cast<double*>(mem + in.size());
+    a.m12 = a.m6 + n_slots * chunk;
+    for (int p0 = 0; p0 < a.P && !rc; p0 += chunk) {
+        a.p0 = p0;
+        a.n_points = std::min(chunk, a.P - p0);
+        const int blocks = (a.n_points + kGridThreads - 1) / kGridThreads;
+        if (wide)
+            grid_moment_kernel<true><<<blocks, kGridThreads, 0, s>>>(a);
+        else
+            grid_moment_kernel<false><<<blocks, kGridThreads, 0, s>>>(a);
+        if (a.n_types > 0) launch_lj(a, blocks, s);
+        rc = cuda_check(ctx, cudaGetLastError(), "map build launch");
+    }
+    cudaFreeAsync(mem, s);
+    return sync_copies(ctx, rc, s, "grid build");
 }
 
 }  // namespace pxd

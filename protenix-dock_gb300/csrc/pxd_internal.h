@@ -283,9 +283,7 @@ cudaError_t launch_with_map_window(const pxd_context* ctx, void (*kern)(KArgs...
 }
 
 // kernels (launchers), one per translation unit
-int launch_grid_build(pxd_context* ctx, const float4* atoms_xyzq, const float4* atoms_lo,
-                      const float2* atoms_se, const double2* atoms_se64, int n_atoms, const int* slot_types,
-                      int n_slots, float4* maps, float* e_lo);
+int launch_grid_build(pxd_context* ctx, const std::vector<int>& types);
 int launch_score(pxd_context* ctx, int n_poses, int max_atoms, const int* lig_ids,
                  const float* xyz, const float* tors, double* energy, float* lig_grad,
                  float* tors_grad, cudaStream_t s);

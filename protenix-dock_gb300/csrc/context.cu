@@ -178,8 +178,12 @@ bool topo_indices_ok(const TopoIn& t) {
 struct TopoOffsets {
     int n_bond_slots, n_angle_slots, n_dih_slots, n_pair_slots;
     size_t bond_ij, bond_p, angle_ijk, angle_p, dih_ijkl, dih_terms, dih_term, pair_ij, pair_p;
+    size_t bond_lo, angle_lo, dih_lo, pair_lo;
     size_t bond_p64, angle_p64, dih_term64, pair_p64;
 };
+
+// What FP32 leaves of v.
+static float remainder32(double v) { return static_cast<float>(v - static_cast<double>(static_cast<float>(v))); }
 
 TopoOffsets pack_topo(Packer& pk, const TopoIn& t) {
     TopoOffsets o{};
@@ -205,6 +209,9 @@ TopoOffsets pack_topo(Packer& pk, const TopoIn& t) {
         o.bond_ij = pk.put(ij);
         o.bond_p = pk.put(p);
         o.bond_p64 = pk.put(p64);
+        std::vector<float2> lo;
+        for (const double2& v : p64) lo.push_back(make_float2(remainder32(v.x), remainder32(v.y)));
+        o.bond_lo = pk.put(lo);
     }
     {
         auto order = schedule_rounds<3>(t.angles, t.n_atoms);
@@ -228,6 +235,9 @@ TopoOffsets pack_topo(Packer& pk, const TopoIn& t) {
         o.angle_ijk = pk.put(ijk);
         o.angle_p = pk.put(p);
         o.angle_p64 = pk.put(p64);
+        std::vector<float> lo;
+        for (const double2& v : p64) lo.push_back(remainder32(v.y));
+        o.angle_lo = pk.put(lo);
     }
     {
         auto order = schedule_rounds<4>(t.dih, t.n_atoms);
@@ -256,6 +266,9 @@ TopoOffsets pack_topo(Packer& pk, const TopoIn& t) {
         o.dih_terms = pk.put(tr);
         o.dih_term = pk.put(terms);
         o.dih_term64 = pk.put(terms64);
+        std::vector<float> lo;
+        for (const double4& v : terms64) lo.push_back(remainder32(v.x));
+        o.dih_lo = pk.put(lo);
     }
     {
         auto order = schedule_rounds<2>(t.pairs, t.n_atoms);
@@ -284,6 +297,9 @@ TopoOffsets pack_topo(Packer& pk, const TopoIn& t) {
         o.pair_ij = pk.put(ij);
         o.pair_p = pk.put(p);
         o.pair_p64 = pk.put(p64);
+        std::vector<float4> lo;
+        for (const double4& v : p64) lo.push_back(make_float4(remainder32(v.x), remainder32(v.y), remainder32(v.z), 0.f));
+        o.pair_lo = pk.put(lo);
     }
     return o;
 }
@@ -304,6 +320,10 @@ DevTopo topo_pointers(void* base, int n_atoms, const TopoOffsets& o) {
     d.dih_term = at<float4>(base, o.dih_term);
     d.pair_ij = at<int2>(base, o.pair_ij);
     d.pair_p = at<float4>(base, o.pair_p);
+    d.bond_lo = at<float2>(base, o.bond_lo);
+    d.angle_lo = at<float>(base, o.angle_lo);
+    d.dih_lo = at<float>(base, o.dih_lo);
+    d.pair_lo = at<float4>(base, o.pair_lo);
     d.bond_p64 = at<double2>(base, o.bond_p64);
     d.angle_p64 = at<double2>(base, o.angle_p64);
     d.dih_term64 = at<double4>(base, o.dih_term64);
@@ -752,6 +772,14 @@ int pxd_decide_grid_dims(double cx, double cy, double cz, double sx, double sy, 
     return PXD_OK;
 }
 
+// v as a sum of n FP32 parts, each the rounding of what is left.
+static void split_parts(double v, float* parts, int n) {
+    for (int k = 0; k < n; ++k) {
+        parts[k] = static_cast<float>(v);
+        v -= static_cast<double>(parts[k]);
+    }
+}
+
 static int alloc_maps(pxd_context* ctx, const pxd_box* box, const std::vector<int>& types) {
     pxd_grid_drop(ctx);
     for (int d = 0; d < 3; ++d)
@@ -789,9 +817,10 @@ static int alloc_maps(pxd_context* ctx, const pxd_box* box, const std::vector<in
     g.P = static_cast<int>(P);
     g.maps = ctx->maps;
     g.e_lo = reinterpret_cast<const float*>(ctx->maps + P * ctx->n_slots);
-    g.init64 = make_double3(box->init_xyz[0], box->init_xyz[1], box->init_xyz[2]);
-    g.spacing64 = box->spacing;
-    g.slope64 = ctx->slope;
+    for (int d = 0; d < 3; ++d) split_parts(box->init_xyz[d], g.init_p[d], 3);
+    split_parts(box->spacing, g.spacing_p, 3);
+    split_parts(1.0 / box->spacing, g.spacing_inv_p, 2);
+    split_parts(ctx->slope, g.slope_p, 2);
     return PXD_OK;
 }
 
@@ -841,7 +870,7 @@ int pxd_grid_set_slope(pxd_context* ctx, double slope) {
     if (!ctx) return PXD_ERR_INVALID;
     ctx->slope = slope;
     ctx->grid.slope = static_cast<float>(slope);
-    ctx->grid.slope64 = slope;
+    split_parts(slope, ctx->grid.slope_p, 2);
     return PXD_OK;
 }
 
@@ -1004,10 +1033,12 @@ int pxd_add_ligand(pxd_context* ctx, const pxd_ligand_desc* lig, int32_t* ligand
     std::vector<float> q(N);
     std::vector<int> slots(N, -1), types(lig->vdw_type, lig->vdw_type + N);
     std::vector<float2> se(N);
+    std::vector<float> q_lo(N);
     std::vector<double> q64(N);
     std::vector<double2> se64(N);
     for (int a = 0; a < N; ++a) {
         q64[a] = lig->ff.charge[a];
+        q_lo[a] = remainder32(q64[a]);
         se64[a] = make_double2(PXD_VDW_SIGMA[types[a]], PXD_VDW_EPSILON[types[a]]);
         q[a] = static_cast<float>(lig->ff.charge[a]);
         se[a] = make_float2(static_cast<float>(PXD_VDW_SIGMA[types[a]]), static_cast<float>(PXD_VDW_EPSILON[types[a]]));
@@ -1018,7 +1049,7 @@ int pxd_add_ligand(pxd_context* ctx, const pxd_ligand_desc* lig, int32_t* ligand
         }
     }
     const size_t o_q = pk.put(q), o_slot = pk.put(slots), o_se = pk.put(se), o_type = pk.put(types);
-    const size_t o_q64 = pk.put(q64), o_se64 = pk.put(se64);
+    const size_t o_q64 = pk.put(q64), o_se64 = pk.put(se64), o_qlo = pk.put(q_lo);
     // torsion tree
     const pxd_torsion_tree& tr = lig->tree;
     if (tr.n_frags > 0) {
@@ -1077,6 +1108,7 @@ int pxd_add_ligand(pxd_context* ctx, const pxd_ligand_desc* lig, int32_t* ligand
     d.charge = at<float>(e.mem, o_q);
     d.map_slot = at<int>(e.mem, o_slot);
     d.se = at<float2>(e.mem, o_se);
+    d.charge_lo = at<float>(e.mem, o_qlo);
     d.charge64 = at<double>(e.mem, o_q64);
     d.se64 = at<double2>(e.mem, o_se64);
     d.type = at<int>(e.mem, o_type);

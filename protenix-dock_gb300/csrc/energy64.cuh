@@ -1,25 +1,34 @@
-// Energy of one pose in FP64, no gradient: the value of
+// Reported energy of one pose, no gradient: the value of
 // binding_system_interactions::put_gradients (interaction.cpp:259-350) at the pose that an
 // optimiser or a search returns, to within 1e-3 kcal/mol of the FP64 reference at any
 // energy. The optimiser steers on the FP32 evaluation (device_eval.cuh); this evaluation
 // gives the reported number. One warp per pose, every lane returns the same value.
 //
+// The ligand's terms and the map lookups are FP32 pairs (device_pairs.cuh): a pose's
+// coordinates are FP32, so their differences are exact pairs, and every term carries ~1e-13
+// of itself. In FP64 the pair terms over 1 kcal/mol alone (present in nearly every round of
+// 32) held the FP64 pipe for 20,000 of the 25,000 cycles of a 42-atom pose:
+// score_kernel took 6.6 ms for 65,536 poses.
+//
 // Precision per term, against the FP64 objective:
-//   - grid lookups (grid.cpp:197-303): FP64 box geometry, penalty and trilinear weights over
-//     map energies E = FP32 record + FP32 residual of the FP64 sum (grid build);
-//   - bonds (interaction.cpp:27-47): FP64 (unbounded in a stretched bond);
-//   - pairs, intra and explicit inter (pair.h:25-60): FP32, recomputed in FP64 from FP64
-//     parameters when the FP32 term exceeds 1 kcal/mol (FP32 carries ~1e-6 of a term, so
-//     a 1e6 clash would be off by 1 kcal/mol; terms under 1 kcal/mol stay below 1e-6);
-//   - angles and dihedrals (interaction.cpp:49-117): FP32 geometry, FP64 sums. These are
+//   - grid lookups (grid.cpp:197-303): an atom's place in its cell from the box's geometry in
+//     three FP32 parts, weights and sums in pairs, over map energies E = FP32 record + FP32
+//     residual of the FP64 sum (grid build);
+//   - bonds (interaction.cpp:27-47) and intra pairs (pair.h:25-60) of the ligand: pairs, FP64
+//     where atoms nearly coincide or fly apart beyond FP32's range;
+//   - angles and dihedrals (interaction.cpp:49-117): FP32 geometry, sums in pairs. These are
 //     bounded (0.5 k pi^2, 2 sum k): an FP32 angle error of ~1e-7 rad moves a term by at
 //     most k |theta - theta0| 1e-7, ~1e-5 kcal/mol;
-//   - receptor rotor atoms (interaction.cpp:316-336): FP64 rotations of FP64 coordinates.
-// Every per-lane sum is FP64 and the warp sum is a fixed butterfly, so the value repeats
-// bit for bit.
+//   - receptor rotor atoms (interaction.cpp:316-336): FP64 rotations of FP64 coordinates; their
+//     terms and the explicit inter pairs in FP32, recomputed in FP64 from FP64 parameters
+//     when the FP32 term exceeds 1 kcal/mol (FP32 carries ~1e-6 of a term, so a 1e6 clash
+//     would be off by 1 kcal/mol; terms under 1 kcal/mol stay below 1e-6).
+// Every per-lane sum runs in a fixed order and the warp sum is a fixed butterfly, so the
+// value repeats bit for bit.
 #pragma once
 
 #include "device_eval.cuh"
+#include "device_pairs.cuh"
 
 namespace pxd {
 
@@ -52,8 +61,8 @@ __device__ __forceinline__ double pair_energy64(double4 p, D3 xi, D3 xj) {
     return p.x / sqrt(r2) + p.y * (u6 * u6 - u6);
 }
 
-// Energy of the terms of `t` (intra_molecular_interactions) with positions given in FP32
-// (P32) and FP64 (P64) by index.
+// Energy of the receptor's rotor-touching terms (intra_molecular_interactions) with positions
+// given in FP32 (P32) and FP64 (P64) by index.
 template <class P32, class P64>
 __device__ double topo_energy64(const DevTopo& t, const P32& pos32, const P64& pos64, int lane) {
     double e = 0.0;
@@ -111,47 +120,156 @@ __device__ double topo_energy64(const DevTopo& t, const P32& pos32, const P64& p
     return e;
 }
 
-// receptor_cache::get (grid.cpp:197-262) energy in FP64 for an atom of charge q at p.
-__device__ __forceinline__ double grid_energy64(const DevGrid& g, int slot, double q, D3 p) {
-    const double sinv = 1.0 / g.spacing64;
-    double f[3] = {(p.x - g.init64.x) * sinv, (p.y - g.init64.y) * sinv, (p.z - g.init64.z) * sinv};
-    const int npm1[3] = {g.npts.x - 1, g.npts.y - 1, g.npts.z - 1};
-    int lo[3];
-    double penalty = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        if (f[d] < 0.0) {
-            lo[d] = 0;
-            penalty -= f[d];
-            f[d] = 0.0;
-        } else if (f[d] < static_cast<double>(npm1[d])) {
-            lo[d] = static_cast<int>(f[d]);
+// Squared distances for which a bond or pair term stays in pairs; outside (coincident atoms,
+// whose 12th power leaves FP32's range, or atoms flung apart) it is FP64.
+constexpr float kPairR2Min = 1e-2f, kPairR2Max = 1e30f;
+
+__device__ __forceinline__ F2 atom_distance2(const float* x, int i, int j) {
+    return pair_norm2(two_diff(x[3 * j], x[3 * i]), two_diff(x[3 * j + 1], x[3 * i + 1]),
+                      two_diff(x[3 * j + 2], x[3 * i + 2]));
+}
+
+// Energy of the ligand's terms at FP32 coordinates x, added to `e` in pairs; terms out of the
+// pairs' range to `e64`.
+__device__ __forceinline__ void ligand_energy(const DevTopo& t, const float* x, F2& e, double& e64, int lane) {
+    auto pos = [x](int i) { return make_float3(x[3 * i], x[3 * i + 1], x[3 * i + 2]); };
+    auto pos64 = [x](int i) {
+        return D3{static_cast<double>(x[3 * i]), static_cast<double>(x[3 * i + 1]), static_cast<double>(x[3 * i + 2])};
+    };
+    for (int s = lane; s < t.n_bond_slots; s += kWarp) {
+        const int2 ij = __ldg(&t.bond_ij[s]);
+        if (ij.x < 0) continue;
+        const F2 r2 = atom_distance2(x, ij.x, ij.y);
+        if (r2.h > kPairR2Min && r2.h < kPairR2Max) {
+            const float2 p = __ldg(&t.bond_p[s]), pl = __ldg(&t.bond_lo[s]);
+            F2 rinv, inv;
+            pair_rsqrt(r2, rinv, inv);
+            const F2 dr = pair_sub(pair_norm(pair_mul(r2, rinv)), {p.y, pl.y});
+            pair_acc(e, pair_mul({0.5f * p.x, 0.5f * pl.x}, pair_square(pair_norm(dr))));
         } else {
-            lo[d] = npm1[d] - 1;
-            penalty += f[d] - npm1[d];
-            f[d] = npm1[d];
+            const double2 p = __ldg(&t.bond_p64[s]);
+            const D3 d = d3_sub(pos64(ij.y), pos64(ij.x));
+            const double dr = sqrt(d3_dot(d, d)) - p.y;
+            e64 += 0.5 * p.x * (dr * dr);
         }
     }
-    const double x = f[0] - lo[0], y = f[1] - lo[1], z = f[2] - lo[2];
-    const double mx = 1.0 - x, my = 1.0 - y, mz = 1.0 - z;
-    const double w[8] = {mx * my * mz, x * my * mz, mx * y * mz, x * y * mz,
-                         mx * my * z,  x * my * z,  mx * y * z,  x * y * z};
+    for (int s = lane; s < t.n_angle_slots; s += kWarp) {
+        const int4 ijk = __ldg(&t.angle_ijk[s]);
+        if (ijk.x < 0) continue;
+        const float2 p = __ldg(&t.angle_p[s]);
+        const float3 xi = pos(ijk.x), xj = pos(ijk.y), xk = pos(ijk.z);
+        const float3 v0 = sub3(xj, xi), v1 = sub3(xj, xk);
+        const float3 c = cross3(v0, v1);
+        const float theta = atan2f(sqrtf(dot3(c, c)), dot3(v0, v1) + kEpsF);
+        const F2 delta = pair_sub({theta, 0.f}, {p.y, __ldg(&t.angle_lo[s])});
+        pair_acc(e, pair_mul(pair_square(pair_norm(delta)), 0.5f * p.x));
+    }
+    for (int s = lane; s < t.n_dih_slots; s += kWarp) {
+        const int4 q = __ldg(&t.dih_ijkl[s]);
+        if (q.x < 0) continue;
+        const float3 pi = pos(q.x), pj = pos(q.y), pk = pos(q.z), pl = pos(q.w);
+        const float3 rij = sub3(pj, pi), rkj = sub3(pj, pk), rkl = sub3(pl, pk);
+        const float3 m = cross3(rij, rkj), n = cross3(rkj, rkl);
+        const float3 w = cross3(m, n);
+        const float phi = atan2f(sqrtf(dot3(w, w)), dot3(m, n) + kEpsF);
+        const float theta = dot3(rij, n) < 0.f ? phi : -phi;
+        const int2 tr = __ldg(&t.dih_terms[s]);
+        for (int u = 0; u < tr.y; ++u) {
+            const float4 term = __ldg(&t.dih_term[tr.x + u]);  // k, periodicity, phase
+            const float delta = theta * term.y - term.z;
+            pair_acc(e, pair_mul({term.x, __ldg(&t.dih_lo[tr.x + u])}, two_diff(1.f, -cosf(delta))));
+        }
+    }
+    for (int s = lane; s < t.n_pair_slots; s += kWarp) {
+        const int2 ij = __ldg(&t.pair_ij[s]);
+        if (ij.x < 0) continue;
+        const F2 r2 = atom_distance2(x, ij.x, ij.y);
+        if (r2.h > kPairR2Min && r2.h < kPairR2Max) {
+            const float4 p = __ldg(&t.pair_p[s]), pl = __ldg(&t.pair_lo[s]);  // A, C, S2
+            F2 rinv, inv;
+            pair_rsqrt(r2, rinv, inv);
+            const F2 u = pair_mul(inv, F2{p.z, pl.z});
+            const F2 u6 = pair_mul(pair_square(u), u);
+            pair_acc(e, pair_mul(pair_sub(pair_square(u6), u6), F2{p.y, pl.y}));
+            pair_acc(e, pair_mul(rinv, F2{p.x, pl.x}));
+        } else {
+            e64 += pair_energy64(t.pair_p64[s], pos64(ij.x), pos64(ij.y));
+        }
+    }
+}
+
+// One axis of an atom's place in the maps (receptor_cache::get, grid.cpp:211-262): its cell,
+// its fraction of the cell as a pair, and how far beyond the box it is (A, 0 inside).
+__device__ __forceinline__ void grid_place(const float* init, const DevGrid& g, int npts, float p, int& cell, F2& frac,
+                                           F2& beyond) {
+    const int last = npts - 2;  // the last cell
+    int c = static_cast<int>(floorf((p - init[0]) * g.spacing_inv));
+    c = min(max(c, 0), last);
+    // r = p - init - c spacing: the leading parts exactly, the small ones in a pair
+    const F2 d = two_diff(p, init[0]);
+    const F2 b = pair_mul({g.spacing_p[0], 0.f}, static_cast<float>(c));  // exact product
+    F2 r = two_diff(d.h, b.h);
+    F2 small{d.l, r.l};
+    pair_acc(small.h, small.l, -b.l, 0.f);
+    pair_acc(small.h, small.l, -init[1], -init[2]);
+    const F2 b1 = pair_mul({g.spacing_p[1], 0.f}, static_cast<float>(c));
+    pair_acc(small.h, small.l, -b1.h, -fmaf(g.spacing_p[2], static_cast<float>(c), b1.l));
+    r.l = 0.f;
+    pair_acc(r, small);
+    r = pair_norm(r);
+    const F2 sp{g.spacing_p[0], g.spacing_p[1]};
+    // the cell's FP32 estimate can be one off next to a grid point
+    if (r.h < 0.f && c > 0) {
+        --c;
+        pair_acc(r, sp);
+    } else if (c < last && (r.h - sp.h) + (r.l - sp.l) >= 0.f) {
+        ++c;
+        r = pair_sub(r, sp);
+    }
+    r = pair_norm(r);
+    const F2 over = pair_norm(pair_sub(r, sp));
+    cell = c;
+    beyond = {0.f, 0.f};
+    if (c == 0 && r.h < 0.f) {
+        beyond = {-r.h, -r.l};
+        frac = {0.f, 0.f};
+    } else if (c == last && over.h >= 0.f) {
+        beyond = over;
+        frac = {1.f, 0.f};
+    } else {
+        frac = pair_norm(pair_mul(r, F2{g.spacing_inv_p[0], g.spacing_inv_p[1]}));
+    }
+}
+
+// receptor_cache::get (grid.cpp:197-262) energy in pairs for an atom of charge q at p.
+__device__ __forceinline__ void grid_energy(const DevGrid& g, int slot, F2 q, float3 p, F2& e, double& e64) {
+    int cx, cy, cz;
+    F2 x, y, z, bx, by, bz;
+    grid_place(g.init_p[0], g, g.npts.x, p.x, cx, x, bx);
+    grid_place(g.init_p[1], g, g.npts.y, p.y, cy, y, by);
+    grid_place(g.init_p[2], g, g.npts.z, p.z, cz, z, bz);
+    pair_acc(bx, by);
+    pair_acc(bx, bz);
+    if (bx.h > 0.f && bx.h < 1e25f)
+        pair_acc(e, pair_mul(pair_norm(bx), F2{g.slope_p[0], g.slope_p[1]}));
+    else if (bx.h > 0.f)  // an atom flung so far that the penalty could leave FP32's range
+        e64 += static_cast<double>(bx.h) * (static_cast<double>(g.slope_p[0]) + static_cast<double>(g.slope_p[1]));
+    const F2 one{1.f, 0.f};
+    const F2 mx = pair_norm(pair_sub(one, x)), my = pair_norm(pair_sub(one, y)), mz = pair_norm(pair_sub(one, z));
+    const F2 xy[4] = {pair_mul(mx, my), pair_mul(x, my), pair_mul(mx, y), pair_mul(x, y)};
     const int sy = g.npts.z, sx = g.npts.y * g.npts.z;
-    const int base = lo[0] * sx + lo[1] * sy + lo[2];
-    const int off[8] = {base,     base + sx,     base + sy,     base + sx + sy,
-                        base + 1, base + sx + 1, base + sy + 1, base + sx + sy + 1};
-    double e = penalty > 0.0 ? penalty * g.spacing64 * g.slope64 : 0.0;
-    double ec = 0.0, ev = 0.0;
+    const int base = cx * sx + cy * sy + cz;
     const size_t P = static_cast<size_t>(g.P);
+    F2 ec{0.f, 0.f}, ev{0.f, 0.f};
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-        ec += (static_cast<double>(__ldg(&g.maps[off[c]].x)) + static_cast<double>(__ldg(&g.e_lo[off[c]]))) * w[c];
-        if (slot > 0)
-            ev += (static_cast<double>(__ldg(&g.maps[slot * P + off[c]].x)) +
-                   static_cast<double>(__ldg(&g.e_lo[slot * P + off[c]]))) *
-                  w[c];
+        const int off = base + (c & 1 ? sx : 0) + (c & 2 ? sy : 0) + (c & 4 ? 1 : 0);
+        const F2 w = pair_mul(xy[c & 3], c & 4 ? z : mz);
+        pair_acc(ec, pair_mul(w, F2{__ldg(&g.maps[off].x), __ldg(&g.e_lo[off])}));
+        if (slot > 0) pair_acc(ev, pair_mul(w, F2{__ldg(&g.maps[slot * P + off].x), __ldg(&g.e_lo[slot * P + off])}));
     }
-    return e + ec * q + ev;
+    pair_acc(e, pair_mul(pair_norm(ec), q));
+    pair_acc(e, ev);
 }
 
 // FP64 energy of the pose x = [ligand xyz (3N) | receptor torsions] (shared memory, the
@@ -196,11 +314,13 @@ static __device__ __noinline__ double energy64(const EvalEnv& env, const DevLiga
         return make_float3(static_cast<float>(loc64[3 * l]), static_cast<float>(loc64[3 * l + 1]),
                            static_cast<float>(loc64[3 * l + 2]));
     };
-    double e = topo_energy64(L.topo, lig32, lig64, lane);
+    F2 ep{0.f, 0.f};
+    double e = 0.0;
+    ligand_energy(L.topo, x, ep, e, lane);
     if (R.n_local > 0) e += topo_energy64(R.intra, loc32, loc64f, lane);
     if (env.grid.has_grid) {
         for (int a = lane; a < N; a += kWarp)
-            e += grid_energy64(env.grid, __ldg(&L.map_slot[a]), __ldg(&L.charge64[a]), lig64(a));
+            grid_energy(env.grid, __ldg(&L.map_slot[a]), F2{__ldg(&L.charge[a]), __ldg(&L.charge_lo[a])}, lig32(a), ep, e);
     }
     // explicit inter pairs, one (ligand atom, receptor atom) pair per lane and step
     const int M = R.n_explicit;
@@ -229,7 +349,10 @@ static __device__ __noinline__ double energy64(const EvalEnv& env, const DevLiga
             e += pair_energy64(p, lig64(i), loc >= 0 ? loc64f(loc) : D3{r64.x, r64.y, r64.z});
         }
     }
-    return warp_sum_d(e) + R.e_const;
+    // the pairs' warp sum in FP32 (two-sum), the FP64 terms' only where a lane has one
+    const double pairs_sum = ds_warp_sum(DS{ep.h, ep.l});
+    if (__any_sync(kFull, e != 0.0)) return pairs_sum + warp_sum_d(e) + R.e_const;
+    return pairs_sum + R.e_const;
 }
 
 }  // namespace pxd

@@ -39,6 +39,7 @@
 #include <vector>
 
 #include "device_eval.cuh"
+#include "device_pairs.cuh"
 #include "../../include/pxdock_gb300_vdw.h"
 
 namespace pxd {
@@ -109,99 +110,56 @@ __device__ __forceinline__ void store_record(const GridArgs& a, int slot, int p,
         fabs(E) < kRecordCeil ? static_cast<float>(E - static_cast<double>(hi)) : 0.f;
 }
 
-// acc += v + e with the rounding of hi + v kept (two-sum); the intrinsics keep the compiler
-// from contracting the pieces.
-__device__ __forceinline__ void pair_acc(float& hi, float& lo, float v, float e) {
-    const float s = __fadd_rn(hi, v);
-    const float b = __fsub_rn(s, hi);
-    const float err = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(v, b));
-    hi = s;
-    lo = __fadd_rn(lo, __fadd_rn(err, e));
-}
-
 struct PointSums {
-    float eh, el, xh, xl, yh, yl, zh, zl;  // Coulomb energy and gradient
-    float m6h, m6l, m12h, m12l;            // LJ sums of the current class
-    double m6d, m12d;                      // its atoms within 2 A
+    F2 e, x, y, z;     // Coulomb energy and gradient
+    F2 m6, m12;        // LJ sums of the current class
+    double m6d, m12d;  // its atoms within 2 A
 };
+
+__device__ __forceinline__ double to_double(F2 a) { return static_cast<double>(a.h) + static_cast<double>(a.l); }
 
 // a.hi - p.hi and the remainder of the difference. kWide: the hi parts are not on a common
 // grid, so the difference's rounding is formed too (two-sum).
 template <bool kWide>
-__device__ __forceinline__ void coord_diff(float ah, float al, float ph, float pl, float& d, float& e) {
-    d = __fsub_rn(ah, ph);
-    e = __fsub_rn(al, pl);
-    if (kWide) {
-        const float b = __fsub_rn(d, ah);
-        e = __fadd_rn(e, __fsub_rn(__fsub_rn(ah, __fsub_rn(d, b)), __fadd_rn(ph, b)));
-    }
+__device__ __forceinline__ F2 coord_diff(float ah, float al, float ph, float pl) {
+    if (kWide) return pair_sub({ah, al}, {ph, pl});
+    return {__fsub_rn(ah, ph), __fsub_rn(al, pl)};
 }
 
 // Adds one receptor atom to the sums of the point (ph + pl, FP64 p64).
 template <bool kLj, bool kWide>
 __device__ __forceinline__ void grid_pair(const float4 ah, const float4 al, const double4* x64, float3 ph, float3 pl,
                                           double3 p64, PointSums& s) {
-    float dx, dy, dz, ex, ey, ez;
-    coord_diff<kWide>(ah.x, al.x, ph.x, pl.x, dx, ex);
-    coord_diff<kWide>(ah.y, al.y, ph.y, pl.y, dy, ey);
-    coord_diff<kWide>(ah.z, al.z, ph.z, pl.z, dz, ez);
-    // r^2 as r2 + r2l
-    const float sx = __fmul_rn(dx, dx), sy = __fmul_rn(dy, dy), sz = __fmul_rn(dz, dz);
-    float r2l = __fadd_rn(__fmaf_rn(dx, dx, -sx), __fadd_rn(__fmaf_rn(dy, dy, -sy), __fmaf_rn(dz, dz, -sz)));
-    const float cross = __fmaf_rn(dx, ex, __fmaf_rn(dy, ey, __fmul_rn(dz, ez)));
-    r2l = __fmaf_rn(2.f, cross, r2l);
-    float r2 = sx;
-    pair_acc(r2, r2l, sy, 0.f);
-    pair_acc(r2, r2l, sz, 0.f);
-    const bool near = r2 < kNearR2;
-    double n6 = 0.0;
+    const F2 dx = coord_diff<kWide>(ah.x, al.x, ph.x, pl.x), dy = coord_diff<kWide>(ah.y, al.y, ph.y, pl.y),
+             dz = coord_diff<kWide>(ah.z, al.z, ph.z, pl.z);
+    F2 r2 = pair_norm2(dx, dy, dz);
+    const bool near = r2.h < kNearR2;
     if (near) {
-        if (r2 < kR2Floor) {
-            r2 = kR2Floor;
-            r2l = 0.f;
-        }
+        if (r2.h < kR2Floor) r2 = {kR2Floor, 0.f};
         if (kLj) {
             const double4 x = *x64;
             const double ux = x.x - p64.x, uy = x.y - p64.y, uz = x.z - p64.z;
             const double inv = 1.0 / fmax(ux * ux + uy * uy + uz * uz, static_cast<double>(kR2Floor));
-            n6 = inv * inv * inv;
+            const double n6 = inv * inv * inv;
             s.m6d += n6;
             s.m12d += n6 * n6;
         }
     }
-    // 1/r = y + c and 1/r^2 = ih + il from y ~ 1/r and h = 1 - r^2 y^2
-    const float y = rsqrtf(r2);
-    const float ih = __fmul_rn(y, y);
-    const float yl = __fmaf_rn(y, y, -ih);
-    float h = __fmaf_rn(-r2, ih, 1.f);
-    h = __fmaf_rn(-r2, yl, h);
-    h = __fmaf_rn(-r2l, ih, h);
-    const float c = __fmul_rn(y, __fmul_rn(h, __fmaf_rn(h, 0.375f, 0.5f)));
-    const float il = __fmaf_rn(ih, __fmaf_rn(h, h, h), yl);
+    F2 rinv, inv;
+    pair_rsqrt(r2, rinv, inv);
     // Coulomb: q/r and q (x - p)/r^3
-    const float q = __fmul_rn(ah.w, y);
-    float ql = __fmaf_rn(ah.w, y, -q);
-    ql = __fmaf_rn(ah.w, c, ql);
-    ql = __fmaf_rn(al.w, y, ql);
-    pair_acc(s.eh, s.el, q, ql);
-    const float w = __fmul_rn(q, ih);
-    float wl = __fmaf_rn(q, ih, -w);
-    wl = __fmaf_rn(q, il, wl);
-    wl = __fmaf_rn(ql, ih, wl);
-    const float gx = __fmul_rn(w, dx), gy = __fmul_rn(w, dy), gz = __fmul_rn(w, dz);
-    pair_acc(s.xh, s.xl, gx, __fmaf_rn(wl, dx, __fmaf_rn(w, ex, __fmaf_rn(w, dx, -gx))));
-    pair_acc(s.yh, s.yl, gy, __fmaf_rn(wl, dy, __fmaf_rn(w, ey, __fmaf_rn(w, dy, -gy))));
-    pair_acc(s.zh, s.zl, gz, __fmaf_rn(wl, dz, __fmaf_rn(w, ez, __fmaf_rn(w, dz, -gz))));
+    const F2 q = pair_mul({ah.w, al.w}, rinv);
+    pair_acc(s.e, q);
+    const F2 w = pair_mul(q, inv);
+    pair_acc(s.x, pair_mul(dx, w));
+    pair_acc(s.y, pair_mul(dy, w));
+    pair_acc(s.z, pair_mul(dz, w));
     if (kLj) {
-        const float i4 = __fmul_rn(ih, ih);
-        const float i4l = __fmaf_rn(__fadd_rn(ih, ih), il, __fmaf_rn(ih, ih, -i4));
-        float i6 = __fmul_rn(i4, ih);
-        float i6l = __fmaf_rn(i4l, ih, __fmaf_rn(i4, il, __fmaf_rn(i4, ih, -i6)));
-        float i12 = __fmul_rn(i6, i6);
-        float i12l = __fmaf_rn(__fadd_rn(i6, i6), i6l, __fmaf_rn(i6, i6, -i12));
-        if (near) i6 = i6l = i12 = i12l = 0.f;  // summed in FP64 above
-        pair_acc(s.m6h, s.m6l, i6, i6l);
-        pair_acc(s.m12h, s.m12l, i12, i12l);
+        F2 i6 = pair_mul(pair_square(inv), inv);
+        F2 i12 = pair_square(i6);
+        if (near) i6 = i12 = {0.f, 0.f};  // summed in FP64 above
+        pair_acc(s.m6, i6);
+        pair_acc(s.m12, i12);
     }
 }
 
@@ -244,23 +202,22 @@ __global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_
                 for (int u = 0; u < n; ++u) grid_pair<false, kWide>(s_hi[u], s_lo[u], nullptr, ph, pl, p64, s);
             }
             // the low part of a long sum would round at ~1e-11 kcal/mol
-            E += static_cast<double>(s.eh) + static_cast<double>(s.el);
-            s.eh = s.el = 0.f;
+            E += to_double(s.e);
+            s.e = {0.f, 0.f};
         }
         if (gc.slot >= 0) {
             if (t < a.n_points) {
                 const size_t o = static_cast<size_t>(gc.slot) * a.n_points + t;
-                a.m6[o] = s.m6d + (static_cast<double>(s.m6h) + static_cast<double>(s.m6l));
-                a.m12[o] = s.m12d + (static_cast<double>(s.m12h) + static_cast<double>(s.m12l));
+                a.m6[o] = s.m6d + to_double(s.m6);
+                a.m12[o] = s.m12d + to_double(s.m12);
             }
-            s.m6h = s.m6l = s.m12h = s.m12l = 0.f;
+            s.m6 = s.m12 = {0.f, 0.f};
             s.m6d = s.m12d = 0.0;
         }
     }
     if (t < a.n_points) {
-        auto total = [](float h, float l) { return (static_cast<double>(h) + static_cast<double>(l)) * kCoulombD; };
-        store_record(a, 0, p, E * kCoulombD, clampf_rec(total(s.xh, s.xl)), clampf_rec(total(s.yh, s.yl)),
-                     clampf_rec(total(s.zh, s.zl)));
+        store_record(a, 0, p, E * kCoulombD, clampf_rec(to_double(s.x) * kCoulombD), clampf_rec(to_double(s.y) * kCoulombD),
+                     clampf_rec(to_double(s.z) * kCoulombD));
     }
 }
 

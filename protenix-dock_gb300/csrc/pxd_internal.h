@@ -39,7 +39,13 @@ struct DevTopo {
     const float4* dih_term;   // k, periodicity, phase, -
     const int2* pair_ij;
     const float4* pair_p;     // A = 332.06 qi qj s_c, C = 4 sqrt(ei ej) s_v, S2 = ((si+sj)/2)^2
-    // the same parameters in FP64, slot for slot, for the final FP64 energy (energy64.cuh)
+    // the parameters' remainders below their FP32 values, slot for slot, for the reported
+    // energy in FP32 pairs (energy64.cuh)
+    const float2* bond_lo;
+    const float* angle_lo;    // theta0
+    const float* dih_lo;      // k, per term
+    const float4* pair_lo;
+    // the same parameters in FP64, for the reported energy's FP64 terms
     const double2* bond_p64;
     const double2* angle_p64;
     const double4* dih_term64;
@@ -105,6 +111,7 @@ struct DevLigand {
     const float* charge;      // [N]
     const int* map_slot;      // [N] vdW map slot of the atom's type (-1: no map)
     const float2* se;         // [N] sigma, epsilon (explicit inter pairs)
+    const float* charge_lo;   // [N] charge64 - charge
     const double* charge64;   // [N] FP64 copies for the final FP64 energy
     const double2* se64;      // [N]
     const int* type;          // [N] ligand vdW type
@@ -150,10 +157,11 @@ struct DevGrid {
     float slope;
     int P;
     const float4* maps;
-    // the final FP64 energy: box geometry and slope in FP64, and per map point the FP64
-    // energy's residual below its FP32 record, E = maps[.].x + e_lo[.]
-    double3 init64;
-    double spacing64, slope64;
+    // the reported energy: box geometry and slope as sums of FP32 parts (init and spacing in
+    // three, 1/spacing and slope in two), and per map point the FP64 energy's residual below
+    // its FP32 record, E = maps[.].x + e_lo[.]
+    float init_p[3][3];       // [axis][part]
+    float spacing_p[3], spacing_inv_p[2], slope_p[2];
     const float* e_lo;        // [n_slots][P]
 };
 

@@ -178,7 +178,7 @@ bool topo_indices_ok(const TopoIn& t) {
 struct TopoOffsets {
     int n_bond_slots, n_angle_slots, n_dih_slots, n_pair_slots;
     size_t bond_ij, bond_p, angle_ijk, angle_p, dih_ijkl, dih_terms, dih_term, pair_ij, pair_p;
-    size_t bond_lo, angle_lo, dih_lo, pair_lo;
+    size_t dih_first, bond_lo, angle_lo, dih_lo, pair_lo;
     size_t bond_p64, angle_p64, dih_term64, pair_p64;
 };
 
@@ -265,6 +265,13 @@ TopoOffsets pack_topo(Packer& pk, const TopoIn& t) {
         o.dih_ijkl = pk.put(ijkl);
         o.dih_terms = pk.put(tr);
         o.dih_term = pk.put(terms);
+        std::vector<float4> heads;
+        for (const int2& r : tr) {
+            float4 h = r.y > 0 ? terms[r.x] : make_float4(0.f, 0.f, 0.f, 0.f);
+            h.w = bits_as_float(r.x | (r.y << kDihCountShift));
+            heads.push_back(h);
+        }
+        o.dih_first = pk.put(heads);
         o.dih_term64 = pk.put(terms64);
         std::vector<float> lo;
         for (const double4& v : terms64) lo.push_back(remainder32(v.x));
@@ -318,6 +325,7 @@ DevTopo topo_pointers(void* base, int n_atoms, const TopoOffsets& o) {
     d.dih_ijkl = at<int4>(base, o.dih_ijkl);
     d.dih_terms = at<int2>(base, o.dih_terms);
     d.dih_term = at<float4>(base, o.dih_term);
+    d.dih_first = at<float4>(base, o.dih_first);
     d.pair_ij = at<int2>(base, o.pair_ij);
     d.pair_p = at<float4>(base, o.pair_p);
     d.bond_lo = at<float2>(base, o.bond_lo);

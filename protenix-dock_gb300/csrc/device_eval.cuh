@@ -175,20 +175,32 @@ __device__ __forceinline__ void rotation_and_jacobian(float3 k, float theta, Mat
 }
 
 // ------------------------------------------------------------- term kernels
-// Adds `g` to the gradient record p (shared memory): one 16-byte load and store.
-__device__ __forceinline__ void add_rec(float4* p, float3 g) {
-    float4 v = *p;
+// Adds `g` to a gradient record.
+__device__ __forceinline__ void add_rec(float4& v, float3 g) {
     v.x += g.x;
     v.y += g.y;
     v.z += g.z;
-    *p = v;
 }
-__device__ __forceinline__ void sub_rec(float4* p, float3 g) {
-    float4 v = *p;
+__device__ __forceinline__ void sub_rec(float4& v, float3 g) {
     v.x -= g.x;
     v.y -= g.y;
     v.z -= g.z;
-    *p = v;
+}
+
+// Adds g of the lanes 0 .. n - 1 to a gradient record of shared memory in lane order (every
+// lane calls it). Atomics to one record from every lane of a warp retry one lane at a time;
+// the pairs of 43 atoms with 4 rotor atoms took 60,000 of an evaluation's 144,000 cycles that
+// way. The caller's warp barrier comes before the record's next read.
+__device__ __forceinline__ void add_lanes(float4* rec, float3 g, int n, int lane) {
+    float4 v = *rec;
+#pragma unroll 8
+    for (int l = 0; l < n; ++l) {
+        v.x += __shfl_sync(kFull, g.x, l);
+        v.y += __shfl_sync(kFull, g.y, l);
+        v.z += __shfl_sync(kFull, g.z, l);
+    }
+    __syncwarp();
+    if (lane == 0) *rec = v;
 }
 
 // Squared pair distances are floored at 1e-4 A^2 (r = 0.01 A) in the FP32 pair terms: below
@@ -213,129 +225,17 @@ __device__ __forceinline__ float3 pair_grad(float4 p, float4 xi, float4 xj, floa
     return mul3(rij, de_dr_r);
 }
 
-// Adds the bonded and non-bonded terms of `t` over coordinates `X`. The gradient of
-// the atom in position k of a term goes to array k: G[k * gs + atom] (shared memory).
-// Within a round the atoms of each position are distinct (host scheduling), so the
-// lanes of a round update distinct records with plain loads and stores; a warp
-// barrier between rounds orders a record's updates from different rounds. Padded
-// slots (-1) compute nothing. Every loop runs a multiple of 32 slots, so all lanes
-// meet every barrier. The caller sums the arrays. Matches
-// intra_molecular_interactions::put_gradients.
-__device__ __forceinline__ void topo_terms(const DevTopo& t, const float4* X, float4* G, int gs, DS& e,
-                                           int lane) {
-    float4* G0 = G;
-    float4* G1 = G + gs;
-    float4* G2 = G + 2 * gs;
-    float4* G3 = G + 3 * gs;
-    __syncwarp();
-    // harmonic bonds (interaction.cpp:27-47)
-    for (int s = lane; s < t.n_bond_slots; s += kWarp) {
-        const int2 ij = __ldg(&t.bond_ij[s]);
-        if (ij.x >= 0) {
-            const float2 p = __ldg(&t.bond_p[s]);
-            const float3 d = sub3(xyz(X[ij.y]), xyz(X[ij.x]));
-            const float r = sqrtf(dot3(d, d));
-            const float dr = r - p.y;
-            ds_add(e, 0.5f * p.x * (dr * dr));
-            const float de_dr = p.x * (1.f - __fdividef(p.y, r + kEpsF));
-            const float3 g = mul3(d, de_dr);
-            sub_rec(&G0[ij.x], g);
-            add_rec(&G1[ij.y], g);
-        }
-        __syncwarp();
-    }
-    // harmonic angles (interaction.cpp:49-74, math.cpp:96-110)
-    for (int s = lane; s < t.n_angle_slots; s += kWarp) {
-        const int4 ijk = __ldg(&t.angle_ijk[s]);
-        if (ijk.x >= 0) {
-            const float2 p = __ldg(&t.angle_p[s]);
-            const float3 xi = xyz(X[ijk.x]), xj = xyz(X[ijk.y]), xk = xyz(X[ijk.z]);
-            const float3 v0 = sub3(xj, xi), v1 = sub3(xj, xk);
-            const float3 c = cross3(v0, v1);
-            const float rp = sqrtf(dot3(c, c));
-            float3 gi = cross3(v0, c), gk = cross3(c, v1);
-            gi = mul3(gi, -__fdividef(1.f, dot3(v0, v0) * rp + kEpsF));
-            gk = mul3(gk, -__fdividef(1.f, dot3(v1, v1) * rp + kEpsF));
-            const float theta = atan2f(rp, dot3(v0, v1) + kEpsF);
-            const float delta = theta - p.y;
-            ds_add(e, 0.5f * p.x * (delta * delta));
-            const float de = p.x * delta;
-            const float3 fi = mul3(gi, de), fk = mul3(gk, de);
-            add_rec(&G0[ijk.x], fi);
-            sub_rec(&G1[ijk.y], add3(fi, fk));
-            add_rec(&G2[ijk.z], fk);
-        }
-        __syncwarp();
-    }
-    // Fourier dihedrals, impropers then propers (interaction.cpp:76-117, math.cpp:130-167)
-    for (int s = lane; s < t.n_dih_slots; s += kWarp) {
-        const int4 q = __ldg(&t.dih_ijkl[s]);
-        if (q.x >= 0) {
-            const float3 pi = xyz(X[q.x]), pj = xyz(X[q.y]), pk = xyz(X[q.z]), pl = xyz(X[q.w]);
-            const float3 rij = sub3(pj, pi), rkj = sub3(pj, pk), rkl = sub3(pl, pk);
-            const float3 m = cross3(rij, rkj), n = cross3(rkj, rkl);
-            const float3 w = cross3(m, n);
-            const float wlen = sqrtf(dot3(w, w));
-            const float phi = atan2f(wlen, dot3(m, n) + kEpsF);
-            const float theta = dot3(rij, n) < 0.f ? phi : -phi;
-            const float nrkj2 = dot3(rkj, rkj);
-            const float nrkj_1 = __fdividef(1.f, sqrtf(nrkj2) + kEpsF);
-            const float nrkj_2 = nrkj_1 * nrkj_1;
-            const float nrkj = nrkj2 * nrkj_1;
-            // + kEpsF: a collapsed dihedral (m or n = 0, possible in FP32 only for a pose
-            // flung ~1e11 A out of the box, where coordinates resolve to ~1e4 A) gives a zero
-            // gradient instead of 0 * inf = NaN; resolvable geometries are unaffected
-            const float a = -__fdividef(nrkj, dot3(m, m) + kEpsF);
-            const float b = __fdividef(nrkj, dot3(n, n) + kEpsF);
-            const float3 gi = mul3(m, -a), gl = mul3(n, -b);
-            const float pp = dot3(rij, rkj) * nrkj_2, qq = dot3(rkj, rkl) * nrkj_2;
-            const float3 sv = sub3(mul3(gi, pp), mul3(gl, qq));
-            const float3 gj = mul3(sub3(gi, sv), -1.f), gk = mul3(add3(gl, sv), -1.f);
-            const int2 tr = __ldg(&t.dih_terms[s]);
-            float de = 0.f, et = 0.f;
-            for (int u = 0; u < tr.y; ++u) {
-                const float4 term = __ldg(&t.dih_term[tr.x + u]);  // k, periodicity, phase
-                const float delta = theta * term.y - term.z;
-                float sd, cd;
-                __sincosf(delta, &sd, &cd);  // |delta| <= 7 pi: fast path within FP32 parity
-                et += term.x * (1.f + cd);
-                de += term.x * term.y * sd;
-            }
-            ds_add(e, et);
-            add_rec(&G0[q.x], mul3(gi, -de));
-            add_rec(&G1[q.y], mul3(gj, -de));
-            add_rec(&G2[q.z], mul3(gk, -de));
-            add_rec(&G3[q.w], mul3(gl, -de));
-        }
-        __syncwarp();
-    }
-    // 1-4 and all other pairs: Coulomb + LJ 12-6 (interaction.cpp:127-168, pair.h:25-60).
-    // The next round's record is loaded while this round computes, so its L1/L2 latency
-    // is not exposed at the round's barrier (the pair rounds are the most numerous).
-    int2 ij_n = lane < t.n_pair_slots ? __ldg(&t.pair_ij[lane]) : make_int2(-1, -1);
-    float4 p_n = lane < t.n_pair_slots ? __ldg(&t.pair_p[lane]) : make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = lane; s < t.n_pair_slots; s += kWarp) {
-        const int2 ij = ij_n;
-        const float4 pp = p_n;
-        if (s + kWarp < t.n_pair_slots) {
-            ij_n = __ldg(&t.pair_ij[s + kWarp]);
-            p_n = __ldg(&t.pair_p[s + kWarp]);
-        }
-        if (ij.x >= 0) {
-            float en;
-            const float3 g = pair_grad(pp, X[ij.x], X[ij.y], en);
-            ds_add(e, en);
-            sub_rec(&G0[ij.x], g);
-            add_rec(&G1[ij.y], g);
-        }
-        __syncwarp();
-    }
+// A pointer into the block's dynamic shared memory, in the form that the compiler knows as
+// shared memory. The out-of-line evaluation gets generic pointers, and through those every
+// access to a record is a generic load or store: slower, and one that no load from global
+// memory may be moved across.
+extern __shared__ __align__(16) unsigned char pxd_dynamic_smem[];
+template <class T>
+__device__ __forceinline__ T* as_shared(T* p) {
+    const size_t off = __cvta_generic_to_shared(p) - __cvta_generic_to_shared(pxd_dynamic_smem);
+    return reinterpret_cast<T*>(pxd_dynamic_smem + off);
 }
 
-// topo_terms for a team of nw warps (warp w of them), which split the rounds: warp w takes
-// rounds w, w + nw, ... into its own arrays G. Kept apart from topo_terms so that the
-// one-warp kernels compile exactly as before.
-//
 // Adds the bonded and non-bonded terms of `t` over coordinates `X`. The gradient of
 // the atom in position k of a term goes to array k: G[k * gs + atom] (shared memory).
 // Within a round the atoms of each position are distinct (host scheduling), so the
@@ -345,117 +245,203 @@ __device__ __forceinline__ void topo_terms(const DevTopo& t, const float4* X, fl
 // meet every barrier. The caller sums the arrays. Matches
 // intra_molecular_interactions::put_gradients.
 //
-// A team of nw warps (warp w of them) splits the rounds: warp w takes rounds w, w + nw, ...
-// into its own arrays G (nw = 1: every round).
-__device__ __forceinline__ void topo_terms_split(const DevTopo& t, const float4* X, float4* G, int gs, DS& e,
-                                           int lane, int w, int nw) {
-    float4* G0 = G;
-    float4* G1 = G + gs;
-    float4* G2 = G + 2 * gs;
-    float4* G3 = G + 3 * gs;
-    const int first = lane + w * kWarp, step = nw * kWarp;
+// kSplit: a team of nw warps (warp w of them) splits the rounds: warp w takes rounds w, w + nw,
+// ... into its own arrays G.
+//
+// A warp's rounds are a chain of dependent latencies (a few warps per scheduler, or one in a
+// search or a small batch), so the loads are taken off it: the topology's pointers and
+// counts are read once, a round's record is loaded while the round before it computes, the
+// gradient records of a round are loaded together (they lie in different arrays), and a
+// dihedral's first Fourier term travels in its own record, the rest are loaded before its
+// geometry.
+template <bool kSplit>
+__device__ __forceinline__ void topo_terms(const DevTopo& t, const float4* Xg, float4* Gg, int gs, DS& e, int lane,
+                                           int w = 0, int nw = 1) {
+    const float4* X = as_shared(Xg);
+    float4* G0 = as_shared(Gg);
+    float4* G1 = G0 + gs;
+    float4* G2 = G0 + 2 * gs;
+    float4* G3 = G0 + 3 * gs;
+    const int first = kSplit ? lane + w * kWarp : lane;
+    const int step = kSplit ? nw * kWarp : kWarp;
     __syncwarp();
     // harmonic bonds (interaction.cpp:27-47)
-    for (int s = first; s < t.n_bond_slots; s += step) {
-        const int2 ij = __ldg(&t.bond_ij[s]);
-        if (ij.x >= 0) {
-            const float2 p = __ldg(&t.bond_p[s]);
-            const float3 d = sub3(xyz(X[ij.y]), xyz(X[ij.x]));
-            const float r = sqrtf(dot3(d, d));
-            const float dr = r - p.y;
-            ds_add(e, 0.5f * p.x * (dr * dr));
-            const float de_dr = p.x * (1.f - __fdividef(p.y, r + kEpsF));
-            const float3 g = mul3(d, de_dr);
-            sub_rec(&G0[ij.x], g);
-            add_rec(&G1[ij.y], g);
+    {
+        const int n = t.n_bond_slots;
+        const int2* const ids = t.bond_ij;
+        const float2* const par = t.bond_p;
+        int2 ij_n = make_int2(-1, -1);
+        float2 p_n = make_float2(0.f, 0.f);
+        if (first < n) {
+            ij_n = __ldg(&ids[first]);
+            p_n = __ldg(&par[first]);
         }
-        __syncwarp();
+        for (int s = first; s < n; s += step) {
+            const int2 ij = ij_n;
+            const float2 p = p_n;
+            if (s + step < n) {
+                ij_n = __ldg(&ids[s + step]);
+                p_n = __ldg(&par[s + step]);
+            }
+            if (ij.x >= 0) {
+                float4 ri = G0[ij.x], rj = G1[ij.y];
+                const float3 d = sub3(xyz(X[ij.y]), xyz(X[ij.x]));
+                const float r = sqrtf(dot3(d, d));
+                const float dr = r - p.y;
+                ds_add(e, 0.5f * p.x * (dr * dr));
+                const float de_dr = p.x * (1.f - __fdividef(p.y, r + kEpsF));
+                const float3 g = mul3(d, de_dr);
+                sub_rec(ri, g);
+                add_rec(rj, g);
+                G0[ij.x] = ri;
+                G1[ij.y] = rj;
+            }
+            __syncwarp();
+        }
     }
     // harmonic angles (interaction.cpp:49-74, math.cpp:96-110)
-    for (int s = first; s < t.n_angle_slots; s += step) {
-        const int4 ijk = __ldg(&t.angle_ijk[s]);
-        if (ijk.x >= 0) {
-            const float2 p = __ldg(&t.angle_p[s]);
-            const float3 xi = xyz(X[ijk.x]), xj = xyz(X[ijk.y]), xk = xyz(X[ijk.z]);
-            const float3 v0 = sub3(xj, xi), v1 = sub3(xj, xk);
-            const float3 c = cross3(v0, v1);
-            const float rp = sqrtf(dot3(c, c));
-            float3 gi = cross3(v0, c), gk = cross3(c, v1);
-            gi = mul3(gi, -__fdividef(1.f, dot3(v0, v0) * rp + kEpsF));
-            gk = mul3(gk, -__fdividef(1.f, dot3(v1, v1) * rp + kEpsF));
-            const float theta = atan2f(rp, dot3(v0, v1) + kEpsF);
-            const float delta = theta - p.y;
-            ds_add(e, 0.5f * p.x * (delta * delta));
-            const float de = p.x * delta;
-            const float3 fi = mul3(gi, de), fk = mul3(gk, de);
-            add_rec(&G0[ijk.x], fi);
-            sub_rec(&G1[ijk.y], add3(fi, fk));
-            add_rec(&G2[ijk.z], fk);
+    {
+        const int n = t.n_angle_slots;
+        const int4* const ids = t.angle_ijk;
+        const float2* const par = t.angle_p;
+        int4 ijk_n = make_int4(-1, -1, -1, -1);
+        float2 p_n = make_float2(0.f, 0.f);
+        if (first < n) {
+            ijk_n = __ldg(&ids[first]);
+            p_n = __ldg(&par[first]);
         }
-        __syncwarp();
+        for (int s = first; s < n; s += step) {
+            const int4 ijk = ijk_n;
+            const float2 p = p_n;
+            if (s + step < n) {
+                ijk_n = __ldg(&ids[s + step]);
+                p_n = __ldg(&par[s + step]);
+            }
+            if (ijk.x >= 0) {
+                const float3 xi = xyz(X[ijk.x]), xj = xyz(X[ijk.y]), xk = xyz(X[ijk.z]);
+                const float3 v0 = sub3(xj, xi), v1 = sub3(xj, xk);
+                const float3 c = cross3(v0, v1);
+                const float rp = sqrtf(dot3(c, c));
+                float3 gi = cross3(v0, c), gk = cross3(c, v1);
+                gi = mul3(gi, -__fdividef(1.f, dot3(v0, v0) * rp + kEpsF));
+                gk = mul3(gk, -__fdividef(1.f, dot3(v1, v1) * rp + kEpsF));
+                const float theta = atan2f(rp, dot3(v0, v1) + kEpsF);
+                const float delta = theta - p.y;
+                ds_add(e, 0.5f * p.x * (delta * delta));
+                const float de = p.x * delta;
+                const float3 fi = mul3(gi, de), fk = mul3(gk, de);
+                float4 ri = G0[ijk.x], rj = G1[ijk.y], rk = G2[ijk.z];
+                add_rec(ri, fi);
+                sub_rec(rj, add3(fi, fk));
+                add_rec(rk, fk);
+                G0[ijk.x] = ri;
+                G1[ijk.y] = rj;
+                G2[ijk.z] = rk;
+            }
+            __syncwarp();
+        }
     }
     // Fourier dihedrals, impropers then propers (interaction.cpp:76-117, math.cpp:130-167)
-    for (int s = first; s < t.n_dih_slots; s += step) {
-        const int4 q = __ldg(&t.dih_ijkl[s]);
-        if (q.x >= 0) {
-            const float3 pi = xyz(X[q.x]), pj = xyz(X[q.y]), pk = xyz(X[q.z]), pl = xyz(X[q.w]);
-            const float3 rij = sub3(pj, pi), rkj = sub3(pj, pk), rkl = sub3(pl, pk);
-            const float3 m = cross3(rij, rkj), n = cross3(rkj, rkl);
-            const float3 w = cross3(m, n);
-            const float wlen = sqrtf(dot3(w, w));
-            const float phi = atan2f(wlen, dot3(m, n) + kEpsF);
-            const float theta = dot3(rij, n) < 0.f ? phi : -phi;
-            const float nrkj2 = dot3(rkj, rkj);
-            const float nrkj_1 = __fdividef(1.f, sqrtf(nrkj2) + kEpsF);
-            const float nrkj_2 = nrkj_1 * nrkj_1;
-            const float nrkj = nrkj2 * nrkj_1;
-            // + kEpsF: a collapsed dihedral (m or n = 0, possible in FP32 only for a pose
-            // flung ~1e11 A out of the box, where coordinates resolve to ~1e4 A) gives a zero
-            // gradient instead of 0 * inf = NaN; resolvable geometries are unaffected
-            const float a = -__fdividef(nrkj, dot3(m, m) + kEpsF);
-            const float b = __fdividef(nrkj, dot3(n, n) + kEpsF);
-            const float3 gi = mul3(m, -a), gl = mul3(n, -b);
-            const float pp = dot3(rij, rkj) * nrkj_2, qq = dot3(rkj, rkl) * nrkj_2;
-            const float3 sv = sub3(mul3(gi, pp), mul3(gl, qq));
-            const float3 gj = mul3(sub3(gi, sv), -1.f), gk = mul3(add3(gl, sv), -1.f);
-            const int2 tr = __ldg(&t.dih_terms[s]);
-            float de = 0.f, et = 0.f;
-            for (int u = 0; u < tr.y; ++u) {
-                const float4 term = __ldg(&t.dih_term[tr.x + u]);  // k, periodicity, phase
-                const float delta = theta * term.y - term.z;
-                float sd, cd;
-                __sincosf(delta, &sd, &cd);  // |delta| <= 7 pi: fast path within FP32 parity
-                et += term.x * (1.f + cd);
-                de += term.x * term.y * sd;
+    {
+        const int n = t.n_dih_slots;
+        const int4* const ids = t.dih_ijkl;
+        const float4* const heads = t.dih_first;
+        const float4* const terms = t.dih_term;
+        int4 q_n = make_int4(-1, -1, -1, -1);
+        float4 h_n = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (first < n) {
+            q_n = __ldg(&ids[first]);
+            h_n = __ldg(&heads[first]);
+        }
+        for (int s = first; s < n; s += step) {
+            const int4 q = q_n;
+            const float4 head = h_n;
+            if (s + step < n) {
+                q_n = __ldg(&ids[s + step]);
+                h_n = __ldg(&heads[s + step]);
             }
-            ds_add(e, et);
-            add_rec(&G0[q.x], mul3(gi, -de));
-            add_rec(&G1[q.y], mul3(gj, -de));
-            add_rec(&G2[q.z], mul3(gk, -de));
-            add_rec(&G3[q.w], mul3(gl, -de));
+            if (q.x >= 0) {
+                const int where = __float_as_int(head.w);
+                const int at = where & kDihFirstMask, count = where >> kDihCountShift;
+                float4 t1 = head, t2 = head;  // the second and third terms, in flight meanwhile
+                if (count > 1) t1 = __ldg(&terms[at + 1]);
+                if (count > 2) t2 = __ldg(&terms[at + 2]);
+                const float3 pi = xyz(X[q.x]), pj = xyz(X[q.y]), pk = xyz(X[q.z]), pl = xyz(X[q.w]);
+                const float3 rij = sub3(pj, pi), rkj = sub3(pj, pk), rkl = sub3(pl, pk);
+                const float3 m = cross3(rij, rkj), nv = cross3(rkj, rkl);
+                const float3 wv = cross3(m, nv);
+                const float wlen = sqrtf(dot3(wv, wv));
+                const float phi = atan2f(wlen, dot3(m, nv) + kEpsF);
+                const float theta = dot3(rij, nv) < 0.f ? phi : -phi;
+                const float nrkj2 = dot3(rkj, rkj);
+                const float nrkj_1 = __fdividef(1.f, sqrtf(nrkj2) + kEpsF);
+                const float nrkj_2 = nrkj_1 * nrkj_1;
+                const float nrkj = nrkj2 * nrkj_1;
+                // + kEpsF: a collapsed dihedral (m or n = 0, possible in FP32 only for a pose
+                // flung ~1e11 A out of the box, where coordinates resolve to ~1e4 A) gives a zero
+                // gradient instead of 0 * inf = NaN; resolvable geometries are unaffected
+                const float a = -__fdividef(nrkj, dot3(m, m) + kEpsF);
+                const float b = __fdividef(nrkj, dot3(nv, nv) + kEpsF);
+                const float3 gi = mul3(m, -a), gl = mul3(nv, -b);
+                const float pp = dot3(rij, rkj) * nrkj_2, qq = dot3(rkj, rkl) * nrkj_2;
+                const float3 sv = sub3(mul3(gi, pp), mul3(gl, qq));
+                const float3 gj = mul3(sub3(gi, sv), -1.f), gk = mul3(add3(gl, sv), -1.f);
+                float de = 0.f, et = 0.f;
+                auto add_term = [theta, &de, &et](float4 term) {  // k, periodicity, phase
+                    const float delta = theta * term.y - term.z;
+                    float sd, cd;
+                    __sincosf(delta, &sd, &cd);  // |delta| <= 7 pi: fast path within FP32 parity
+                    et += term.x * (1.f + cd);
+                    de += term.x * term.y * sd;
+                };
+                if (count > 0) add_term(head);
+                if (count > 1) add_term(t1);
+                if (count > 2) add_term(t2);
+                for (int u = 3; u < count; ++u) add_term(__ldg(&terms[at + u]));
+                ds_add(e, et);
+                float4 ri = G0[q.x], rj = G1[q.y], rk = G2[q.z], rl = G3[q.w];
+                add_rec(ri, mul3(gi, -de));
+                add_rec(rj, mul3(gj, -de));
+                add_rec(rk, mul3(gk, -de));
+                add_rec(rl, mul3(gl, -de));
+                G0[q.x] = ri;
+                G1[q.y] = rj;
+                G2[q.z] = rk;
+                G3[q.w] = rl;
+            }
+            __syncwarp();
         }
-        __syncwarp();
     }
-    // 1-4 and all other pairs: Coulomb + LJ 12-6 (interaction.cpp:127-168, pair.h:25-60).
-    // The next round's record is loaded while this round computes, so its L1/L2 latency
-    // is not exposed at the round's barrier (the pair rounds are the most numerous).
-    int2 ij_n = first < t.n_pair_slots ? __ldg(&t.pair_ij[first]) : make_int2(-1, -1);
-    float4 p_n = first < t.n_pair_slots ? __ldg(&t.pair_p[first]) : make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = first; s < t.n_pair_slots; s += step) {
-        const int2 ij = ij_n;
-        const float4 pp = p_n;
-        if (s + step < t.n_pair_slots) {
-            ij_n = __ldg(&t.pair_ij[s + step]);
-            p_n = __ldg(&t.pair_p[s + step]);
+    // 1-4 and all other pairs: Coulomb + LJ 12-6 (interaction.cpp:127-168, pair.h:25-60)
+    {
+        const int n = t.n_pair_slots;
+        const int2* const ids = t.pair_ij;
+        const float4* const par = t.pair_p;
+        int2 ij_n = make_int2(-1, -1);
+        float4 p_n = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (first < n) {
+            ij_n = __ldg(&ids[first]);
+            p_n = __ldg(&par[first]);
         }
-        if (ij.x >= 0) {
-            float en;
-            const float3 g = pair_grad(pp, X[ij.x], X[ij.y], en);
-            ds_add(e, en);
-            sub_rec(&G0[ij.x], g);
-            add_rec(&G1[ij.y], g);
+        for (int s = first; s < n; s += step) {
+            const int2 ij = ij_n;
+            const float4 p = p_n;
+            if (s + step < n) {
+                ij_n = __ldg(&ids[s + step]);
+                p_n = __ldg(&par[s + step]);
+            }
+            if (ij.x >= 0) {
+                float4 ri = G0[ij.x], rj = G1[ij.y];
+                float en;
+                const float3 g = pair_grad(p, X[ij.x], X[ij.y], en);
+                ds_add(e, en);
+                sub_rec(ri, g);
+                add_rec(rj, g);
+                G0[ij.x] = ri;
+                G1[ij.y] = rj;
+            }
+            __syncwarp();
         }
-        __syncwarp();
     }
 }
 
@@ -611,9 +597,17 @@ struct EvalEnv {
 // directional derivative), accumulated while the flat gradient is written. Replaces
 // binding_system_interactions::put_gradients as the optimiser's closure calls it
 // (optimizer.cpp:155-167).
-__device__ __forceinline__ double eval_pose_body(const EvalEnv& env, const DevLigand& L, const float* x0,
-                                                const float* d, float t, float* gout, const PoseBufs& b,
-                                                int lane, const float* gdir = nullptr, double* gdot = nullptr) {
+//
+// Every vector and buffer argument lies in the block's dynamic shared memory (as_shared).
+__device__ __forceinline__ double eval_pose_body(const EvalEnv& env, const DevLigand& L, const float* x0g,
+                                                const float* dg, float t, float* goutg, const PoseBufs& bg,
+                                                int lane, const float* gdirg = nullptr, double* gdot = nullptr) {
+    const PoseBufs b{as_shared(bg.lig_xyz), as_shared(bg.lig_grad), as_shared(bg.loc_xyz), as_shared(bg.loc_grad),
+                     as_shared(bg.mov_jac), bg.lig_gs, bg.loc_gs};
+    const float* const x0 = as_shared(x0g);
+    const float* const d = dg ? as_shared(dg) : nullptr;
+    float* const gout = as_shared(goutg);
+    const float* const gdir = gdirg ? as_shared(gdirg) : nullptr;
     const int N = L.n_atoms;
     const int n3 = 3 * N;
     const DevReceptor& R = env.rec;
@@ -650,8 +644,8 @@ __device__ __forceinline__ double eval_pose_body(const EvalEnv& env, const DevLi
     }
     __syncwarp();
     DS e{0.f, 0.f};
-    topo_terms(L.topo, b.lig_xyz, b.lig_grad, b.lig_gs, e, lane);
-    if (R.n_local > 0) topo_terms(R.intra, b.loc_xyz, b.loc_grad, b.loc_gs, e, lane);
+    topo_terms<false>(L.topo, b.lig_xyz, b.lig_grad, b.lig_gs, e, lane);
+    if (R.n_local > 0) topo_terms<false>(R.intra, b.loc_xyz, b.loc_grad, b.loc_gs, e, lane);
     // grid lookups (inter_molecular_interactions, cached branch)
     if (env.grid.has_grid) {
         for (int a = lane; a < N; a += kWarp) {
@@ -659,9 +653,9 @@ __device__ __forceinline__ double eval_pose_body(const EvalEnv& env, const DevLi
             const float ea = grid_lookup(env.grid, __ldg(&L.map_slot[a]), __ldg(&L.charge[a]),
                                          xyz(b.lig_xyz[a]), g);
             ds_add(e, ea);
-            add_rec(&b.lig_grad[a], g);  // one lane per atom; topo_terms ended on a barrier
+            add_rec(b.lig_grad[a], g);  // one lane per atom; topo_terms ended on a barrier
         }
-        __syncwarp();  // the explicit pairs below add to the same records atomically
+        __syncwarp();  // the explicit pairs below add to the same records
     }
     // explicit inter pairs (rotor atoms with maps, every receptor atom without)
     const int M = R.n_explicit;
@@ -689,18 +683,20 @@ __device__ __forceinline__ double eval_pose_body(const EvalEnv& env, const DevLi
                 ds_add(e, C * (u12 - u6));
                 const float3 g = mul3(rij, (C * (6.f * u6 - 12.f * u12) - ec) * rinv2);
                 gi = sub3(gi, g);
-                if (loc >= 0) atomic_add3(&b.loc_grad[loc], g);
+                if (loc >= 0) add_rec(b.loc_grad[loc], g);  // one lane per receptor atom
             }
             gi.x = warp_sum_f(gi.x);
             gi.y = warp_sum_f(gi.y);
             gi.z = warp_sum_f(gi.z);
-            if (lane == 0) atomic_add3(&b.lig_grad[i], gi);
+            if (lane == 0) add_rec(b.lig_grad[i], gi);
         }
     } else if (M > 0) {
-        for (int i = lane; i < N; i += kWarp) {
-            const float3 xi = xyz(b.lig_xyz[i]);
-            const float qi = __ldg(&L.charge[i]);
-            const float2 sei = __ldg(&L.se[i]);
+        for (int i0 = 0; i0 < N; i0 += kWarp) {
+            const int i = i0 + lane, n = min(N - i0, kWarp);
+            const bool on = lane < n;
+            const float3 xi = on ? xyz(b.lig_xyz[i]) : make_float3(0.f, 0.f, 0.f);
+            const float qi = on ? __ldg(&L.charge[i]) : 0.f;
+            const float2 sei = on ? __ldg(&L.se[i]) : make_float2(0.f, 0.f);
             float3 gi = make_float3(0.f, 0.f, 0.f);
             for (int j = 0; j < M; ++j) {
                 const int loc = __ldg(&R.ex_local[j]);
@@ -716,13 +712,16 @@ __device__ __forceinline__ double eval_pose_body(const EvalEnv& env, const DevLi
                 const float u6 = xx * xx * xx, u12 = u6 * u6;
                 const float C = sqrtf(sei.y * sej.y) * 4.f;
                 const float ec = kCoulombF * qi * rj.w * rinv;
-                ds_add(e, ec);
-                ds_add(e, C * (u12 - u6));
                 const float3 g = mul3(rij, (C * (6.f * u6 - 12.f * u12) - ec) * rinv2);
-                gi = sub3(gi, g);
-                if (loc >= 0) atomic_add3(&b.loc_grad[loc], g);
+                if (on) {
+                    ds_add(e, ec);
+                    ds_add(e, C * (u12 - u6));
+                    gi = sub3(gi, g);
+                }
+                if (loc >= 0) add_lanes(&b.loc_grad[loc], g, n, lane);
             }
-            atomic_add3(&b.lig_grad[i], gi);
+            if (on) add_rec(b.lig_grad[i], gi);
+            __syncwarp();
         }
     }
     __syncwarp();
@@ -764,9 +763,15 @@ __device__ __forceinline__ double eval_pose_body(const EvalEnv& env, const DevLi
 // eval_pose_body for a team of warps (Team): the members split the terms, lookups and
 // explicit pairs and sum each other's parts in member order. Kept apart from
 // eval_pose_body so that the one-warp kernels compile exactly as before.
-__device__ __forceinline__ double eval_pose_team_body(const EvalEnv& env, const DevLigand& L, const float* x0,
-                                                     const float* d, float t, float* gout, const PoseBufs& b,
-                                                     int lane, const float* gdir, double* gdot, const Team* team) {
+__device__ __forceinline__ double eval_pose_team_body(const EvalEnv& env, const DevLigand& L, const float* x0g,
+                                                     const float* dg, float t, float* goutg, const PoseBufs& bg,
+                                                     int lane, const float* gdirg, double* gdot, const Team* team) {
+    const PoseBufs b{as_shared(bg.lig_xyz), as_shared(bg.lig_grad), as_shared(bg.loc_xyz), as_shared(bg.loc_grad),
+                     as_shared(bg.mov_jac), bg.lig_gs, bg.loc_gs};
+    const float* const x0 = as_shared(x0g);
+    const float* const d = dg ? as_shared(dg) : nullptr;
+    float* const gout = as_shared(goutg);
+    const float* const gdir = gdirg ? as_shared(gdirg) : nullptr;
     const int N = L.n_atoms;
     const int n3 = 3 * N;
     const DevReceptor& R = env.rec;
@@ -807,8 +812,8 @@ __device__ __forceinline__ double eval_pose_team_body(const EvalEnv& env, const 
     const int tf4 = team->f4;
     TeamShared* ts = team->ts;
     DS e{0.f, 0.f};
-    topo_terms_split(L.topo, b.lig_xyz, b.lig_grad, b.lig_gs, e, lane, tw, tn);
-    if (R.n_local > 0) topo_terms_split(R.intra, b.loc_xyz, b.loc_grad, b.loc_gs, e, lane, tw, tn);
+    topo_terms<true>(L.topo, b.lig_xyz, b.lig_grad, b.lig_gs, e, lane, tw, tn);
+    if (R.n_local > 0) topo_terms<true>(R.intra, b.loc_xyz, b.loc_grad, b.loc_gs, e, lane, tw, tn);
     // grid lookups (inter_molecular_interactions, cached branch)
     if (env.grid.has_grid) {
         for (int a = lane + tw * kWarp; a < N; a += tn * kWarp) {
@@ -816,9 +821,9 @@ __device__ __forceinline__ double eval_pose_team_body(const EvalEnv& env, const 
             const float ea = grid_lookup(env.grid, __ldg(&L.map_slot[a]), __ldg(&L.charge[a]),
                                          xyz(b.lig_xyz[a]), g);
             ds_add(e, ea);
-            add_rec(&b.lig_grad[a], g);  // one lane per atom; topo_terms ended on a barrier
+            add_rec(b.lig_grad[a], g);  // one lane per atom; topo_terms ended on a barrier
         }
-        __syncwarp();  // the explicit pairs below add to the same records atomically
+        __syncwarp();  // the explicit pairs below add to the same records
     }
     // explicit inter pairs (rotor atoms with maps, every receptor atom without)
     const int M = R.n_explicit;
@@ -846,18 +851,20 @@ __device__ __forceinline__ double eval_pose_team_body(const EvalEnv& env, const 
                 ds_add(e, C * (u12 - u6));
                 const float3 g = mul3(rij, (C * (6.f * u6 - 12.f * u12) - ec) * rinv2);
                 gi = sub3(gi, g);
-                if (loc >= 0) atomic_add3(&b.loc_grad[loc], g);
+                if (loc >= 0) add_rec(b.loc_grad[loc], g);  // one lane per receptor atom
             }
             gi.x = warp_sum_f(gi.x);
             gi.y = warp_sum_f(gi.y);
             gi.z = warp_sum_f(gi.z);
-            if (lane == 0) atomic_add3(&b.lig_grad[i], gi);
+            if (lane == 0) add_rec(b.lig_grad[i], gi);
         }
     } else if (M > 0) {
-        for (int i = lane + tw * kWarp; i < N; i += tn * kWarp) {
-            const float3 xi = xyz(b.lig_xyz[i]);
-            const float qi = __ldg(&L.charge[i]);
-            const float2 sei = __ldg(&L.se[i]);
+        for (int i0 = tw * kWarp; i0 < N; i0 += tn * kWarp) {
+            const int i = i0 + lane, n = min(N - i0, kWarp);
+            const bool on = lane < n;
+            const float3 xi = on ? xyz(b.lig_xyz[i]) : make_float3(0.f, 0.f, 0.f);
+            const float qi = on ? __ldg(&L.charge[i]) : 0.f;
+            const float2 sei = on ? __ldg(&L.se[i]) : make_float2(0.f, 0.f);
             float3 gi = make_float3(0.f, 0.f, 0.f);
             for (int j = 0; j < M; ++j) {
                 const int loc = __ldg(&R.ex_local[j]);
@@ -873,13 +880,16 @@ __device__ __forceinline__ double eval_pose_team_body(const EvalEnv& env, const 
                 const float u6 = xx * xx * xx, u12 = u6 * u6;
                 const float C = sqrtf(sei.y * sej.y) * 4.f;
                 const float ec = kCoulombF * qi * rj.w * rinv;
-                ds_add(e, ec);
-                ds_add(e, C * (u12 - u6));
                 const float3 g = mul3(rij, (C * (6.f * u6 - 12.f * u12) - ec) * rinv2);
-                gi = sub3(gi, g);
-                if (loc >= 0) atomic_add3(&b.loc_grad[loc], g);
+                if (on) {
+                    ds_add(e, ec);
+                    ds_add(e, C * (u12 - u6));
+                    gi = sub3(gi, g);
+                }
+                if (loc >= 0) add_lanes(&b.loc_grad[loc], g, n, lane);
             }
-            atomic_add3(&b.lig_grad[i], gi);
+            if (on) add_rec(b.lig_grad[i], gi);
+            __syncwarp();
         }
     }
     __syncwarp();

@@ -278,20 +278,18 @@ static __device__ void strong_wolfe(Cl& c, const LbfgsConsts& p, const float* d,
 // its SM (the single-walker search) waits on. Lane-element order, products and accumulation
 // are those of the shared-vector loops, so the result is the same bit for bit. kF32: the
 // coefficients in FP32 (see lbfgs_pose). Writes g_prev = g and d; returns g . d.
-// Dot product of a lane's E register elements (x[j] * y[j] where lane + 32 j < D) with
-// the products' exact errors, summed as a pairwise two-sum tree (depth log2 E instead of E
-// dependent compensated additions), rounded once to FP32, then summed over the warp by a
-// plain FP32 butterfly: the same value on every lane. The single-walker search's two-loop
-// dot products, whose dependent chain is what a warp alone on its SM waits on.
+// Dot product of a lane's E register elements (zero past D) with the products' exact
+// errors, summed as a pairwise two-sum tree (depth log2 E instead of E dependent compensated
+// additions), rounded once to FP32, then summed over the warp by a plain FP32 butterfly: the
+// same value on every lane. The single-walker search's two-loop dot products, whose
+// dependent chain is what a warp alone on its SM waits on.
 template <int E>
-__device__ __forceinline__ float lane_tree_warp_dot(const float* x, const float* y, int lane, int D) {
+__device__ __forceinline__ float lane_tree_warp_dot(const float* x, const float* y) {
     float p[E], pe = 0.f;
 #pragma unroll
     for (int j = 0; j < E; ++j) {
-        const bool ok = lane + j * kWarp < D;
-        const float a = ok ? x[j] : 0.f, b = ok ? y[j] : 0.f;
-        p[j] = a * b;
-        pe += fmaf(a, b, -p[j]);
+        p[j] = x[j] * y[j];
+        pe += fmaf(x[j], y[j], -p[j]);
     }
 #pragma unroll
     for (int w = 1; w < E; w *= 2) {
@@ -309,72 +307,108 @@ __device__ __forceinline__ float lane_tree_warp_dot(const float* x, const float*
     return f;
 }
 
+// A lane's E elements (lane + 32 j) of a history vector; v points at element `lane`.
+template <int E>
+__device__ __forceinline__ void load_lane(float* x, const float* v) {
+#pragma unroll
+    for (int j = 0; j < E; ++j) x[j] = v[j * kWarp];
+}
+
 // two_loop_regs with FP32 coefficients and the per-pass dot products of
 // lane_tree_warp_dot (the single-walker search). Writes g_prev = g and d; returns g . d.
+//
+// A warp alone on its SM waits on each pass's chain: dot product, coefficient, axpy. The
+// vectors and the rho of the next pass are therefore loaded while a pass runs, so that
+// neither L1 / L2 latency nor the FP64-to-FP32 conversion of rho is on the chain, and E is
+// the count of elements that holds D exactly (a 43-atom ligand's 129 need 5, not 8), the
+// last row of the history zero past D, so that no element needs a bounds test.
 template <int E>
-static __device__ __forceinline__ double two_loop_regs_tree(const Vecs& v, int base, int count, int slots,
-                                                            size_t Dp, int D, int lane, float hd) {
-    float r[E], xv[E];
+static __device__ __noinline__ double two_loop_regs_tree(const Vecs& vg, int base, int count, int slots, int Dp,
+                                                         int D, int lane, float hd) {
+    const float* const S = vg.S + lane;
+    const float* const Y = vg.Y + lane;
+    const float* const g = as_shared(vg.g);
+    float* const gp = as_shared(vg.gp);
+    float* const dir = as_shared(vg.d);
+    const double* const ro = as_shared(vg.ro);
+    float* const alf = reinterpret_cast<float*>(as_shared(vg.al));
+    auto older = [slots](int sl) { return sl == 0 ? slots - 1 : sl - 1; };
+    auto newer = [slots](int sl) { return sl + 1 == slots ? 0 : sl + 1; };
+    float r[E], xv[E], yv[E], xn[E], yn[E];
     int sl = base + count - 1 >= slots ? base + count - 1 - slots : base + count - 1;
-    {
-        const float* sk = v.S + sl * Dp;
+    load_lane<E>(xv, S + sl * Dp);
+    load_lane<E>(yv, Y + sl * Dp);
 #pragma unroll
-        for (int j = 0; j < E; ++j) {
-            const int e = lane + j * kWarp;
-            r[j] = 0.f;
-            xv[j] = 0.f;
-            if (e < D) {
-                const float ge = v.g[e];
-                r[j] = -ge;
-                v.gp[e] = ge;
-                xv[j] = sk[e];
-            }
+    for (int j = 0; j < E; ++j) {
+        const int e = lane + j * kWarp;
+        r[j] = 0.f;
+        if (e < D) {
+            const float ge = g[e];
+            r[j] = -ge;
+            gp[e] = ge;
         }
     }
-    float dot = lane_tree_warp_dot<E>(xv, r, lane, D);
-    float* alf = reinterpret_cast<float*>(v.al);
+    float rho = static_cast<float>(ro[sl]);
+    float dot = lane_tree_warp_dot<E>(xv, r);
+    int next = older(sl);
+    if (count > 1) load_lane<E>(xv, S + next * Dp);
     for (int k = count - 1; k >= 0; --k) {
-        const float* yk = v.Y + sl * Dp;
-        const int sn_slot = sl == 0 ? slots - 1 : sl - 1;
-        const float* sn = v.S + sn_slot * Dp;
-        float yv[E];
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-            const int e = lane + j * kWarp;
-            yv[j] = e < D ? yk[e] : 0.f;
-            xv[j] = e < D && k > 0 ? sn[e] : 0.f;
+        // for the pass after this one: y of the next older pair, s of the one before that
+        const int after = older(next);
+        float rho_n = 0.f;
+        if (k > 0) {
+            rho_n = static_cast<float>(ro[next]);
+            load_lane<E>(yn, Y + next * Dp);
         }
-        const float a = dot * static_cast<float>(v.ro[sl]);
+        if (k > 1) load_lane<E>(xn, S + after * Dp);
+        const float a = dot * rho;
         alf[k] = a;  // every lane holds the same value
 #pragma unroll
         for (int j = 0; j < E; ++j) r[j] = fmaf(yv[j], -a, r[j]);
         if (k > 0) {
-            dot = lane_tree_warp_dot<E>(xv, r, lane, D);
+            dot = lane_tree_warp_dot<E>(xv, r);
+            rho = rho_n;
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                xv[j] = xn[j];
+                yv[j] = yn[j];
+            }
+            next = after;
         } else {
+            // the second loop starts with the oldest pair: its s is loaded before its dot
+            load_lane<E>(xv, S + base * Dp);
 #pragma unroll
             for (int j = 0; j < E; ++j) r[j] *= hd;
-            dot = lane_tree_warp_dot<E>(yv, r, lane, D);
+            dot = lane_tree_warp_dot<E>(yv, r);
         }
-        sl = sn_slot;
     }
     __syncwarp();
+    // second loop: xv = s of the pair, yv = y of the next newer pair (the gradient after the last)
     sl = base;
+    rho = static_cast<float>(ro[sl]);
+    next = newer(sl);
+    if (count > 1) load_lane<E>(yv, Y + next * Dp);
     for (int k = 0; k < count; ++k) {
-        const float* sk = v.S + sl * Dp;
-        const int nx_slot = sl + 1 == slots ? 0 : sl + 1;
-        const float* nx = k + 1 < count ? v.Y + nx_slot * Dp : v.g;
-        float sv[E];
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-            const int e = lane + j * kWarp;
-            sv[j] = e < D ? sk[e] : 0.f;
-            xv[j] = e < D ? nx[e] : 0.f;
+        const int after = newer(next);
+        float rho_n = 0.f;
+        if (k + 1 < count) {
+            rho_n = static_cast<float>(ro[next]);
+            load_lane<E>(xn, S + next * Dp);
         }
-        const float w = alf[k] - dot * static_cast<float>(v.ro[sl]);
+        if (k + 2 < count) load_lane<E>(yn, Y + after * Dp);
+        const float w = alf[k] - dot * rho;
 #pragma unroll
-        for (int j = 0; j < E; ++j) r[j] = fmaf(sv[j], w, r[j]);
-        if (k + 1 < count) dot = lane_tree_warp_dot<E>(xv, r, lane, D);
-        sl = nx_slot;
+        for (int j = 0; j < E; ++j) r[j] = fmaf(xv[j], w, r[j]);
+        if (k + 1 < count) {
+            dot = lane_tree_warp_dot<E>(yv, r);
+            rho = rho_n;
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                xv[j] = xn[j];
+                yv[j] = yn[j];
+            }
+            next = after;
+        }
     }
     // g . d for the line search, compensated as elsewhere
     DS acc{0.f, 0.f};
@@ -382,15 +416,30 @@ static __device__ __forceinline__ double two_loop_regs_tree(const Vecs& v, int b
     for (int j = 0; j < E; ++j) {
         const int e = lane + j * kWarp;
         if (e < D) {
-            v.d[e] = r[j];
-            ds_dot_acc(acc, v.g[e], r[j]);
+            dir[e] = r[j];
+            ds_dot_acc(acc, g[e], r[j]);
         }
     }
     __syncwarp();
     return ds_warp_sum(acc);
 }
 
-template <int E, bool kF32>
+// two_loop_regs_tree for a direction of E * 32 elements, E = 1 .. 8.
+static __device__ __forceinline__ double two_loop_tree(int E, const Vecs& v, int base, int count, int slots, int Dp,
+                                                       int D, int lane, float hd) {
+    switch (E) {
+        case 1: return two_loop_regs_tree<1>(v, base, count, slots, Dp, D, lane, hd);
+        case 2: return two_loop_regs_tree<2>(v, base, count, slots, Dp, D, lane, hd);
+        case 3: return two_loop_regs_tree<3>(v, base, count, slots, Dp, D, lane, hd);
+        case 4: return two_loop_regs_tree<4>(v, base, count, slots, Dp, D, lane, hd);
+        case 5: return two_loop_regs_tree<5>(v, base, count, slots, Dp, D, lane, hd);
+        case 6: return two_loop_regs_tree<6>(v, base, count, slots, Dp, D, lane, hd);
+        case 7: return two_loop_regs_tree<7>(v, base, count, slots, Dp, D, lane, hd);
+        default: return two_loop_regs_tree<8>(v, base, count, slots, Dp, D, lane, hd);
+    }
+}
+
+template <int E>
 static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, int count, int slots,
                                                        size_t Dp, int D, int lane, float hd) {
     float r[E];
@@ -410,7 +459,6 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
             }
         }
     }
-    float* alf = reinterpret_cast<float*>(v.al);
     for (int k = count - 1; k >= 0; --k) {
         const float* yk = v.Y + sl * Dp;
         const int sn_slot = sl == 0 ? slots - 1 : sl - 1;
@@ -422,16 +470,9 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
             yv[j] = e < D ? yk[e] : 0.f;
             sv[j] = e < D && k > 0 ? sn[e] : 0.f;
         }
-        float nal;
-        if constexpr (kF32) {
-            const float a = ds_warp_sum_f(acc) * static_cast<float>(v.ro[sl]);
-            if (lane == 0) alf[k] = a;
-            nal = -a;
-        } else {
-            const double al = ds_warp_sum(acc) * v.ro[sl];
-            if (lane == 0) v.al[k] = al;
-            nal = static_cast<float>(-al);
-        }
+        const double al = ds_warp_sum(acc) * v.ro[sl];
+        if (lane == 0) v.al[k] = al;
+        const float nal = static_cast<float>(-al);
         acc = DS{0.f, 0.f};
         if (k > 0) {
 #pragma unroll
@@ -452,7 +493,7 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
         }
         sl = sn_slot;
     }
-    __syncwarp();  // alf written by lane 0 above, read by every lane below
+    __syncwarp();  // al written by lane 0 above, read by every lane below
     sl = base;
     for (int k = 0; k < count; ++k) {
         const float* sk = v.S + sl * Dp;
@@ -465,11 +506,7 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
             sv[j] = e < D ? sk[e] : 0.f;
             nv[j] = e < D ? nx[e] : 0.f;
         }
-        float w;
-        if constexpr (kF32)
-            w = alf[k] - ds_warp_sum_f(acc) * static_cast<float>(v.ro[sl]);
-        else
-            w = static_cast<float>(v.al[k] - ds_warp_sum(acc) * v.ro[sl]);
+        const float w = static_cast<float>(v.al[k] - ds_warp_sum(acc) * v.ro[sl]);
         acc = DS{0.f, 0.f};
 #pragma unroll
         for (int j = 0; j < E; ++j) {
@@ -529,6 +566,10 @@ static __device__ int lbfgs_pose(Cl& c, const LbfgsConsts& p, const Vecs& v, int
                 ds_dot_acc(a_ys, y, sv);
                 ds_dot_acc(a_yy, y, y);
             }
+            if constexpr (kFast) {  // two_loop_regs_tree reads whole rows
+                const int e = (D - 1) / kWarp * kWarp + lane;
+                if (e >= D) ys_[e] = ss_[e] = 0.f;
+            }
             reset = warp_max(ymax) > p.reset;
             if (!reset) {
                 const double ys = ds_warp_sum(a_ys);
@@ -569,17 +610,15 @@ static __device__ int lbfgs_pose(Cl& c, const LbfgsConsts& p, const Vecs& v, int
             } else {
                 S.t = p.lr;
             }
-        } else if (kFast && D <= 4 * kWarp) {
-            gtd = two_loop_regs_tree<4>(v, S.base, S.count, slots, Dp, D, lane, static_cast<float>(S.H_diag));
-            S.t = p.lr;
         } else if (kFast && D <= 8 * kWarp) {
-            gtd = two_loop_regs_tree<8>(v, S.base, S.count, slots, Dp, D, lane, static_cast<float>(S.H_diag));
+            gtd = two_loop_tree((D + kWarp - 1) / kWarp, v, S.base, S.count, slots, static_cast<int>(Dp), D, lane,
+                                static_cast<float>(S.H_diag));
             S.t = p.lr;
         } else if (kRegLoop && D <= 4 * kWarp) {
-            gtd = two_loop_regs<4, kFast>(v, S.base, S.count, slots, Dp, D, lane, static_cast<float>(S.H_diag));
+            gtd = two_loop_regs<4>(v, S.base, S.count, slots, Dp, D, lane, static_cast<float>(S.H_diag));
             S.t = p.lr;
         } else if (kRegLoop && D <= 8 * kWarp) {
-            gtd = two_loop_regs<8, kFast>(v, S.base, S.count, slots, Dp, D, lane, static_cast<float>(S.H_diag));
+            gtd = two_loop_regs<8>(v, S.base, S.count, slots, Dp, D, lane, static_cast<float>(S.H_diag));
             S.t = p.lr;
         } else {
             // first loop, newest to oldest: q = -g - sum al_k y_k. The ring's base and count

@@ -25,6 +25,8 @@ namespace pxd {
 
 constexpr int kWarp = 32;
 constexpr int kMaxDihTerms = 6;
+// dih_first[s].w as int bits: first term (low bits) and number of terms (high bits)
+constexpr int kDihCountShift = 24, kDihFirstMask = (1 << kDihCountShift) - 1;
 
 // Molecule terms on the device (ligand, or the receptor's rotor-touching terms).
 struct DevTopo {
@@ -37,6 +39,7 @@ struct DevTopo {
     const int4* dih_ijkl;
     const int2* dih_terms;    // first term, number of terms
     const float4* dih_term;   // k, periodicity, phase, -
+    const float4* dih_first;  // per slot: its first term and, in .w, where and how many (kDihFirstMask)
     const int2* pair_ij;
     const float4* pair_p;     // A = 332.06 qi qj s_c, C = 4 sqrt(ei ej) s_v, S2 = ((si+sj)/2)^2
     // the parameters' remainders below their FP32 values, slot for slot, for the reported

@@ -317,14 +317,22 @@ __device__ __forceinline__ void load_lane(float* x, const float* v) {
 // two_loop_regs with FP32 coefficients and the per-pass dot products of
 // lane_tree_warp_dot (the single-walker search). Writes g_prev = g and d; returns g . d.
 //
-// A warp alone on its SM waits on each pass's chain: dot product, coefficient, axpy. The
-// vectors and the rho of the next pass are therefore loaded while a pass runs, so that
-// neither L1 / L2 latency nor the FP64-to-FP32 conversion of rho is on the chain, and E is
-// the count of elements that holds D exactly (a 43-atom ligand's 129 need 5, not 8), the
-// last row of the history zero past D, so that no element needs a bounds test.
+// A warp alone on its SM waits on each pass's chain: dot product, coefficient, axpy (~230
+// cycles, 150 of them the warp sum's shuffles). The vectors, rho and coefficient of a pass are
+// therefore loaded two passes ahead into three sets of registers that take turns, so that
+// neither the L2 latency of a long history nor the FP64-to-FP32 conversion of rho is on the
+// chain, and a pass has one branch. E is the count of elements that holds D exactly (a
+// 43-atom ligand's 129 need 5, not 8), the last row of the history zero past D, so that no
+// element needs a bounds test.
+template <int E>
+struct TwoLoopStage {
+    float x[E], y[E], rho, al;
+};
+
 template <int E>
 static __device__ __noinline__ double two_loop_regs_tree(const Vecs& vg, int base, int count, int slots, int Dp,
                                                          int D, int lane, float hd) {
+    using Stage = TwoLoopStage<E>;
     const float* const S = vg.S + lane;
     const float* const Y = vg.Y + lane;
     const float* const g = as_shared(vg.g);
@@ -332,12 +340,20 @@ static __device__ __noinline__ double two_loop_regs_tree(const Vecs& vg, int bas
     float* const dir = as_shared(vg.d);
     const double* const ro = as_shared(vg.ro);
     float* const alf = reinterpret_cast<float*>(as_shared(vg.al));
-    auto older = [slots](int sl) { return sl == 0 ? slots - 1 : sl - 1; };
-    auto newer = [slots](int sl) { return sl + 1 == slots ? 0 : sl + 1; };
-    float r[E], xv[E], yv[E], xn[E], yn[E];
-    int sl = base + count - 1 >= slots ? base + count - 1 - slots : base + count - 1;
-    load_lane<E>(xv, S + sl * Dp);
-    load_lane<E>(yv, Y + sl * Dp);
+    float r[E], dot = 0.f;
+    // first loop, newest to oldest. Pass k takes y_k and, for the dot of the pass after it,
+    // s_{k-1}; passes are loaded in order, the slots past the oldest pair without use.
+    int slot = base + count - 1 >= slots ? base + count - 1 - slots : base + count - 1;
+    auto load_back = [&](Stage& t) {  // y of `slot`, s of the next older one
+        load_lane<E>(t.y, Y + slot * Dp);
+        t.rho = static_cast<float>(ro[slot]);
+        slot = slot == 0 ? slots - 1 : slot - 1;
+        load_lane<E>(t.x, S + slot * Dp);
+    };
+    Stage a, b, c;
+    load_lane<E>(c.x, S + slot * Dp);
+    load_back(a);
+    load_back(b);
 #pragma unroll
     for (int j = 0; j < E; ++j) {
         const int e = lane + j * kWarp;
@@ -348,67 +364,55 @@ static __device__ __noinline__ double two_loop_regs_tree(const Vecs& vg, int bas
             gp[e] = ge;
         }
     }
-    float rho = static_cast<float>(ro[sl]);
-    float dot = lane_tree_warp_dot<E>(xv, r);
-    int next = older(sl);
-    if (count > 1) load_lane<E>(xv, S + next * Dp);
-    for (int k = count - 1; k >= 0; --k) {
-        // for the pass after this one: y of the next older pair, s of the one before that
-        const int after = older(next);
-        float rho_n = 0.f;
-        if (k > 0) {
-            rho_n = static_cast<float>(ro[next]);
-            load_lane<E>(yn, Y + next * Dp);
-        }
-        if (k > 1) load_lane<E>(xn, S + after * Dp);
-        const float a = dot * rho;
-        alf[k] = a;  // every lane holds the same value
+    dot = lane_tree_warp_dot<E>(c.x, r);
+    auto back = [&](int k, const Stage& t, Stage& ahead) {
+        load_back(ahead);
+        const float al = dot * t.rho;
+        alf[k] = al;  // every lane holds the same value
 #pragma unroll
-        for (int j = 0; j < E; ++j) r[j] = fmaf(yv[j], -a, r[j]);
+        for (int j = 0; j < E; ++j) r[j] = fmaf(t.y[j], -al, r[j]);
         if (k > 0) {
-            dot = lane_tree_warp_dot<E>(xv, r);
-            rho = rho_n;
-#pragma unroll
-            for (int j = 0; j < E; ++j) {
-                xv[j] = xn[j];
-                yv[j] = yn[j];
-            }
-            next = after;
+            dot = lane_tree_warp_dot<E>(t.x, r);
         } else {
-            // the second loop starts with the oldest pair: its s is loaded before its dot
-            load_lane<E>(xv, S + base * Dp);
 #pragma unroll
             for (int j = 0; j < E; ++j) r[j] *= hd;
-            dot = lane_tree_warp_dot<E>(yv, r);
+            dot = lane_tree_warp_dot<E>(t.y, r);
         }
+    };
+    for (int k = count - 1; k >= 0; k -= 3) {
+        back(k, a, c);
+        if (k < 1) break;
+        back(k - 1, b, a);
+        if (k < 2) break;
+        back(k - 2, c, b);
     }
     __syncwarp();
-    // second loop: xv = s of the pair, yv = y of the next newer pair (the gradient after the last)
-    sl = base;
-    rho = static_cast<float>(ro[sl]);
-    next = newer(sl);
-    if (count > 1) load_lane<E>(yv, Y + next * Dp);
-    for (int k = 0; k < count; ++k) {
-        const int after = newer(next);
-        float rho_n = 0.f;
-        if (k + 1 < count) {
-            rho_n = static_cast<float>(ro[next]);
-            load_lane<E>(xn, S + next * Dp);
-        }
-        if (k + 2 < count) load_lane<E>(yn, Y + after * Dp);
-        const float w = alf[k] - dot * rho;
+    // second loop, oldest to newest. Pass k takes s_k and, for the dot of the pass after it,
+    // y_{k+1}.
+    slot = base;
+    int kl = 0;
+    auto load_forward = [&](Stage& t) {  // s of `slot`, y of the next newer one
+        load_lane<E>(t.x, S + slot * Dp);
+        t.rho = static_cast<float>(ro[slot]);
+        t.al = alf[min(kl++, count - 1)];
+        slot = slot + 1 == slots ? 0 : slot + 1;
+        load_lane<E>(t.y, Y + slot * Dp);
+    };
+    load_forward(a);
+    load_forward(b);
+    auto forward = [&](int k, const Stage& t, Stage& ahead) {
+        load_forward(ahead);
+        const float w = t.al - dot * t.rho;
 #pragma unroll
-        for (int j = 0; j < E; ++j) r[j] = fmaf(xv[j], w, r[j]);
-        if (k + 1 < count) {
-            dot = lane_tree_warp_dot<E>(yv, r);
-            rho = rho_n;
-#pragma unroll
-            for (int j = 0; j < E; ++j) {
-                xv[j] = xn[j];
-                yv[j] = yn[j];
-            }
-            next = after;
-        }
+        for (int j = 0; j < E; ++j) r[j] = fmaf(t.x[j], w, r[j]);
+        if (k + 1 < count) dot = lane_tree_warp_dot<E>(t.y, r);
+    };
+    for (int k = 0; k < count; k += 3) {
+        forward(k, a, c);
+        if (k + 1 >= count) break;
+        forward(k + 1, b, a);
+        if (k + 2 >= count) break;
+        forward(k + 2, c, b);
     }
     // g . d for the line search, compensated as elsewhere
     DS acc{0.f, 0.f};

@@ -411,6 +411,10 @@ void free_receptor(pxd_context* ctx) {
     if (ctx->rec_ex_all) cudaFree(ctx->rec_ex_all);
     if (ctx->rec_ex_mov) cudaFree(ctx->rec_ex_mov);
     if (ctx->rec_score_mem) cudaFree(ctx->rec_score_mem);
+    for (float2*& t : ctx->d_vdw) {
+        if (t) cudaFree(t);
+        t = nullptr;
+    }
     ctx->rec_mem = ctx->rec_ex_all = ctx->rec_ex_mov = ctx->rec_score_mem = nullptr;
     ctx->rec_score = DevRecScore{};
     ctx->rec = DevReceptor{};
@@ -762,7 +766,7 @@ int pxd_set_receptor(pxd_context* ctx, const pxd_receptor_desc* r) {
     if (rc) return rc;
     ctx->has_receptor = true;
     ctx->ligands_dirty = true;
-    return PXD_OK;
+    return build_score_tables(ctx);
 }
 
 int pxd_decide_grid_dims(double cx, double cy, double cz, double sx, double sy, double sz,

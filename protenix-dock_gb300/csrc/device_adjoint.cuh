@@ -272,8 +272,8 @@ struct AdjPose {
 };
 
 template <class S>
-__device__ __forceinline__ typename Vec<S>::type rec_pos_g(const DevRecScore& rs, const float4* loc_xyz, int j) {
-    return lift3<S>(rec_pos(rs, loc_xyz, j));
+__device__ __forceinline__ typename Vec<S>::type rec_pos_g(const float4* loc_xyz, float4 v) {
+    return lift3<S>(rec_pos(v, loc_xyz));
 }
 
 // Features of the pose in X (every lane returns the same f[28]); with kGrad, adds
@@ -364,9 +364,8 @@ __device__ void score_adjoint_pose(const ScoreEnv& env, const DevLigand& L, cons
             S e = lift<S>(0.f);
             V gi = zero3<S>();
             for (int b = lane; b < rs.n_hyd; b += kWarp) {
-                const int j = __ldg(&rs.hyd[b]);
-                const float r1 = (s1 + __ldg(&rs.all_se[j]).x) * sf.hydro_factor + sf.hydro_min;
-                const V dv = sub3(xi, rec_pos_g<S>(rs, loc_xyz, j));
+                const float r1 = (s1 + __ldg(&rs.hyd_sigma[b])) * sf.hydro_factor + sf.hydro_min;
+                const V dv = sub3(xi, rec_pos_g<S>(loc_xyz, __ldg(&rs.hyd[b])));
                 const S d = sqrt_(dot3(dv, dv));
                 e = e - ramp_g(d, r1, r1 + sf.hydro_max);
                 if (kGrad && val(d) > 0.f)
@@ -386,13 +385,13 @@ __device__ void score_adjoint_pose(const ScoreEnv& env, const DevLigand& L, cons
         const int na = k == 0 ? ls.n_cat : ls.n_an;
         const int* la = k == 0 ? ls.cat : ls.an;
         const int nb = k == 0 ? rs.n_an : rs.n_cat;
-        const int* rb = k == 0 ? rs.an : rs.cat;
+        const float4* rb = k == 0 ? rs.an : rs.cat;
         for (int a = 0; a < na; ++a) {
             const int i = __ldg(&la[a]);
             const V xi = atom3<S>(X, XT, i);
             V gi = zero3<S>();
             for (int b = lane; b < nb; b += kWarp) {
-                const V dv = sub3(xi, rec_pos_g<S>(rs, loc_xyz, __ldg(&rb[b])));
+                const V dv = sub3(xi, rec_pos_g<S>(loc_xyz, __ldg(&rb[b])));
                 const S d = sqrt_(dot3(dv, dv));
                 f_ion[k] -= part(ramp_g(d, sf.ionic[k][0], sf.ionic[k][1]));
                 if (kGrad && val(d) > 0.f)
@@ -436,7 +435,7 @@ __device__ void score_adjoint_pose(const ScoreEnv& env, const DevLigand& L, cons
         lig_ring_g<S>(X, XT, ring, c, n);
         V gc = zero3<S>();
         for (int b = lane; b < rs.n_cat; b += kWarp) {
-            const V dv = sub3(c, rec_pos_g<S>(rs, loc_xyz, __ldg(&rs.cat[b])));
+            const V dv = sub3(c, rec_pos_g<S>(loc_xyz, __ldg(&rs.cat[b])));
             const S d = sqrt_(dot3(dv, dv));
             f_pc[k] -= part(ramp_g(d, sf.picat[k][0], sf.picat[k][1]));
             if (kGrad && val(d) > 0.f)
@@ -486,11 +485,11 @@ __device__ void score_adjoint_pose(const ScoreEnv& env, const DevLigand& L, cons
             V gd = zero3<S>(), gh = zero3<S>(), gdummy = zero3<S>();
             for (int u = 0; u < 2; ++u) {
                 const int na = u == 0 ? rs.n_accc : rs.n_accn;
-                const int* al = u == 0 ? rs.accc : rs.accn;
+                const float4* al = u == 0 ? rs.accc : rs.accn;
                 const int k = 2 * c + u;
                 const float sk = s_hb * W[PXD_W_HBOND + k];
                 for (int b = lane; b < na; b += kWarp)
-                    f_hb[k] += part(hbond_pair_adj<kGrad, S>(dp, hp, rec_pos_g<S>(rs, loc_xyz, __ldg(&al[b])),
+                    f_hb[k] += part(hbond_pair_adj<kGrad, S>(dp, hp, rec_pos_g<S>(loc_xyz, __ldg(&al[b])),
                                                              sf.hbond[k], sk, gd, gh, gdummy));
             }
             if (kGrad) {
@@ -511,14 +510,13 @@ __device__ void score_adjoint_pose(const ScoreEnv& env, const DevLigand& L, cons
             V ga = zero3<S>(), gd = zero3<S>(), gh = zero3<S>();
             for (int c = 0; c < 2; ++c) {
                 const int nd = c == 0 ? rs.n_donc : rs.n_donn;
-                const int2* dl = c == 0 ? rs.donc : rs.donn;
+                const float4* const* dl = c == 0 ? rs.donc : rs.donn;
                 const int k = 4 + 2 * c + u;
                 const float sk = s_hb * W[PXD_W_HBOND + k];
                 for (int b = lane; b < nd; b += kWarp) {
-                    const int2 dh = __ldg(&dl[b]);
-                    f_hb[k] += part(hbond_pair_adj<kGrad, S>(rec_pos_g<S>(rs, loc_xyz, dh.x),
-                                                             rec_pos_g<S>(rs, loc_xyz, dh.y), apos, sf.hbond[k], sk,
-                                                             gd, gh, ga));
+                    f_hb[k] += part(hbond_pair_adj<kGrad, S>(rec_pos_g<S>(loc_xyz, __ldg(&dl[0][b])),
+                                                             rec_pos_g<S>(loc_xyz, __ldg(&dl[1][b])), apos, sf.hbond[k],
+                                                             sk, gd, gh, ga));
                 }
             }
             if (kGrad) {

@@ -28,11 +28,13 @@ __device__ __forceinline__ float dist3(float3 a, float3 b) {
 struct ScoreEnv {
     DevRecScore rs;
     const DevSf* sf;
+    const float2* vdw;  // [99][rs.n_cls] mean sigma, 4 sqrt(eps eps) under sf (score_vdw_kernel)
 };
 
-__device__ __forceinline__ float3 rec_pos(const DevRecScore& rs, const float4* loc_xyz, int j) {
-    const int l = __ldg(&rs.all_local[j]);
-    return l >= 0 ? xyz(loc_xyz[l]) : xyz(__ldg(&rs.all_xyzq[j]));
+// Position of a listed receptor atom (DevRecScore): its own, or its rotor's.
+__device__ __forceinline__ float3 rec_pos(float4 v, const float4* loc_xyz) {
+    const int l = __float_as_int(v.w);
+    return l >= 0 ? xyz(loc_xyz[l]) : xyz(v);
 }
 
 __device__ __forceinline__ void lig_ring(const float4* X, const int* r, float3& c, float3& n) {
@@ -91,73 +93,68 @@ __device__ __forceinline__ float signed_dihedral(float3 pi, float3 pj, float3 pk
     return dot3(rij, n) < 0.f ? phi : -phi;
 }
 
-// Score of the pose in X (ligand, smem) with receptor rotor atoms in loc_xyz (smem).
-// Returns sum(coef * term) over the active terms except GB/SA; when `terms` is given,
-// lane 0 stores the unweighted values.
-//
-// kTeam (a team of warps of one block, PoseBufs' team fields in tw / tn / ts): the members
-// split the all-pairs Coulomb / LJ loop, members 1, 2 and 3 add the hydrophobic, the
-// ionic / cation-pi / stacking and the hydrogen-bond / torsion-strain terms, and the
-// partials are summed in member order, so every member returns the same score.
-template <bool kTeam = false>
-static __device__ double score_pose(const ScoreEnv& env, const DevLigand& L, const DevLigScore& ls,
-                             const float4* X, const float4* loc_xyz, int lane, double* terms,
-                             int tw = 0, int tn = 1, TeamShared* ts = nullptr) {
+// This warp's share (w of nw) of the terms of the pose in X (ligand, smem) with receptor
+// rotor atoms in loc_xyz (smem), added up per lane into acc. The warps split the Coulomb / LJ
+// pairs by receptor atom and the hydrophobic contacts by ligand atom, whose partial sums are
+// compensated; the other terms are FP32 sums of one warp each. The terms read the receptor
+// lists by value, one record per atom: through index lists a contact was a chain of four
+// loads, and a pose of 55 atoms in a pocket of 1,866 took one warp 460,000 cycles.
+static __device__ __forceinline__ void score_terms(const ScoreEnv& env, const DevLigand& L, const DevLigScore& ls,
+                                                   const float4* X, const float4* loc_xyz, int lane, int w, int nw,
+                                                   DS* acc) {
     const DevRecScore& rs = env.rs;
     const DevSf& sf = *env.sf;
     const int N = L.n_atoms;
-    if (!kTeam) {
-        tw = 0;
-        tn = 1;
-    }
-    // the members that add the terms other than Coulomb / LJ (all of them on a lone warp)
-    const bool own_hyd = tw == 1 % tn, own_ion = tw == 2 % tn, own_hb = tw == 3 % tn;
-    DS acc[PXD_NUM_TERMS - 1];
+    const bool own_hb = w == nw - 1, own_ion = w == max(nw - 2, 0);
+    const int hyd_warps = nw > 2 ? nw - 2 : nw;  // the warps that share the hydrophobic contacts
 #pragma unroll
     for (int k = 0; k < PXD_NUM_TERMS - 1; ++k) acc[k] = DS{0.f, 0.f};
     const bool coul = sf.coef[PXD_TERM_COULOMB] != 0.f, vdw = sf.coef[PXD_TERM_VDW] != 0.f;
     // Coulomb and clamped LJ over every ligand x receptor pair (scorer.cpp:222-276). Each
     // lane takes receptor atoms and walks the ligand atoms (shared memory and L1-resident
     // records, read by every lane at once): a receptor atom's records are loaded once per
-    // call instead of once per ligand atom, which leaves a lone warp (the single-walker
-    // search) arithmetic instead of load latency. The pairs are the same; their sum runs
-    // in another order.
+    // call instead of once per ligand atom. Mean sigma and 4 sqrt(eps eps) of a (type, class)
+    // come from a table; their square root per pair was a quarter of the loop.
     if (coul || vdw) {
-        for (int j = lane + tw * kWarp; j < rs.n_all; j += tn * kWarp) {
+        const float cutoff = sf.vdw_cutoff;
+        const float* const charge = L.charge;
+        const int* const type = L.type;
+        for (int j = lane + w * kWarp; j < rs.n_all; j += nw * kWarp) {
             const float4 rj = __ldg(&rs.all_xyzq[j]);
-            const int l = __ldg(&rs.all_local[j]);
-            const float3 xj = l >= 0 ? xyz(loc_xyz[l]) : xyz(rj);
-            const float2 sej = __ldg(&rs.all_se[j]);
+            const int2 lc = __ldg(&rs.all_lc[j]);
+            const float3 xj = lc.x >= 0 ? xyz(loc_xyz[lc.x]) : xyz(rj);
+            const float2* const row = env.vdw + lc.y;
             float ec = 0.f, ev = 0.f;
 #pragma unroll 4
             for (int i = 0; i < N; ++i) {
                 const float3 xi = xyz(X[i]);
-                const float qi = __ldg(&L.charge[i]);
-                const float2 ti = sf.vdw_type[__ldg(&L.type[i])];
+                const float qi = __ldg(&charge[i]);
+                const float2 sc = __ldg(&row[__ldg(&type[i]) * rs.n_cls]);
                 const float d = dist3(xi, xj);
                 const float rinv = 1.f / (d + kEpsF);
                 ec = fmaf(qi * rj.w, rinv, ec);
-                const float s = (ti.x + sej.x) * 0.5f * rinv;
+                const float s = sc.x * rinv;
                 const float s2 = s * s;
                 const float u6 = s2 * s2 * s2;
-                const float v = (u6 * u6 - u6) * (sqrtf(ti.y * sej.y) * 4.f);
-                ev += fminf(fmaxf(v, -sf.vdw_cutoff), sf.vdw_cutoff);
+                const float v = (u6 * u6 - u6) * sc.y;
+                ev += fminf(fmaxf(v, -cutoff), cutoff);
             }
             ds_add(acc[PXD_TERM_COULOMB], ec * kCoulombF);
             ds_add(acc[PXD_TERM_VDW], ev);
         }
     }
     // hydrophobic contacts (scorer.cpp:278-311)
-    if (own_hyd && sf.coef[PXD_TERM_HYDROPHOBIC] != 0.f) {
-        for (int a = 0; a < ls.n_hyd; ++a) {
+    if (sf.coef[PXD_TERM_HYDROPHOBIC] != 0.f && w < hyd_warps) {
+        const float hydro_factor = sf.hydro_factor, hydro_min = sf.hydro_min, hydro_max = sf.hydro_max;
+        for (int a = w; a < ls.n_hyd; a += hyd_warps) {
             const int i = __ldg(&ls.hyd[a]);
             const float3 xi = xyz(X[i]);
             const float s1 = sf.vdw_sigma_raw[__ldg(&L.type[i])];
             float e = 0.f;
+#pragma unroll 4
             for (int b = lane; b < rs.n_hyd; b += kWarp) {
-                const int j = __ldg(&rs.hyd[b]);
-                const float r1 = (s1 + __ldg(&rs.all_se[j]).x) * sf.hydro_factor + sf.hydro_min;
-                e -= ramp_down(dist3(xi, rec_pos(rs, loc_xyz, j)), r1, r1 + sf.hydro_max);
+                const float r1 = (s1 + __ldg(&rs.hyd_sigma[b])) * hydro_factor + hydro_min;
+                e -= ramp_down(dist3(xi, rec_pos(__ldg(&rs.hyd[b]), loc_xyz)), r1, r1 + hydro_max);
             }
             ds_add(acc[PXD_TERM_HYDROPHOBIC], e);
         }
@@ -169,13 +166,13 @@ static __device__ double score_pose(const ScoreEnv& env, const DevLigand& L, con
             const float3 xi = xyz(X[__ldg(&ls.cat[a])]);
             for (int b = lane; b < rs.n_an; b += kWarp)
                 e -= sf.ionic_coef[0] *
-                     ramp_down(dist3(xi, rec_pos(rs, loc_xyz, __ldg(&rs.an[b]))), sf.ionic[0][0], sf.ionic[0][1]);
+                     ramp_down(dist3(xi, rec_pos(__ldg(&rs.an[b]), loc_xyz)), sf.ionic[0][0], sf.ionic[0][1]);
         }
         for (int a = 0; a < ls.n_an; ++a) {
             const float3 xi = xyz(X[__ldg(&ls.an[a])]);
             for (int b = lane; b < rs.n_cat; b += kWarp)
                 e -= sf.ionic_coef[1] *
-                     ramp_down(dist3(rec_pos(rs, loc_xyz, __ldg(&rs.cat[b])), xi), sf.ionic[1][0], sf.ionic[1][1]);
+                     ramp_down(dist3(rec_pos(__ldg(&rs.cat[b]), loc_xyz), xi), sf.ionic[1][0], sf.ionic[1][1]);
         }
         ds_add(acc[PXD_TERM_IONIC], e);
     }
@@ -196,14 +193,14 @@ static __device__ double score_pose(const ScoreEnv& env, const DevLigand& L, con
             const int k = five ? 2 : 3;
             for (int b = lane; b < rs.n_cat; b += kWarp)
                 e -= sf.picat_coef[k] *
-                     ramp_down(dist3(c, rec_pos(rs, loc_xyz, __ldg(&rs.cat[b]))), sf.picat[k][0], sf.picat[k][1]);
+                     ramp_down(dist3(c, rec_pos(__ldg(&rs.cat[b]), loc_xyz)), sf.picat[k][0], sf.picat[k][1]);
         }
         ds_add(acc[PXD_TERM_PI_CATION], e);
     }
     // pi stacking, face-to-face (centre 0) and edge-to-face (centre 90) (scorer.cpp:638-724)
-    for (int w = 0; w < 2; ++w) {
-        if (!own_ion || sf.coef[PXD_TERM_F2F + w] == 0.f) continue;
-        const float center = w == 0 ? 0.f : 90.f;
+    for (int f = 0; f < 2; ++f) {
+        if (!own_ion || sf.coef[PXD_TERM_F2F + f] == 0.f) continue;
+        const float center = f == 0 ? 0.f : 90.f;
         float e = 0.f;
         for (int r = 0; r < ls.n_r5 + ls.n_r6; ++r) {
             const bool five = r < ls.n_r5;
@@ -212,13 +209,13 @@ static __device__ double score_pose(const ScoreEnv& env, const DevLigand& L, con
             // l5r5, l5r6, l6r5, l6r6 in the reference's argument order
             const int k5 = five ? 0 : 2, k6 = five ? 1 : 3;
             for (int b = lane; b < rs.n_r5; b += kWarp)
-                e += sf.stack_coef[w][k5] * stack_pair(xyz(__ldg(&rs.r5c[b])), xyz(__ldg(&rs.r5n[b])), lc, ln,
-                                                       sf.stack[w][k5], center);
+                e += sf.stack_coef[f][k5] * stack_pair(xyz(__ldg(&rs.r5c[b])), xyz(__ldg(&rs.r5n[b])), lc, ln,
+                                                       sf.stack[f][k5], center);
             for (int b = lane; b < rs.n_r6; b += kWarp)
-                e += sf.stack_coef[w][k6] * stack_pair(xyz(__ldg(&rs.r6c[b])), xyz(__ldg(&rs.r6n[b])), lc, ln,
-                                                       sf.stack[w][k6], center);
+                e += sf.stack_coef[f][k6] * stack_pair(xyz(__ldg(&rs.r6c[b])), xyz(__ldg(&rs.r6n[b])), lc, ln,
+                                                       sf.stack[f][k6], center);
         }
-        ds_add(acc[PXD_TERM_F2F + w], e);
+        ds_add(acc[PXD_TERM_F2F + f], e);
     }
     // hydrogen bonds, 8 donor/acceptor classes (scorer.cpp:464-577)
     if (own_hb && sf.coef[PXD_TERM_HBOND] != 0.f) {
@@ -231,11 +228,11 @@ static __device__ double score_pose(const ScoreEnv& env, const DevLigand& L, con
                 const float3 dp = xyz(X[dh.x]), hp = xyz(X[dh.y]);
                 for (int u = 0; u < 2; ++u) {  // receptor acceptors (charged, neutral)
                     const int na = u == 0 ? rs.n_accc : rs.n_accn;
-                    const int* al = u == 0 ? rs.accc : rs.accn;
+                    const float4* al = u == 0 ? rs.accc : rs.accn;
                     const int k = 2 * c + u;
                     float s = 0.f;
                     for (int b = lane; b < na; b += kWarp)
-                        s += hbond_pair(dp, hp, rec_pos(rs, loc_xyz, __ldg(&al[b])), sf.hbond[k]);
+                        s += hbond_pair(dp, hp, rec_pos(__ldg(&al[b]), loc_xyz), sf.hbond[k]);
                     e += sf.hbond_coef[k] * s;
                 }
             }
@@ -247,13 +244,12 @@ static __device__ double score_pose(const ScoreEnv& env, const DevLigand& L, con
                 const float3 ap = xyz(X[__ldg(&al[a])]);
                 for (int c = 0; c < 2; ++c) {  // receptor donors (charged, neutral)
                     const int nd = c == 0 ? rs.n_donc : rs.n_donn;
-                    const int2* dl = c == 0 ? rs.donc : rs.donn;
+                    const float4* const* dl = c == 0 ? rs.donc : rs.donn;
                     const int k = 4 + 2 * c + u;
                     float s = 0.f;
-                    for (int b = lane; b < nd; b += kWarp) {
-                        const int2 dh = __ldg(&dl[b]);
-                        s += hbond_pair(rec_pos(rs, loc_xyz, dh.x), rec_pos(rs, loc_xyz, dh.y), ap, sf.hbond[k]);
-                    }
+                    for (int b = lane; b < nd; b += kWarp)
+                        s += hbond_pair(rec_pos(__ldg(&dl[0][b]), loc_xyz), rec_pos(__ldg(&dl[1][b]), loc_xyz), ap,
+                                        sf.hbond[k]);
                     e += sf.hbond_coef[k] * s;
                 }
             }
@@ -277,9 +273,29 @@ static __device__ double score_pose(const ScoreEnv& env, const DevLigand& L, con
             if (j > 0) ds_add(acc[PXD_TERM_TSTRAIN], tmp / j);
         }
     }
+}
+
+// Completes the term values (scales, the constant rotatable term, GB/SA 0) and returns
+// sum(coef * term) over the active terms except GB/SA.
+static __device__ __forceinline__ double score_total(const DevSf& sf, const DevLigScore& ls, double* vals) {
+    vals[PXD_TERM_VDW] *= sf.vdw_scale;
+    vals[PXD_TERM_HYDROPHOBIC] *= sf.hydro_scale;
+    vals[PXD_TERM_ROTATABLE] = sf.coef[PXD_TERM_ROTATABLE] != 0.f ? -1.0 / (2.620643 + ls.n_rot) : 0.0;
+    vals[PXD_TERM_GBSA] = 0.0;
     double total = 0.0;
+#pragma unroll
+    for (int k = 0; k < PXD_NUM_TERMS; ++k) total += static_cast<double>(sf.coef[k]) * vals[k];
+    return total;
+}
+
+// Score of the pose in X, by a team of warps of one block (or one warp, tn = 1): the
+// members' partials are summed in member order, so every member returns the same score.
+static __device__ __noinline__ double score_pose(const ScoreEnv& env, const DevLigand& L, const float4* X,
+                                                 const float4* loc_xyz, int lane, int tw, int tn, TeamShared* ts) {
+    DS acc[PXD_NUM_TERMS - 1];
+    score_terms(env, L, L.score, X, loc_xyz, lane, tw, tn, acc);
     double vals[PXD_NUM_TERMS];
-    if (kTeam && tn > 1) {
+    if (tn > 1) {
 #pragma unroll
         for (int k = 0; k < PXD_NUM_TERMS - 1; ++k) {
             const DS r = ds_warp_reduce(acc[k]);
@@ -299,16 +315,7 @@ static __device__ double score_pose(const ScoreEnv& env, const DevLigand& L, con
 #pragma unroll
         for (int k = 0; k < PXD_NUM_TERMS - 1; ++k) vals[k] = ds_warp_sum(acc[k]);
     }
-    vals[PXD_TERM_VDW] *= sf.vdw_scale;
-    vals[PXD_TERM_HYDROPHOBIC] *= sf.hydro_scale;
-    vals[PXD_TERM_ROTATABLE] = sf.coef[PXD_TERM_ROTATABLE] != 0.f ? -1.0 / (2.620643 + ls.n_rot) : 0.0;
-    vals[PXD_TERM_GBSA] = 0.0;
-#pragma unroll
-    for (int k = 0; k < PXD_NUM_TERMS; ++k) total += static_cast<double>(sf.coef[k]) * vals[k];
-    if (terms && lane == 0) {
-        for (int k = 0; k < PXD_NUM_TERMS; ++k) terms[k] = vals[k];
-    }
-    return total;
+    return score_total(*env.sf, L.score, vals);
 }
 
 }  // namespace pxd

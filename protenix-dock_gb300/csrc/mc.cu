@@ -228,7 +228,7 @@ __device__ double mc_pscore(const McArgs& a, const DevLigand& L, const float* x,
         b.loc_xyz[l] = make_float4(p.x, p.y, p.z, 0.f);
     }
     __syncwarp();
-    return score_pose<true>(a.senv, L, L.score, b.lig_xyz, b.loc_xyz, lane, nullptr, tm.w, tm.n, tm.ts);
+    return score_pose(a.senv, L, b.lig_xyz, b.loc_xyz, lane, tm.w, tm.n, tm.ts);
 }
 
 __device__ void atomic_min_double(double* p, double v) {
@@ -596,6 +596,7 @@ int pxd_mc_search_dev(pxd_context* ctx, const pxd_mc_params* p, int32_t n_walker
     a.env.grid = ctx->grid;
     a.senv.rs = ctx->rec_score;
     a.senv.sf = ctx->d_sf[0];
+    a.senv.vdw = ctx->d_vdw[0];
     a.ligands = ctx->d_ligands;
     a.n_ligands = static_cast<int>(ctx->ligands.size());
     a.lig_ids = lig_ids;

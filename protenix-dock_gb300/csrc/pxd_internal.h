@@ -72,19 +72,24 @@ struct DevRecScore {
     int n_all;
     const float4* all_xyzq;    // every receptor atom: position, charge
     const float2* all_se;      // sigma, epsilon
-    const int* all_local;      // rotor-atom local index or -1
+    const int2* all_lc;        // rotor-atom local index or -1; (sigma, epsilon) class
+    int n_cls;
+    const float2* cls_se;      // [n_cls] sigma, epsilon of a class
     int n_hyd, n_cat, n_an, n_r5, n_r6, n_donc, n_donn, n_accc, n_accn;
-    const int* hyd;
-    const int* cat;
-    const int* an;
+    // the lists' atoms by value, so that a term reads one record per atom: position, and in
+    // .w the rotor-atom local index (int bits, -1: fixed)
+    const float4* hyd;
+    const float* hyd_sigma;
+    const float4* cat;
+    const float4* an;
     const float4* r5c;         // ring centroid
     const float4* r5n;         // ring normal
     const float4* r6c;
     const float4* r6n;
-    const int2* donc;
-    const int2* donn;
-    const int* accc;
-    const int* accn;
+    const float4* donc[2];     // donor heavy atoms, hydrogens
+    const float4* donn[2];
+    const float4* accc;
+    const float4* accn;
     const int* pclass;         // [n_all] pair-table class (C N O other: 0-3), -1 none; NULL: no table term
     const float4* pair_rec;    // [n_all] sigma, sqrt(epsilon), pair-table class, rotor local index (int bits)
 };
@@ -226,6 +231,7 @@ struct pxd_context {
     void* rec_score_mem = nullptr;
     std::vector<double> rec_gb_radius, rec_gb_screen;
     pxd::DevSf* d_sf[2] = {nullptr, nullptr};
+    float2* d_vdw[2] = {nullptr, nullptr};  // [99][n_cls] per scoring function (score_vdw_kernel)
     pxd_sf_params sf_host[2];
     bool sf_set[2] = {false, false};
     // autotuned L-BFGS variant (minimum resident blocks per SM) per size-class bound
@@ -318,6 +324,7 @@ int launch_ligand_pose_backward(pxd_context* ctx, int lig, int n_poses, const fl
                                 const float* quats, const float* grad, float* out_center, float* out_quat,
                                 float* out_tors, cudaStream_t s);
 int pair_class(int is_receptor, int z);
+int build_score_tables(pxd_context* ctx);
 int upload_receptor_scoring(pxd_context* ctx, const pxd_score_lists* l, const std::vector<int>& local_of);
 int upload_ligand_scoring(pxd_context* ctx, LigandEntry& e, const pxd_score_lists* l);
 void gbsa_properties(const pxd_score_lists* l, int n, std::vector<double>& radius,

@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -140,7 +141,6 @@ int upload_receptor_scoring(pxd_context* ctx, const pxd_score_lists* l, const st
     d.n_all = M;
     d.all_xyzq = at<float4>(ctx->rec_ex_all, ctx->ex_all_off[0]);
     d.all_se = at<float2>(ctx->rec_ex_all, ctx->ex_all_off[1]);
-    d.all_local = at<int>(ctx->rec_ex_all, ctx->ex_all_off[2]);
     gbsa_properties(l, M, ctx->rec_gb_radius, ctx->rec_gb_screen);
     if (l && !lists_ok(l, M)) return set_error(ctx, PXD_ERR_INVALID, "receptor interaction list atom out of range");
     // per-atom record of the differentiable score's pair loop: sigma, sqrt(epsilon),
@@ -152,8 +152,20 @@ int upload_receptor_scoring(pxd_context* ctx, const pxd_score_lists* l, const st
                                  static_cast<float>(std::sqrt(ctx->rec_epsilon[a])),
                                  __int_as_float_host(pcls.empty() ? -1 : pcls[a]),
                                  __int_as_float_host(ctx->is_mov[a] ? local_of[a] : -1));
+    std::vector<float2> cls;
+    std::vector<int2> lc(M);
+    {
+        std::map<std::pair<float, float>, int> seen;
+        for (int a = 0; a < M; ++a) {
+            const float2 se = make_float2(static_cast<float>(ctx->rec_sigma[a]), static_cast<float>(ctx->rec_epsilon[a]));
+            const auto it = seen.emplace(std::make_pair(se.x, se.y), static_cast<int>(cls.size())).first;
+            if (it->second == static_cast<int>(cls.size())) cls.push_back(se);
+            lc[a] = make_int2(ctx->is_mov[a] ? local_of[a] : -1, it->second);
+        }
+    }
     Pack pk;
-    const size_t o_pair = pk.put(pairrec);
+    const size_t o_pair = pk.put(pairrec), o_lc = pk.put(lc), o_cls = pk.put(cls);
+    d.n_cls = static_cast<int>(cls.size());
     if (!l) {
         int rc0 = cuda_check(ctx, cudaMalloc(&ctx->rec_score_mem, pk.bytes.size()), "receptor score lists");
         if (rc0) return rc0;
@@ -161,6 +173,8 @@ int upload_receptor_scoring(pxd_context* ctx, const pxd_score_lists* l, const st
                          "receptor score lists copy");
         if (rc0) return rc0;
         d.pair_rec = at<float4>(ctx->rec_score_mem, o_pair);
+        d.all_lc = at<int2>(ctx->rec_score_mem, o_lc);
+        d.cls_se = at<float2>(ctx->rec_score_mem, o_cls);
         return PXD_OK;
     }
     // ring centroids and normals (to_ring_centroid / to_ring_normal, scorer.cpp:128-172)
@@ -192,14 +206,28 @@ int upload_receptor_scoring(pxd_context* ctx, const pxd_score_lists* l, const st
                                         static_cast<float>(nn[2] / len), 0.f));
         }
     }
-    const size_t o_hyd = pk.put(ints(l->hydrophobic, l->n_hydrophobic));
-    const size_t o_cat = pk.put(ints(l->cation, l->n_cation));
-    const size_t o_an = pk.put(ints(l->anion, l->n_anion));
+    // a list's atoms (every `step`-th index from `ids`) by value
+    auto atoms = [&](const int32_t* ids, int n, int step = 1) {
+        std::vector<float4> v;
+        for (int i = 0; i < n; ++i) {
+            const int a = ids[step * i];
+            v.push_back(make_float4(static_cast<float>(ctx->rec_xyz[3 * a]), static_cast<float>(ctx->rec_xyz[3 * a + 1]),
+                                    static_cast<float>(ctx->rec_xyz[3 * a + 2]), __int_as_float_host(lc[a].x)));
+        }
+        return v;
+    };
+    std::vector<float> hyd_sigma;
+    for (int i = 0; i < l->n_hydrophobic; ++i) hyd_sigma.push_back(static_cast<float>(ctx->rec_sigma[l->hydrophobic[i]]));
+    const size_t o_hyd = pk.put(atoms(l->hydrophobic, l->n_hydrophobic)), o_hyds = pk.put(hyd_sigma);
+    const size_t o_cat = pk.put(atoms(l->cation, l->n_cation));
+    const size_t o_an = pk.put(atoms(l->anion, l->n_anion));
     const size_t o_r5c = pk.put(rc[0]), o_r5n = pk.put(rn[0]), o_r6c = pk.put(rc[1]), o_r6n = pk.put(rn[1]);
-    const size_t o_donc = pk.put(pairs2(l->don_charged, l->n_don_charged));
-    const size_t o_donn = pk.put(pairs2(l->don_neutral, l->n_don_neutral));
-    const size_t o_accc = pk.put(ints(l->acc_charged, l->n_acc_charged));
-    const size_t o_accn = pk.put(ints(l->acc_neutral, l->n_acc_neutral));
+    const size_t o_donc = pk.put(atoms(l->don_charged, l->n_don_charged, 2));
+    const size_t o_donch = pk.put(atoms(l->don_charged + 1, l->n_don_charged, 2));
+    const size_t o_donn = pk.put(atoms(l->don_neutral, l->n_don_neutral, 2));
+    const size_t o_donnh = pk.put(atoms(l->don_neutral + 1, l->n_don_neutral, 2));
+    const size_t o_accc = pk.put(atoms(l->acc_charged, l->n_acc_charged));
+    const size_t o_accn = pk.put(atoms(l->acc_neutral, l->n_acc_neutral));
     const size_t o_pcl = pk.put(pcls);
     int rc_ = cuda_check(ctx, cudaMalloc(&ctx->rec_score_mem, pk.bytes.size()), "receptor score lists");
     if (rc_) return rc_;
@@ -217,17 +245,22 @@ int upload_receptor_scoring(pxd_context* ctx, const pxd_score_lists* l, const st
     d.n_donn = l->n_don_neutral;
     d.n_accc = l->n_acc_charged;
     d.n_accn = l->n_acc_neutral;
-    d.hyd = at<int>(b, o_hyd);
-    d.cat = at<int>(b, o_cat);
-    d.an = at<int>(b, o_an);
+    d.all_lc = at<int2>(b, o_lc);
+    d.cls_se = at<float2>(b, o_cls);
+    d.hyd = at<float4>(b, o_hyd);
+    d.hyd_sigma = at<float>(b, o_hyds);
+    d.cat = at<float4>(b, o_cat);
+    d.an = at<float4>(b, o_an);
     d.r5c = at<float4>(b, o_r5c);
     d.r5n = at<float4>(b, o_r5n);
     d.r6c = at<float4>(b, o_r6c);
     d.r6n = at<float4>(b, o_r6n);
-    d.donc = at<int2>(b, o_donc);
-    d.donn = at<int2>(b, o_donn);
-    d.accc = at<int>(b, o_accc);
-    d.accn = at<int>(b, o_accn);
+    d.donc[0] = at<float4>(b, o_donc);
+    d.donc[1] = at<float4>(b, o_donch);
+    d.donn[0] = at<float4>(b, o_donn);
+    d.donn[1] = at<float4>(b, o_donnh);
+    d.accc = at<float4>(b, o_accc);
+    d.accn = at<float4>(b, o_accn);
     d.pclass = pcls.empty() ? nullptr : at<int>(b, o_pcl);
     d.pair_rec = at<float4>(b, o_pair);
     return PXD_OK;
@@ -308,7 +341,35 @@ int upload_ligand_scoring(pxd_context* ctx, LigandEntry& e, const pxd_score_list
 }
 
 // ------------------------------------------------------------------ kernels
-constexpr int kScoreWarps = 4;
+// Mean sigma and 4 sqrt(eps eps) of every (ligand type, receptor class) under a scoring
+// function, which the pair loop of score_terms would otherwise form per pair.
+__global__ void score_vdw_kernel(const DevSf* sf, const float2* cls, int n_cls, float2* out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= PXD_NUM_VDW_TYPES * n_cls) return;
+    const float2 ti = sf->vdw_type[k / n_cls], se = cls[k % n_cls];
+    out[k] = make_float2((ti.x + se.x) * 0.5f, sqrtf(ti.y * se.y) * 4.f);
+}
+
+// (Re)builds the tables of the installed scoring functions for the installed receptor.
+int build_score_tables(pxd_context* ctx) {
+    for (int w = 0; w < 2; ++w) {
+        if (!ctx->sf_set[w] || !ctx->has_receptor) continue;
+        const int n = PXD_NUM_VDW_TYPES * ctx->rec_score.n_cls;
+        if (ctx->d_vdw[w]) cudaFree(ctx->d_vdw[w]);
+        ctx->d_vdw[w] = nullptr;
+        int rc = cuda_check(ctx, cudaMalloc(&ctx->d_vdw[w], sizeof(float2) * std::max(n, 1)), "score tables");
+        if (rc) return rc;
+        if (n > 0)
+            score_vdw_kernel<<<(n + 127) / 128, 128, 0, ctx->stream>>>(ctx->d_sf[w], ctx->rec_score.cls_se,
+                                                                       ctx->rec_score.n_cls, ctx->d_vdw[w]);
+        rc = cuda_check(ctx, cudaGetLastError(), "score_vdw_kernel launch");
+        if (!rc) rc = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "score tables");
+        if (rc) return rc;
+    }
+    return PXD_OK;
+}
+
+constexpr int kMaxScoreWarps = 16;
 
 struct EsArgs {
     ScoreEnv env;
@@ -324,45 +385,58 @@ struct EsArgs {
     double* terms;
 };
 
-// Rotor atom positions for the torsions t (torsional_receptor::apply_parameters).
-__device__ void receptor_rotors(const DevReceptor& R, const float* t, float4* loc, int lane) {
-    for (int l = lane; l < R.n_mov; l += kWarp) {
-        const float4 v = __ldg(&R.local_xyz0[l]);
-        const int r = __float_as_int(v.w);
-        Mat3 Rm, Jm;
-        rotation_and_jacobian(xyz(__ldg(&R.rotor_axis[r])), t[r], Rm, Jm);
-        const float3 p = add3(mat_apply(Rm, xyz(v)), xyz(__ldg(&R.rotor_origin[r])));
-        loc[l] = make_float4(p.x, p.y, p.z, 0.f);
-    }
-    __syncwarp();
-}
-
-__global__ void __launch_bounds__(kScoreWarps * kWarp) empirical_score_kernel(const EsArgs a) {
+// One block per pose, its warps sharing the terms (score_terms).
+__global__ void __launch_bounds__(kMaxScoreWarps * kWarp) empirical_score_kernel(const __grid_constant__ EsArgs a) {
     extern __shared__ __align__(16) float smem[];
+    __shared__ float2 s_part[kMaxScoreWarps][PXD_NUM_TERMS - 1];
     const int lane = threadIdx.x & (kWarp - 1);
-    const int wib = threadIdx.x / kWarp;
-    const int per_warp = 4 * (a.max_atoms + a.rec.n_mov + 1) + PXD_MAX_RECEPTOR_TORSIONS;
-    float4* X = reinterpret_cast<float4*>(smem + wib * per_warp);
+    const int w = threadIdx.x / kWarp, nw = blockDim.x / kWarp;
+    float4* X = reinterpret_cast<float4*>(smem);
     float4* loc = X + a.max_atoms;
-    float* tq = reinterpret_cast<float*>(loc + a.rec.n_mov + 1);
     const int R = a.rec.n_rotors;
-    for (int pose = blockIdx.x * kScoreWarps + wib; pose < a.n_poses; pose += gridDim.x * kScoreWarps) {
+    for (int pose = blockIdx.x; pose < a.n_poses; pose += gridDim.x) {
         const int lid = a.lig_ids[pose];
         if (lid < 0 || lid >= a.n_ligands || !a.ligands[lid].score.has ||
             a.ligands[lid].n_atoms > a.max_atoms) {
-            if (lane == 0) a.score[pose] = nan("");
+            if (threadIdx.x == 0) a.score[pose] = nan("");
             continue;
         }
         const DevLigand& L = a.ligands[lid];
         const float* px = a.xyz + static_cast<size_t>(pose) * a.max_atoms * 3;
-        for (int i = lane; i < L.n_atoms; i += kWarp) X[i] = make_float4(px[3 * i], px[3 * i + 1], px[3 * i + 2], 0.f);
-        for (int r = lane; r < R; r += kWarp) tq[r] = a.tors[static_cast<size_t>(pose) * R + r];
-        __syncwarp();
-        receptor_rotors(a.rec, tq, loc, lane);
-        const double s = score_pose(a.env, L, L.score, X, loc, lane,
-                                    a.terms ? a.terms + static_cast<size_t>(pose) * PXD_NUM_TERMS : nullptr);
-        if (lane == 0) a.score[pose] = s;
-        __syncwarp();
+        for (int i = threadIdx.x; i < L.n_atoms; i += blockDim.x)
+            X[i] = make_float4(px[3 * i], px[3 * i + 1], px[3 * i + 2], 0.f);
+        // rotor atom positions (torsional_receptor::apply_parameters)
+        for (int l = threadIdx.x; l < a.rec.n_mov; l += blockDim.x) {
+            const float4 v = __ldg(&a.rec.local_xyz0[l]);
+            const int r = __float_as_int(v.w);
+            Mat3 Rm, Jm;
+            rotation_and_jacobian(xyz(__ldg(&a.rec.rotor_axis[r])), a.tors[static_cast<size_t>(pose) * R + r], Rm, Jm);
+            const float3 p = add3(mat_apply(Rm, xyz(v)), xyz(__ldg(&a.rec.rotor_origin[r])));
+            loc[l] = make_float4(p.x, p.y, p.z, 0.f);
+        }
+        __syncthreads();
+        DS acc[PXD_NUM_TERMS - 1];
+        score_terms(a.env, L, L.score, X, loc, lane, w, nw, acc);
+#pragma unroll
+        for (int k = 0; k < PXD_NUM_TERMS - 1; ++k) {
+            const DS r = ds_warp_reduce(acc[k]);
+            if (lane == 0) s_part[w][k] = make_float2(r.hi, r.lo);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double vals[PXD_NUM_TERMS];
+#pragma unroll
+            for (int k = 0; k < PXD_NUM_TERMS - 1; ++k) {
+                DS t{s_part[0][k].x, s_part[0][k].y};
+                for (int u = 1; u < nw; ++u) ds_add_ds(t, DS{s_part[u][k].x, s_part[u][k].y});
+                vals[k] = static_cast<double>(t.hi) + static_cast<double>(t.lo);
+            }
+            a.score[pose] = score_total(*a.env.sf, L.score, vals);
+            if (a.terms)
+                for (int k = 0; k < PXD_NUM_TERMS; ++k) a.terms[static_cast<size_t>(pose) * PXD_NUM_TERMS + k] = vals[k];
+        }
+        // s_part and X are rewritten only after the next pose's first barrier has seen thread 0
+        __syncthreads();
     }
 }
 
@@ -718,7 +792,7 @@ int pxd_set_scoring_function(pxd_context* ctx, int32_t which, const pxd_sf_param
     if (rc) return rc;
     ctx->sf_host[which] = *p;
     ctx->sf_set[which] = true;
-    return PXD_OK;
+    return build_score_tables(ctx);
 }
 
 int pxd_score_dev(pxd_context* ctx, int32_t which, int32_t n_poses, int32_t max_atoms, const int32_t* ids,
@@ -736,6 +810,7 @@ int pxd_score_dev(pxd_context* ctx, int32_t which, int32_t n_poses, int32_t max_
     EsArgs a{};
     a.env.rs = ctx->rec_score;
     a.env.sf = ctx->d_sf[which];
+    a.env.vdw = ctx->d_vdw[which];
     a.rec = ctx->rec;
     a.ligands = ctx->d_ligands;
     a.n_ligands = static_cast<int>(ctx->ligands.size());
@@ -746,16 +821,17 @@ int pxd_score_dev(pxd_context* ctx, int32_t which, int32_t n_poses, int32_t max_
     a.n_poses = n_poses;
     a.score = score;
     a.terms = terms;
-    const int per_warp = 4 * (max_atoms + ctx->rec.n_mov + 1) + PXD_MAX_RECEPTOR_TORSIONS;
-    const size_t smem = sizeof(float) * per_warp * kScoreWarps;
+    const size_t smem = sizeof(float4) * (max_atoms + ctx->rec.n_mov + 1);
     if (smem > 48 * 1024) {
         rc = raise_smem_limit(ctx, reinterpret_cast<const void*>(empirical_score_kernel), smem, "score smem");
         if (rc) return rc;
     }
-    int blocks = (n_poses + kScoreWarps - 1) / kScoreWarps;
-    if (blocks > ctx->n_sm * 16) blocks = ctx->n_sm * 16;
+    // enough warps to fill the chip: four per pose once the poses do, up to 16 for a few poses
+    int warps = 4;
+    while (warps < kMaxScoreWarps && static_cast<long long>(n_poses) * warps < 16LL * ctx->n_sm) warps *= 2;
+    const int blocks = std::min(n_poses, ctx->n_sm * 64);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-    empirical_score_kernel<<<blocks, kScoreWarps * kWarp, smem, s>>>(a);
+    empirical_score_kernel<<<blocks, warps * kWarp, smem, s>>>(a);
     return cuda_check(ctx, cudaGetLastError(), "empirical_score_kernel launch");
 }
 

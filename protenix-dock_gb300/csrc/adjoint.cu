@@ -2,12 +2,12 @@
 // persistent blocks) with its deterministic reductions, the C ABI, and the
 // device-buffer pose kinematics used by gradient pipelines.
 //
-// Per block, the weight gradient (36 doubles per warp, each warp adding its poses in
-// order) and the pair-table gradient (8,192 floats, shared atomics) are accumulated in
-// shared memory and written once as a per-block partial; partial_sum_kernel then adds
-// the partials of all blocks in a fixed order, in FP64, into the caller's accumulators.
-// No global atomics: scores, coordinate and weight gradients repeat bit for bit; the
-// table gradient's shared atomics leave its last bits to the order of arrival.
+// The weight gradient is linear in the features, so each warp adds its poses' dL/dS-weighted
+// features (28 doubles) in order, and weight_grad_kernel adds the blocks' sums in a fixed
+// order and maps them to the 36 weights once. The pair-table gradient (8,192 floats) goes to
+// partials that table_sum_kernel adds in FP64. Scores, coordinate and weight gradients repeat
+// bit for bit; the table gradient's atomic additions leave its last bits to the order of
+// arrival.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -18,6 +18,9 @@
 namespace pxd {
 
 constexpr int kAdjWarps = 8;
+// Partials of the table gradient in global memory, at most: two blocks per SM, so that a bin is
+// hardly ever added to by two blocks at once.
+constexpr int kTablePartials = 304;
 
 // One receptor context as the kernel sees it.
 struct AdjCtx {
@@ -45,8 +48,9 @@ struct AdjArgs {
     double* score;           // [n_poses] or NULL
     double* features;        // [n_poses][28] or NULL
     float* dxyz;             // [n_poses][max_atoms][3] or NULL
-    double* part_w;          // [gridDim][36] per-block weight-gradient partials
-    float* part_t;           // [gridDim][32 * 256] per-block table-gradient partials or NULL
+    double* part_f;          // [gridDim][28] per-block sums of dL/dS-weighted features
+    float* part_t;           // [n_part_t][32 * 256] table-gradient partials or NULL
+    int n_part_t;
 };
 
 // Rotor atom positions for the torsions t (torsional_receptor::apply_parameters).
@@ -63,15 +67,23 @@ __device__ void adj_receptor_rotors(const DevReceptor& R, const float* t, float4
 }
 
 // S = float: scores, features and gradients; S = Dual: their derivatives along xyz_t.
+//
+// Bound by FP32 issue and its latencies: about 100 instructions per pair of a ligand and a
+// receptor atom, at 8 to 16 warps per SM. The table gradient's additions go to global memory,
+// where they return nothing: in shared memory a float addition is a compare-and-swap loop that
+// the warp waits for, and the table's 32 KB took L1 from the receptor. A training step of 4,096
+// poses in 32 pockets: 4.56 -> 3.85 ms, with the loads taken out of the pair loop. A tangent
+// launch keeps its table in shared memory: its dual numbers bound it, and it measures the same.
 template <bool kGrad, bool kMulti, class S>
 __global__ void __launch_bounds__(kAdjWarps * kWarp, 2) score_adjoint_kernel(const __grid_constant__ AdjArgs a) {
     extern __shared__ __align__(16) unsigned char adj_smem[];
     double* s_w = reinterpret_cast<double*>(adj_smem);  // [36] weights
-    double* s_dw = s_w + kNumW;                         // [warps][36] weight gradient per warp
-    float* s_wf = reinterpret_cast<float*>(s_dw + kAdjWarps * kNumW);  // [36] FP32 weights
-    float* s_tg = s_wf + kNumW + 4;                     // [32 * 256] when table gradients are asked for
+    double* s_f = s_w + kNumW;                          // [warps][28] weighted features per warp
+    float* s_wf = reinterpret_cast<float*>(s_f + kAdjWarps * kNumF);  // [36] FP32 weights
+    float* s_tg = s_wf + kNumW + 4;                     // [32 * 256] table gradient (kBlockTable)
     const bool tgrad = kGrad && a.part_t && a.tables;
-    float* warp_base = tgrad ? s_tg + kTabN : s_tg;
+    constexpr bool kBlockTable = IsDual<S>::value;
+    float* warp_base = kBlockTable && tgrad ? s_tg + kTabN : s_tg;
     const int lane = threadIdx.x & (kWarp - 1);
     const int wib = threadIdx.x / kWarp;
     constexpr int kSlices = IsDual<S>::value ? 3 : 2;  // X, G (and the tangents XT)
@@ -85,8 +97,8 @@ __global__ void __launch_bounds__(kAdjWarps * kWarp, 2) score_adjoint_kernel(con
         s_w[k] = a.weights[k];
         s_wf[k] = static_cast<float>(a.weights[k]);
     }
-    for (int k = threadIdx.x; k < kAdjWarps * kNumW; k += blockDim.x) s_dw[k] = 0.0;
-    if (tgrad)
+    for (int k = threadIdx.x; k < kAdjWarps * kNumF; k += blockDim.x) s_f[k] = 0.0;
+    if (kBlockTable && tgrad)
         for (int k = threadIdx.x; k < kTabN; k += blockDim.x) s_tg[k] = 0.f;
     __syncthreads();
     for (int pose = blockIdx.x * kAdjWarps + wib; pose < a.n_poses; pose += gridDim.x * kAdjWarps) {
@@ -116,7 +128,9 @@ __global__ void __launch_bounds__(kAdjWarps * kWarp, 2) score_adjoint_kernel(con
         AdjPose ap;
         ap.wf = s_wf;
         ap.tab = a.tables;
-        ap.tgrad = tgrad ? s_tg : nullptr;
+        ap.tgrad = !tgrad       ? nullptr
+                   : kBlockTable ? s_tg
+                                 : a.part_t + static_cast<size_t>(blockIdx.x % a.n_part_t) * kTabN;
         ap.g = kGrad ? static_cast<float>(a.grad_out[pose]) : 0.f;
         double f[kNumF];
         score_adjoint_pose<kGrad, S>(C.env, L, X, XT, loc, ap, G, lane, f);
@@ -128,7 +142,8 @@ __global__ void __launch_bounds__(kAdjWarps * kWarp, 2) score_adjoint_kernel(con
                 if (lane == (k & (kWarp - 1))) fo[k] = f[k];
         }
         if (kGrad) {
-            if (lane == 0) combine_grad(s_w, f, a.grad_out[pose], s_dw + wib * kNumW);
+            if (lane == 0)
+                for (int k = 0; k < kNumF; ++k) s_f[wib * kNumF + k] += a.grad_out[pose] * f[k];
             __syncwarp();
             if (dx) {
                 for (int i = lane; i < a.max_atoms; i += kWarp) {
@@ -143,32 +158,59 @@ __global__ void __launch_bounds__(kAdjWarps * kWarp, 2) score_adjoint_kernel(con
     }
     if (!kGrad) return;
     __syncthreads();
-    for (int k = threadIdx.x; k < kNumW; k += blockDim.x) {
+    if (a.part_f && threadIdx.x < kNumF) {
         double t = 0.0;
-        for (int w = 0; w < kAdjWarps; ++w) t += s_dw[w * kNumW + k];
-        a.part_w[static_cast<size_t>(blockIdx.x) * kNumW + k] = t;
+        for (int w = 0; w < kAdjWarps; ++w) t += s_f[w * kNumF + threadIdx.x];
+        a.part_f[static_cast<size_t>(blockIdx.x) * kNumF + threadIdx.x] = t;
     }
-    if (tgrad) {
+    if (kBlockTable && tgrad) {
         float* pt = a.part_t + static_cast<size_t>(blockIdx.x) * kTabN;
         for (int k = threadIdx.x; k < kTabN; k += blockDim.x) pt[k] = s_tg[k];
     }
 }
 
-// out[k] += sum over blocks b (in order) of part[b][k], in FP64.
-template <class T>
-__global__ void partial_sum_kernel(const T* __restrict__ part, int n_blocks, int n, double* out) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    double s = 0.0;
-    for (int b = 0; b < n_blocks; ++b) s += static_cast<double>(part[static_cast<size_t>(b) * n + k]);
-    out[k] += s;
+// out[k] += sum over the partials (in order within each of eight interleaved runs, then the
+// runs) of part[p][k], in FP64: 32 bins per block, a run of partials per warp.
+__global__ void __launch_bounds__(256) table_sum_kernel(const float* __restrict__ part, int n_part, double* out) {
+    __shared__ double s[8][kWarp];
+    const int lane = threadIdx.x & (kWarp - 1), run = threadIdx.x / kWarp;
+    const int k = blockIdx.x * kWarp + lane;
+    double v = 0.0;
+    for (int p = run; p < n_part; p += 8) v += static_cast<double>(part[static_cast<size_t>(p) * kTabN + k]);
+    s[run][lane] = v;
+    __syncthreads();
+    if (run == 0) {
+        for (int u = 1; u < 8; ++u) v += s[u][lane];
+        out[k] += v;
+    }
+}
+
+// dweights[k] += dS/dw[k] of the summed features: the blocks' sums in order within each of 32
+// interleaved runs, then the runs.
+__global__ void __launch_bounds__(1024) weight_grad_kernel(const double* __restrict__ part, int n_part,
+                                                           const double* __restrict__ weights, double* out) {
+    __shared__ double s[32][kNumF], f[kNumF];
+    const int k = threadIdx.x & (kWarp - 1), run = threadIdx.x / kWarp;
+    if (k < kNumF) {
+        double v = 0.0;
+        for (int p = run; p < n_part; p += 32) v += part[static_cast<size_t>(p) * kNumF + k];
+        s[run][k] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < kNumF) {
+        double v = 0.0;
+        for (int u = 0; u < 32; ++u) v += s[u][threadIdx.x];
+        f[threadIdx.x] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < kNumW) out[threadIdx.x] += combine_grad(weights, f, threadIdx.x);
 }
 
 static size_t adj_smem_bytes(int max_atoms, int n_mov, bool tgrad, bool tangent) {
     const size_t per_warp =
         4 * ((tangent ? 3 : 2) * static_cast<size_t>(max_atoms) + n_mov + 1) + PXD_MAX_RECEPTOR_TORSIONS;
-    return sizeof(double) * (1 + kAdjWarps) * kNumW + sizeof(float) * (kNumW + 4) +
-           (tgrad ? sizeof(float) * kTabN : 0) +
+    return sizeof(double) * (kNumW + kAdjWarps * kNumF) + sizeof(float) * (kNumW + 4) +
+           (tgrad && tangent ? sizeof(float) * kTabN : 0) +
            sizeof(float) * per_warp * kAdjWarps;
 }
 
@@ -263,8 +305,7 @@ static int launch_adjoint(pxd_context* const* ctxs, int32_t n_ctx, int32_t which
                     "adjoint occupancy");
     if (rc) return rc;
     if (per_sm < 1) per_sm = 1;
-    int blocks = (n_poses + kAdjWarps - 1) / kAdjWarps;
-    if (blocks > ctx->n_sm * per_sm) blocks = ctx->n_sm * per_sm;
+    const int blocks = std::min((n_poses + kAdjWarps - 1) / kAdjWarps, ctx->n_sm * per_sm);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
     AdjArgs a{};
     a.one = table[0];
@@ -284,12 +325,14 @@ static int launch_adjoint(pxd_context* const* ctxs, int32_t n_ctx, int32_t which
     a.score = tangent ? nullptr : score;
     a.features = features;
     a.dxyz = dxyz;
-    a.part_w = nullptr;
+    a.part_f = nullptr;
     a.part_t = nullptr;
-    // one stream-ordered allocation: context table, weight and table partials
+    // one stream-ordered allocation: context table, feature and table partials
     const size_t cbytes = multi ? (sizeof(AdjCtx) * n_ctx + 255) / 256 * 256 : 0;
-    const size_t wbytes = grad ? (sizeof(double) * kNumW * blocks + 255) / 256 * 256 : 0;
-    const size_t tbytes = tgrad ? sizeof(float) * kTabN * blocks : 0;
+    const bool wgrad = grad && dweights;
+    const size_t wbytes = wgrad ? (sizeof(double) * kNumF * blocks + 255) / 256 * 256 : 0;
+    a.n_part_t = tangent ? blocks : std::min(blocks, kTablePartials);
+    const size_t tbytes = tgrad ? sizeof(float) * kTabN * a.n_part_t : 0;
     void* mem = nullptr;
     if (cbytes + wbytes + tbytes) {
         rc = cuda_check(ctx, cudaMallocAsync(&mem, cbytes + wbytes + tbytes, s), "adjoint scratch");
@@ -301,20 +344,23 @@ static int launch_adjoint(pxd_context* const* ctxs, int32_t n_ctx, int32_t which
                         "context table copy");
         a.ctxs = reinterpret_cast<const AdjCtx*>(base);
     }
-    if (grad) a.part_w = reinterpret_cast<double*>(base + cbytes);
-    if (tgrad) a.part_t = reinterpret_cast<float*>(base + cbytes + wbytes);
+    if (wgrad) a.part_f = reinterpret_cast<double*>(base + cbytes);
+    if (tgrad) {
+        a.part_t = reinterpret_cast<float*>(base + cbytes + wbytes);
+        if (!rc && !tangent) rc = cuda_check(ctx, cudaMemsetAsync(a.part_t, 0, tbytes, s), "table gradient partials");
+    }
     if (!rc) {
         void* params[] = {&a};
         rc = cuda_check(ctx, cudaLaunchKernel(fn, dim3(blocks), dim3(kAdjWarps * kWarp), params, smem, s),
                         "score_adjoint_kernel launch");
     }
-    if (!rc && grad && dweights) {
-        partial_sum_kernel<double><<<1, 64, 0, s>>>(a.part_w, blocks, kNumW, dweights);
-        rc = cuda_check(ctx, cudaGetLastError(), "partial_sum_kernel launch");
+    if (!rc && wgrad) {
+        weight_grad_kernel<<<1, 1024, 0, s>>>(a.part_f, blocks, weights, dweights);
+        rc = cuda_check(ctx, cudaGetLastError(), "weight_grad_kernel launch");
     }
     if (!rc && tgrad) {
-        partial_sum_kernel<float><<<(kTabN + 255) / 256, 256, 0, s>>>(a.part_t, blocks, kTabN, dtables);
-        rc = cuda_check(ctx, cudaGetLastError(), "partial_sum_kernel launch");
+        table_sum_kernel<<<kTabN / kWarp, 256, 0, s>>>(a.part_t, a.n_part_t, dtables);
+        rc = cuda_check(ctx, cudaGetLastError(), "table_sum_kernel launch");
     }
     if (mem) cudaFreeAsync(mem, s);
     return rc;

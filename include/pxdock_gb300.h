@@ -537,6 +537,12 @@ int pxd_score_adjoint_multi_dev(pxd_context* const* contexts, int32_t n_contexts
                                 double* score_dev, double* features_dev, float* dxyz_dev,
                                 double* dweights_dev, double* dtables_dev, void* stream);
 
+/* dweights_dev [36] += sum_p grad_out_p dS_p/dw from the features [n_poses][28] that a score
+ * launch wrote for the same weights (the score is linear in its features). */
+int pxd_score_weight_grad_dev(pxd_context* ctx, int32_t n_poses, const double* features_dev,
+                              const double* grad_out_dev, const double* weights_dev,
+                              double* dweights_dev, void* stream);
+
 /* Second-order products of the same score along a direction of the ligand coordinates
  * (forward-mode over the adjoint, derivatives almost everywhere): for each pose p with
  * direction xyz_dir [P][max_atoms][3] and output weight grad_out[p],

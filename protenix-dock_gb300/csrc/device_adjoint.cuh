@@ -249,7 +249,7 @@ __device__ __forceinline__ double combine_grad(const double* w, const double* f,
         case PXD_W_COEF + PXD_TERM_HYDROPHOBIC: return w[PXD_W_HYDRO_SCALE] * f[F_HYD];
         case PXD_W_COEF + PXD_TERM_TSTRAIN: return f[F_TSTRAIN];
         case PXD_W_COEF + PXD_TERM_ROTATABLE: return f[F_ROT];
-        case PXD_W_COEF + PXD_TERM_GBSA: return 0.0;
+        case PXD_W_COEF + PXD_TERM_GBSA: return 0.0 * f[F_COUL];  // not part of this score
         case PXD_W_VDW_SCALE: return w[PXD_W_COEF + PXD_TERM_VDW] * f[F_VDW];
         case PXD_W_HYDRO_SCALE: return w[PXD_W_COEF + PXD_TERM_HYDROPHOBIC] * f[F_HYD];
         case PXD_W_HBOND_SCALE: return w[PXD_W_COEF + PXD_TERM_HBOND] * dot(PXD_W_HBOND, F_HBOND, 8);

@@ -82,7 +82,9 @@ class _EmpiricalScore(torch.autograd.Function):
         if fctx.needs_input_grad[0]:
             gx = (dx * g.to(torch.float32)[:, None, None]).to(xdt)
         if fctx.needs_input_grad[1]:
-            gw = abi.weights_grad(w, (feats * g[:, None]).sum(0)).to(wdt)
+            gw = torch.zeros(abi.NUM_SF_WEIGHTS, dtype=torch.float64, device=x.device)
+            pctxs[0].score_weight_grad_dev(P, _ptr(feats), _ptr(g), _ptr(w), _ptr(gw), _stream())
+            gw = gw.to(wdt)
         if has_tab and fctx.needs_input_grad[2]:
             if bool((g == g[0]).all()):
                 gt = (dt * g[0]).view(abi.PAIR_TYPES, abi.PAIR_BINS).to(tdt)

@@ -99,6 +99,7 @@ def load(auto_build=False):
     lib.pxd_score_adjoint_multi_dev.argtypes = [C.POINTER(vp), C.c_int32, C.c_int32, C.c_int32, C.c_int32] + [vp] * 13
     lib.pxd_ligand_pose_multi_dev.argtypes = [C.POINTER(vp), C.c_int32, C.c_int32, C.c_int32, C.c_int32] + [vp] * 8
     lib.pxd_score_grad_multi_dev.argtypes = [C.POINTER(vp), C.c_int32, C.c_int32, C.c_int32] + [vp] * 8
+    lib.pxd_score_weight_grad_dev.argtypes = [vp, C.c_int32] + [vp] * 5
     lib.pxd_score_hvp_multi_dev.argtypes = [C.POINTER(vp), C.c_int32, C.c_int32, C.c_int32, C.c_int32] + [vp] * 13
     lib.pxd_lbfgs_autotune_dev.argtypes = [vp, C.POINTER(abi.LbfgsParams), C.c_int32, C.c_int32, vp, vp, vp,
                                            C.c_int32, C.c_int32, abi.i32p, vp]
@@ -409,6 +410,11 @@ class Context:
         if not grads:
             return s, f
         return s, f, dx, dw, dt.reshape(abi.PAIR_TYPES, abi.PAIR_BINS)
+
+    def score_weight_grad_dev(self, n_poses, features_ptr, grad_out_ptr, weights_ptr, dweights_ptr, stream=None):
+        """pxd_score_weight_grad_dev (integer device addresses)."""
+        self._check(self.lib.pxd_score_weight_grad_dev(self.h, n_poses, features_ptr, grad_out_ptr, weights_ptr,
+                                                       dweights_ptr, stream))
 
     def score_adjoint_dev(self, which, n_poses, max_atoms, ids_ptr, xyz_ptr, tors_ptr, weights_ptr, tables_ptr,
                           grad_out_ptr, score_ptr, features_ptr, dxyz_ptr, dweights_ptr, dtables_ptr, stream=None):

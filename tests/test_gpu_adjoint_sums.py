@@ -61,3 +61,24 @@ def test_sums_over_poses(n, tangent):
     parts = sum(launch(a, min(a + 8, n))[1] for a in range(0, n, 8))
     np.testing.assert_allclose(dt, parts, rtol=0, atol=1e-4 * np.max(np.abs(parts)))
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [0, 1, 33, 8192, 20001])
+def test_weight_grad_of_features(n):
+    """The same map from given features (FP64 sums: 1e-12 of the sum of magnitudes), added to
+    what the output holds; no pose leaves it as it is."""
+    torch = pytest.importorskip("torch")
+    native.load(auto_build=True)
+    rng = np.random.default_rng(n)
+    f, g = rng.normal(size=(n, abi.NUM_SCORE_FEATURES)), rng.normal(size=n)
+    w, before = rng.normal(size=abi.NUM_SF_WEIGHTS), rng.normal(size=abi.NUM_SF_WEIGHTS)
+    fd, gd, wd, dw = (torch.tensor(a, device="cuda") for a in (np.vstack([f, f[:1] * 0 if n else np.zeros((1, 28))]),
+                                                               np.append(g, 7.0), w, before))
+    ctx = native.Context(0)
+    torch.cuda.synchronize()
+    ctx.score_weight_grad_dev(n, fd.data_ptr(), gd.data_ptr(), wd.data_ptr(), dw.data_ptr())
+    torch.cuda.synchronize()
+    want = before + abi.weights_grad(w, (f * g[:, None]).sum(0))
+    size = np.abs(before) + abi.weights_grad(np.abs(w), np.abs(f * g[:, None]).sum(0))
+    assert np.all(np.abs(dw.cpu().numpy() - want) <= 1e-12 * size)
+    ctx.close()

@@ -72,7 +72,7 @@ __device__ void adj_receptor_rotors(const DevReceptor& R, const float* t, float4
 // receptor atom, at 8 to 16 warps per SM. The table gradient's additions go to global memory,
 // where they return nothing: in shared memory a float addition is a compare-and-swap loop that
 // the warp waits for, and the table's 32 KB took L1 from the receptor. A training step of 4,096
-// poses in 32 pockets: 4.56 -> 3.85 ms, with the loads taken out of the pair loop. A tangent
+// poses in 16 pockets: 4.56 -> 3.85 ms, with the loads taken out of the pair loop. A tangent
 // launch keeps its table in shared memory: its dual numbers bound it, and it measures the same.
 template <bool kGrad, bool kMulti, class S>
 __global__ void __launch_bounds__(kAdjWarps * kWarp, 2) score_adjoint_kernel(const __grid_constant__ AdjArgs a) {

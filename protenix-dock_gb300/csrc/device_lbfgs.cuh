@@ -100,8 +100,9 @@ __device__ __forceinline__ double closure_eval(TeamClosure& c, double t, const f
     return eval_pose<true>(*c.env, *c.L, c.x0, d, static_cast<float>(t), g, *c.b, c.lane, gdot, c.team);
 }
 
-__device__ __forceinline__ double cubic_interpolate(double x1, double f1, double g1, double x2,
-                                                    double f2, double g2, double lo, double hi) {
+// Out of line: its FP64 divisions are long, and the line search calls it from two places.
+static __device__ __noinline__ double cubic_interpolate(double x1, double f1, double g1, double x2, double f2,
+                                                        double g2, double lo, double hi) {
     double d1 = g1 + g2 - 3.0 * (f1 - f2) / (x1 - x2);
     const double d2sq = d1 * d1 - g1 * g2;
     if (d2sq >= 0.0) {
@@ -271,8 +272,9 @@ static __device__ void strong_wolfe(Cl& c, const LbfgsConsts& p, const float* d,
 //
 // energy receives the FP64 objective at the returned pose (energy64), or, with
 // final_energy false (a caller that does not use it), the last FP32 loss.
-// The two-loop recursion for D <= E * 32, the direction held in registers (E elements per
-// lane) instead of the shared vectors q and d. Each pass's history elements are loaded
+// The two-loop recursion for (E - 1) * 32 < D <= E * 32, the direction held in registers (E
+// elements per lane, only the last of them tested against D) instead of the shared vectors q
+// and d. Each pass's history elements are loaded
 // before the reduction its coefficient waits on, and no pass stores or reloads the
 // direction, so the only dependent chain left is the reduction itself: what a warp alone on
 // its SM (the single-walker search) waits on. Lane-element order, products and accumulation
@@ -454,8 +456,9 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
 #pragma unroll
         for (int j = 0; j < E; ++j) {
             const int e = lane + j * kWarp;
+            const bool in = j < E - 1 || e < D;
             r[j] = 0.f;
-            if (e < D) {
+            if (in) {
                 const float ge = v.g[e];
                 r[j] = -ge;
                 v.gp[e] = ge;
@@ -463,6 +466,7 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
             }
         }
     }
+#pragma unroll 1
     for (int k = count - 1; k >= 0; --k) {
         const float* yk = v.Y + sl * Dp;
         const int sn_slot = sl == 0 ? slots - 1 : sl - 1;
@@ -471,8 +475,9 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
 #pragma unroll
         for (int j = 0; j < E; ++j) {
             const int e = lane + j * kWarp;
-            yv[j] = e < D ? yk[e] : 0.f;
-            sv[j] = e < D && k > 0 ? sn[e] : 0.f;
+            const bool in = j < E - 1 || e < D;
+            yv[j] = in ? yk[e] : 0.f;
+            sv[j] = in && k > 0 ? sn[e] : 0.f;
         }
         const double al = ds_warp_sum(acc) * v.ro[sl];
         if (lane == 0) v.al[k] = al;
@@ -481,7 +486,7 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
         if (k > 0) {
 #pragma unroll
             for (int j = 0; j < E; ++j) {
-                if (lane + j * kWarp < D) {
+                if (j < E - 1 || lane + j * kWarp < D) {
                     r[j] = fmaf(yv[j], nal, r[j]);
                     ds_dot_acc(acc, sv[j], r[j]);
                 }
@@ -489,7 +494,7 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
         } else {
 #pragma unroll
             for (int j = 0; j < E; ++j) {
-                if (lane + j * kWarp < D) {
+                if (j < E - 1 || lane + j * kWarp < D) {
                     r[j] = fmaf(yv[j], nal, r[j]) * hd;
                     ds_dot_acc(acc, yv[j], r[j]);
                 }
@@ -499,6 +504,7 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
     }
     __syncwarp();  // al written by lane 0 above, read by every lane below
     sl = base;
+#pragma unroll 1
     for (int k = 0; k < count; ++k) {
         const float* sk = v.S + sl * Dp;
         const int nx_slot = sl + 1 == slots ? 0 : sl + 1;
@@ -507,14 +513,15 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
 #pragma unroll
         for (int j = 0; j < E; ++j) {
             const int e = lane + j * kWarp;
-            sv[j] = e < D ? sk[e] : 0.f;
-            nv[j] = e < D ? nx[e] : 0.f;
+            const bool in = j < E - 1 || e < D;
+            sv[j] = in ? sk[e] : 0.f;
+            nv[j] = in ? nx[e] : 0.f;
         }
         const float w = static_cast<float>(v.al[k] - ds_warp_sum(acc) * v.ro[sl]);
         acc = DS{0.f, 0.f};
 #pragma unroll
         for (int j = 0; j < E; ++j) {
-            if (lane + j * kWarp < D) {
+            if (j < E - 1 || lane + j * kWarp < D) {
                 r[j] = fmaf(sv[j], w, r[j]);
                 ds_dot_acc(acc, nv[j], r[j]);
             }
@@ -524,10 +531,27 @@ static __device__ __forceinline__ double two_loop_regs(const Vecs& v, int base, 
 #pragma unroll
     for (int j = 0; j < E; ++j) {
         const int e = lane + j * kWarp;
-        if (e < D) v.d[e] = r[j];
+        if (j < E - 1 || e < D) v.d[e] = r[j];
     }
     __syncwarp();
     return ds_warp_sum(acc);  // g . d after the last step
+}
+
+// two_loop_regs for a direction of E rows of 32 elements, E = 1 .. 8. A 43-atom ligand's 129
+// elements took the recursion for 8 rows before: 236 -> 208 ms for 65,536 poses, and 29.1 ->
+// 23.2 ms for one ligand's 48 poses with 100 kept pairs.
+static __device__ __forceinline__ double two_loop_rows(int E, const Vecs& v, int base, int count, int slots, size_t Dp,
+                                                       int D, int lane, float hd) {
+    switch (E) {
+        case 1: return two_loop_regs<1>(v, base, count, slots, Dp, D, lane, hd);
+        case 2: return two_loop_regs<2>(v, base, count, slots, Dp, D, lane, hd);
+        case 3: return two_loop_regs<3>(v, base, count, slots, Dp, D, lane, hd);
+        case 4: return two_loop_regs<4>(v, base, count, slots, Dp, D, lane, hd);
+        case 5: return two_loop_regs<5>(v, base, count, slots, Dp, D, lane, hd);
+        case 6: return two_loop_regs<6>(v, base, count, slots, Dp, D, lane, hd);
+        case 7: return two_loop_regs<7>(v, base, count, slots, Dp, D, lane, hd);
+        default: return two_loop_regs<8>(v, base, count, slots, Dp, D, lane, hd);
+    }
 }
 
 template <bool kFast = false, bool kRegLoop = kFast, class Cl>
@@ -555,12 +579,13 @@ static __device__ int lbfgs_pose(Cl& c, const LbfgsConsts& p, const Vecs& v, int
         ++n_iter;
         bool reset = n_iter == 1;
         if (!reset) {
-            const int spare = (S.base + S.count) % slots;
+            const int spare = S.base + S.count >= slots ? S.base + S.count - slots : S.base + S.count;
             float* ys_ = v.Y + spare * Dp;
             float* ss_ = v.S + spare * Dp;
             const float tf = static_cast<float>(S.t);
             float ymax = 0.f;
             DS a_ys{0.f, 0.f}, a_yy{0.f, 0.f};
+#pragma unroll 1
             for (int e = lane; e < D; e += kWarp) {
                 const float y = v.g[e] - v.gp[e];
                 const float sv = v.d[e] * tf;
@@ -580,7 +605,7 @@ static __device__ int lbfgs_pose(Cl& c, const LbfgsConsts& p, const Vecs& v, int
                 const double yy = ds_warp_sum(a_yy);
                 if (ys > 1e-10) {
                     if (S.count == m)
-                        S.base = (S.base + 1) % slots;  // the oldest slot becomes the spare
+                        S.base = S.base + 1 == slots ? 0 : S.base + 1;  // the oldest slot becomes the spare
                     else
                         ++S.count;
                     S.H_diag = ys / yy;
@@ -598,6 +623,7 @@ static __device__ int lbfgs_pose(Cl& c, const LbfgsConsts& p, const Vecs& v, int
             }
             const float hd = static_cast<float>(S.H_diag);
             DS acc{0.f, 0.f}, a_abs{0.f, 0.f};
+#pragma unroll 1
             for (int e = lane; e < D; e += kWarp) {
                 const float ge = v.g[e];
                 const float de = reset ? -ge : (-ge) * hd;
@@ -618,11 +644,9 @@ static __device__ int lbfgs_pose(Cl& c, const LbfgsConsts& p, const Vecs& v, int
             gtd = two_loop_tree((D + kWarp - 1) / kWarp, v, S.base, S.count, slots, static_cast<int>(Dp), D, lane,
                                 static_cast<float>(S.H_diag));
             S.t = p.lr;
-        } else if (kRegLoop && D <= 4 * kWarp) {
-            gtd = two_loop_regs<4>(v, S.base, S.count, slots, Dp, D, lane, static_cast<float>(S.H_diag));
-            S.t = p.lr;
         } else if (kRegLoop && D <= 8 * kWarp) {
-            gtd = two_loop_regs<8>(v, S.base, S.count, slots, Dp, D, lane, static_cast<float>(S.H_diag));
+            gtd = two_loop_rows((D + kWarp - 1) / kWarp, v, S.base, S.count, slots, Dp, D, lane,
+                                 static_cast<float>(S.H_diag));
             S.t = p.lr;
         } else {
             // first loop, newest to oldest: q = -g - sum al_k y_k. The ring's base and count
@@ -717,6 +741,7 @@ static __device__ int lbfgs_pose(Cl& c, const LbfgsConsts& p, const Vecs& v, int
         // x += t d, with max|g| and max|t d| for the convergence tests
         const float tf = static_cast<float>(S.t);
         float gmax = 0.f, smax = 0.f;
+#pragma unroll 1
         for (int e = lane; e < D; e += kWarp) {
             const float de = v.d[e];
             v.x[e] = fmaf(de, tf, v.x[e]);

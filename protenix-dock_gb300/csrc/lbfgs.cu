@@ -36,7 +36,12 @@ struct LbfgsArgs {
 };
 
 constexpr int kWarpsPerBlock = 4;
-constexpr int kDefaultMinBlocks = 5;  // measured best on GB300 for the 42-atom bench ligand (296.7k poses/s against 293.3k for 4)
+// Poses/s of 4 blocks of 128 registers against 5 of 96 (65,536 poses of a 43-atom ligand: 180
+// against 187 ms; 16,384 of 60 and 80 atoms: 71 against 77, 109 against 109; 2,000 poses: 12.7
+// against 13.0; 28,800 poses of 24 ligands of 10 to 47 heavy atoms: 151 against 151) and 3 (187,
+// 75, 113, 12.1, 149): fewer spills, and fewer warps that take each other's instructions out of
+// the cache.
+constexpr int kDefaultMinBlocks = 4;
 
 // Floats of one warp's shared-memory slice: the evaluation buffers, the optimiser
 // vectors and scalars, the history when it is held there, and for rigid-body + torsion

@@ -1,6 +1,7 @@
 // Persistent batched L-BFGS kernel (one warp per pose, dynamic pose queue) and the
 // score+gradient kernel, with their launchers.
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <mutex>
 #include <type_traits>
@@ -228,20 +229,33 @@ static LbfgsKernelFn dof_kernel() { return lbfgs_kernel<kDefaultMinBlocks, true>
 // Size class of a per-warp atom capacity: the smallest bound of 32, 64, ..., 256 it fits.
 static int class_bound(int cap) { return std::min(256, (cap + 31) / 32 * 32); }
 
+// Blocks per SM of a launch of n_poses, unless chosen otherwise: when all poses are resident at
+// once with a larger register budget (two blocks without a cap, or three), nothing is gained by
+// room for more warps, and each pose runs faster without spills. 48 poses: 19.8 against 22.6 ms
+// with four blocks; 2,000 poses, which four blocks just hold: 11.4 (three) and 12.2 (two)
+// against 12.4.
+static int default_min_blocks(const pxd_context* ctx, int n_poses) {
+    if (n_poses <= 2 * kWarpsPerBlock * ctx->n_sm) return 0;
+    return n_poses <= 3 * kWarpsPerBlock * ctx->n_sm ? 3 : kDefaultMinBlocks;
+}
+
 // The variant of a size class: the autotuner's choice for the class (pxd_lbfgs_autotune_dev),
 // else PXD_LBFGS_MIN_BLOCKS (| kHistSmem when PXD_LBFGS_HIST_SMEM=1), else the default.
-static int lbfgs_variant_id(const pxd_context* ctx, int cap) {
+static int lbfgs_variant_id(const pxd_context* ctx, int cap, int n_poses) {
     auto it = ctx->lbfgs_tuned.find(class_bound(cap));
     if (it != ctx->lbfgs_tuned.end()) return it->second;
-    static int choice = [] {
+    static const int blocks = [] {
         const char* v = std::getenv("PXD_LBFGS_MIN_BLOCKS");
-        const char* h = std::getenv("PXD_LBFGS_HIST_SMEM");
-        return (v ? std::atoi(v) : kDefaultMinBlocks) | (h && std::atoi(h) ? kHistSmem : 0);
+        return v ? std::atoi(v) : -1;
     }();
-    return choice;
+    static const int flags = [] {
+        const char* h = std::getenv("PXD_LBFGS_HIST_SMEM");
+        return h && std::atoi(h) ? kHistSmem : 0;
+    }();
+    return (blocks >= 0 ? blocks : default_min_blocks(ctx, n_poses)) | flags;
 }
-static LbfgsKernelFn lbfgs_variant(const pxd_context* ctx, int cap, bool dof) {
-    return dof ? dof_kernel() : variant_fn(lbfgs_variant_id(ctx, cap));
+static LbfgsKernelFn lbfgs_variant(const pxd_context* ctx, int cap, int n_poses, bool dof) {
+    return dof ? dof_kernel() : variant_fn(lbfgs_variant_id(ctx, cap, n_poses));
 }
 
 // Padded length of the optimiser's vectors for ligands of up to `cap` atoms: 3 cap + R
@@ -498,11 +512,19 @@ int launch_lbfgs(pxd_context* ctx, const pxd_lbfgs_params& p, int n_poses, int m
                     "shared memory limit");
     if (rc) return rc;
     const bool dof = p.dof_mode == PXD_DOF_RIGID_TORSION;
+    if (!ctx->lbfgs_loaded) {  // a later call of another size finds its variant loaded, also under capture
+        for (int blocks : {0, 3, kDefaultMinBlocks}) {
+            cudaFuncAttributes fa;
+            rc = cuda_check(ctx, cudaFuncGetAttributes(&fa, variant_fn(blocks)), "lbfgs variants");
+            if (rc) return rc;
+        }
+        ctx->lbfgs_loaded = true;
+    }
     for (int cap : caps) {
         Plan q;
         q.cap = cap;
-        q.kern = lbfgs_variant(ctx, cap, dof);
-        q.hist_smem = (lbfgs_variant_id(ctx, cap) & kHistSmem) ? 1 : 0;
+        q.kern = lbfgs_variant(ctx, cap, n_poses, dof);
+        q.hist_smem = (lbfgs_variant_id(ctx, cap, n_poses) & kHistSmem) ? 1 : 0;
         // a pinned shared-memory history that does not fit this class falls back to the slab
         if (q.hist_smem && lbfgs_block_smem(ctx, cap, p.history, true, dof) > static_cast<size_t>(smem_limit))
             q.hist_smem = 0;
@@ -660,7 +682,7 @@ int launch_lbfgs_noalloc(pxd_context* ctx, const pxd_lbfgs_params& p, int n_pose
     a.D_pad = vec_pad(ctx, max_atoms, dof);
     a.X_pad = dof_xpad(ctx, max_atoms, dof);
     const size_t smem = lbfgs_block_smem(ctx, max_atoms, p.history, false, dof);
-    const LbfgsKernelFn kern = lbfgs_variant(ctx, max_atoms, dof);
+    const LbfgsKernelFn kern = lbfgs_variant(ctx, max_atoms, INT_MAX, dof);
     rc = raise_smem_limit(ctx, reinterpret_cast<const void*>(kern), smem, "lbfgs smem attribute");
     if (rc) return rc;
     int per_sm = 0;

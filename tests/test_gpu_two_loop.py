@@ -32,3 +32,25 @@ def test_rows(heavy, seed, atoms):
         assert abs(out["energy"][k] - want["energy"]) <= 1e-3 + 1e-4 * abs(want["energy"])
         np.testing.assert_allclose(out["xyz"][k], want["xyz"], rtol=0, atol=1e-3)
     ctx.close()
+
+
+def test_register_budgets_agree():
+    """A launch's register budget follows its pose count: the same poses end bit for bit the same
+    in launches on both sides of each limit."""
+    torch = pytest.importorskip("torch")
+    native.load(auto_build=True)
+    n_sm = torch.cuda.get_device_properties(0).multi_processor_count
+    rec = model.Receptor.from_json(synth.make_receptor(seed=2, n_heavy=60, cube=16.0, cavity=5.0, n_rotors=1))
+    lig = model.Ligand.from_json(synth.make_ligand(seed=1, n_heavy=9, n_rot=1))
+    ctx = native.Context(0)
+    ctx.set_receptor(rec)
+    ctx.build_grid(model.make_box((0.0, 0.0, 0.0), (12.0, 12.0, 12.0), 0.5), sorted(set(int(t) for t in lig.vdw_type)))
+    lid = ctx.add_ligand(lig)
+    x = lig.poses[0] + np.random.default_rng(0).normal(scale=0.1, size=(12 * n_sm + 1, lig.n_atoms, 3))
+    p = native.lbfgs_params(max_iter=30, history=8)
+    want = ctx.lbfgs(p, lid, x[:5])
+    for n in (8 * n_sm, 8 * n_sm + 1, 12 * n_sm, 12 * n_sm + 1):
+        got = ctx.lbfgs(p, lid, x[:n])
+        for key in ("energy", "nevals", "status", "xyz", "torsions"):
+            np.testing.assert_array_equal(got[key][:5], want[key], err_msg=key)
+    ctx.close()

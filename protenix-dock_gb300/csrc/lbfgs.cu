@@ -163,7 +163,10 @@ struct ScoreArgs {
     int D_pad;
 };
 
-__global__ void __launch_bounds__(kWarpsPerBlock * kWarp) score_kernel(const __grid_constant__ ScoreArgs a) {
+// kMinBlocks > 0 caps the registers for that many blocks per SM (score_variant).
+template <int kMinBlocks>
+__global__ void __launch_bounds__(kWarpsPerBlock * kWarp, kMinBlocks > 0 ? kMinBlocks : 1)
+    score_kernel(const __grid_constant__ ScoreArgs a) {
     extern __shared__ __align__(16) float smem[];
     const int lane = threadIdx.x & (kWarp - 1);
     const int wib = threadIdx.x / kWarp;
@@ -276,6 +279,19 @@ static size_t lbfgs_block_smem(const pxd_context* ctx, int cap, int history, boo
                              dof_xpad(ctx, cap, dof));
 }
 
+// The register budget of a score launch. A warp waits for map gathers most of the time, so more
+// of them help, as long as their shared memory leaves L1 for the maps. 65,536 poses of a
+// 43-atom ligand (19 KB per block): 2.39 ms uncapped (4 blocks), 2.22 / 1.89 / 2.33 ms with 6 /
+// 8 / 10 blocks; 32,768 of 65 atoms (27 KB): 1.73, 1.61 / 1.89 with 6 / 8; of 73 atoms (30 KB):
+// 2.55, 2.38 / 3.45. A batch that is resident at once without a cap keeps it: 1,000 poses take
+// 94 us, and 104 with 8 blocks.
+using ScoreKernelFn = void (*)(ScoreArgs);
+static ScoreKernelFn score_variant(const pxd_context* ctx, int n_poses, size_t block_smem) {
+    if (n_poses <= 4 * kWarpsPerBlock * ctx->n_sm) return score_kernel<0>;
+    if (8 * block_smem <= size_t(152) << 10) return score_kernel<8>;
+    return 6 * block_smem <= size_t(184) << 10 ? score_kernel<6> : score_kernel<0>;
+}
+
 int launch_score(pxd_context* ctx, int n_poses, int max_atoms, const int* lig_ids,
                  const float* xyz, const float* tors, double* energy, float* lig_grad,
                  float* tors_grad, cudaStream_t s) {
@@ -298,15 +314,24 @@ int launch_score(pxd_context* ctx, int n_poses, int max_atoms, const int* lig_id
     a.D_pad = padded(3 * max_atoms + ctx->rec.n_rotors);
     const size_t smem =
         sizeof(float) * kWarpsPerBlock * (pose_bufs_floats(max_atoms, a.n_local) + 2 * a.D_pad);
+    if (!ctx->score_loaded) {  // as for the optimiser's variants
+        for (ScoreKernelFn k : {score_kernel<0>, score_kernel<6>, score_kernel<8>}) {
+            cudaFuncAttributes fa;
+            rc = cuda_check(ctx, cudaFuncGetAttributes(&fa, k), "score variants");
+            if (rc) return rc;
+        }
+        ctx->score_loaded = true;
+    }
+    const ScoreKernelFn kern = score_variant(ctx, n_poses, smem);
     if (smem > 48 * 1024) {
-        rc = raise_smem_limit(ctx, reinterpret_cast<const void*>(score_kernel), smem, "score smem attribute");
+        rc = raise_smem_limit(ctx, reinterpret_cast<const void*>(kern), smem, "score smem attribute");
         if (rc) return rc;
     }
     const int warps = (n_poses + 0);
     int blocks = (warps + kWarpsPerBlock - 1) / kWarpsPerBlock;
     const int cap = ctx->n_sm * 16;
     if (blocks > cap) blocks = cap;
-    score_kernel<<<blocks, kWarpsPerBlock * kWarp, smem, s>>>(a);
+    kern<<<blocks, kWarpsPerBlock * kWarp, smem, s>>>(a);
     return cuda_check(ctx, cudaGetLastError(), "score_kernel launch");
 }
 

@@ -237,6 +237,7 @@ struct pxd_context {
     // autotuned L-BFGS variant (minimum resident blocks per SM) per size-class bound
     std::map<int, int> lbfgs_tuned;
     bool lbfgs_loaded = false;  // lbfgs_kernel's default variants are on the device
+    bool score_loaded = false;  // score_kernel's
     // L2 residency of the maps (pxd_set_l2_residency): persisting set-aside this context
     // holds (0: off) and the device's largest access-policy window
     size_t l2_setaside = 0;

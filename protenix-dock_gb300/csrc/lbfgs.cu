@@ -161,6 +161,7 @@ struct ScoreArgs {
     int n_poses;
     int n_local;
     int D_pad;
+    int split;         // 1 (uncapped variant): two warps per pose, for the gradient and for the energy
 };
 
 // kMinBlocks > 0 caps the registers for that many blocks per SM (score_variant).
@@ -176,11 +177,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, kMinBlocks > 0 ? kMinB
     float* x = base + pose_bufs_floats(a.max_atoms, a.n_local);
     float* g = x + a.D_pad;
     const int R = a.env.rec.n_rotors;
-    const int nw = gridDim.x * kWarpsPerBlock;
-    for (int pose = blockIdx.x * kWarpsPerBlock + wib; pose < a.n_poses; pose += nw) {
+    const int split = kMinBlocks > 0 ? 0 : a.split;
+    const int nw = (gridDim.x * kWarpsPerBlock) >> split;
+    const bool gradient = !split || (wib & 1) == 0, reported = !split || (wib & 1) == 1;
+    for (int pose = (blockIdx.x * kWarpsPerBlock + wib) >> split; pose < a.n_poses; pose += nw) {
         const int lid = a.lig_ids[pose];
         if (lid < 0 || lid >= a.n_ligands || a.ligands[lid].n_atoms > a.max_atoms) {
-            if (lane == 0) a.energy[pose] = nan("");
+            if (lane == 0 && reported) a.energy[pose] = nan("");
             continue;
         }
         const DevLigand L = a.ligands[lid];
@@ -189,14 +192,18 @@ __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, kMinBlocks > 0 ? kMinB
         for (int e = lane; e < 3 * N; e += kWarp) x[e] = px[e];
         for (int r = lane; r < R; r += kWarp) x[3 * N + r] = a.tors[static_cast<size_t>(pose) * R + r];
         __syncwarp();
-        eval_pose_body(a.env, L, x, nullptr, 0.f, g, b, lane);
-        float* og = a.lig_grad + static_cast<size_t>(pose) * a.max_atoms * 3;
-        for (int k = lane; k < 3 * N; k += kWarp) og[k] = g[k];
-        for (int r = lane; r < R; r += kWarp)
-            a.tors_grad[static_cast<size_t>(pose) * R + r] = g[3 * N + r];
+        if (gradient) {
+            eval_pose_body(a.env, L, x, nullptr, 0.f, g, b, lane);
+            float* og = a.lig_grad + static_cast<size_t>(pose) * a.max_atoms * 3;
+            for (int k = lane; k < 3 * N; k += kWarp) og[k] = g[k];
+            for (int r = lane; r < R; r += kWarp)
+                a.tors_grad[static_cast<size_t>(pose) * R + r] = g[3 * N + r];
+        }
         // the energy is the FP64 objective, the gradient the FP32 one
-        const double e = energy64(a.env, a.ligands[lid], x, b, lane);
-        if (lane == 0) a.energy[pose] = e;
+        if (reported) {
+            const double e = energy64(a.env, a.ligands[lid], x, b, lane);
+            if (lane == 0) a.energy[pose] = e;
+        }
         __syncwarp();
     }
 }
@@ -327,7 +334,10 @@ int launch_score(pxd_context* ctx, int n_poses, int max_atoms, const int* lig_id
         rc = raise_smem_limit(ctx, reinterpret_cast<const void*>(kern), smem, "score smem attribute");
         if (rc) return rc;
     }
-    const int warps = (n_poses + 0);
+    // While twice the poses' warps are resident at once, a pose's energy and its gradient are two
+    // warps' work: 88 -> 68 us for 300 poses, 97 -> 77 for 1,000.
+    a.split = n_poses <= 2 * kWarpsPerBlock * ctx->n_sm ? 1 : 0;
+    const int warps = n_poses << a.split;
     int blocks = (warps + kWarpsPerBlock - 1) / kWarpsPerBlock;
     const int cap = ctx->n_sm * 16;
     if (blocks > cap) blocks = cap;

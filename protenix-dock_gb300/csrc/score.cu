@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(kMaxScoreWarps * kWarp) empirical_score_kernel
 //   - r, 1/r and f, 1/f come from one rsqrt each.
 // Every sum has a fixed order, so the energies repeat bit for bit. The work is split over
 // warps (Born sums) and 64 x 64 tiles of atom pairs (energies), which fills the chip at one
-// pose: 8 poses of 42 atoms in a pocket of 1,866 take 2.3 ms of kernel time; with one thread
+// pose: 8 poses of 42 atoms in a pocket of 1,866 take 2.4 ms of kernel time; with one thread
 // per atom and three systems per pose they took 186 ms.
 constexpr double kGbOffset = 0.09;
 constexpr int kGbTile = 64;
@@ -481,9 +481,11 @@ __device__ __forceinline__ double gb_born_term(double4 xi, double sr, double4 xj
     const double U = r + sr;
     if (U < rho) return 0.0;
     const double L = fmax(rho, fabs(r - sr));
-    const double Ui = 1.0 / U, Li = 1.0 / L;
-    const double D = 0.25 * (r - sr * sr * ri) * (Ui * Ui - Li * Li);
-    return 0.5 * (D + (Li - Ui + 0.5 * log(L * Ui + 1e-20) * ri));
+    // one division: 1/L - 1/U and 1/L + 1/U as (U -+ L) / (U L), which also keeps the digits that
+    // the difference of two reciprocals loses
+    const double i = 1.0 / (U * L), d = (U - L) * i;
+    const double D = -0.25 * (r - sr * sr * ri) * (d * ((U + L) * i));
+    return 0.5 * (D + (d + 0.5 * log(L * L * i + 1e-20) * ri));
 }
 
 __device__ __forceinline__ double gb_inverse_born(double sum, double4 p) {
@@ -577,11 +579,34 @@ __device__ __forceinline__ double gb_prefactor(double f) {
     return 0.5 * kGbCoulomb * (1.0 - exp(-kGbKappa * f) / kGbSolvent);
 }
 
-// Pair energies of one 64 x 64 tile (rows bi <= columns bj of the triangle i < j).
+// exp(y) by Tang's table-driven method (ACM Trans. Math. Softw. 15, 144, 1989): y = n ln2 / 128 + r,
+// exp(y) = 2^(n / 128) (1 + p(r)), |r| <= 0.0028, p to r^5 (the next term is 6e-19). table[k] =
+// 2^(k / 128). Ten FP64 operations, within 1 ulp of exp. Beyond |y| = 690, and for NaN, the
+// library's exp.
+constexpr int kExpTable = 128;
+__device__ __forceinline__ double gb_exp(double y, const double* table) {
+    const int top = __double2hiint(y) & 0x7fffffff;
+    if (top > 0x40859000) return exp(y);
+    const double round = 6755399441055744.0;  // 1.5 * 2^52: the sum's low bits are the nearest integer
+    const double t = fma(y, 184.6649652337873, round);
+    const int n = __double2loint(t);
+    const double nd = t - round;
+    const double r = fma(nd, -1.2655086083325438e-13, fma(nd, -0.005415212347998022, y));
+    const double q = fma(r, fma(r, fma(r, 1.0 / 120.0, 1.0 / 24.0), 1.0 / 6.0), 0.5);
+    const double p = fma(q, r * r, r);
+    const double v = table[n & (kExpTable - 1)];
+    const double e = fma(v, p, v);
+    return __hiloint2double(__double2hiint(e) + ((n >> 7) << 20), __double2loint(e));
+}
+
+// Pair energies of one 64 x 64 tile (rows bi <= columns bj of the triangle i < j). The FP64 pipe
+// bounds it (86 % busy), so the operations per pair are what counts: 66 with the library's exp
+// and a division per pair, 45 with gb_exp, the division as a multiplication and the constant
+// factors outside the loop (2.00 -> 1.35 ms for 8 poses in a pocket of 1,866 atoms).
 __global__ void __launch_bounds__(kGbThreads) gb_pair_kernel(const __grid_constant__ GbArgs a) {
     __shared__ double4 s_x[kGbTile];
     __shared__ double s_ib[kGbTile], s_b[kGbTile];
-    __shared__ double s_sum[kGbThreads / kWarp];
+    __shared__ double s_sum[kGbThreads / kWarp], s_exp[kExpTable];
     const GbSystem y = gb_system(a, blockIdx.y);
     const int nb = (y.n + kGbTile - 1) / kGbTile;
     int bi = 0, t = blockIdx.x;
@@ -591,9 +616,11 @@ __global__ void __launch_bounds__(kGbThreads) gb_pair_kernel(const __grid_consta
     const int ni = min(kGbTile, y.n - i0);
     for (int u = threadIdx.x; u < ni; u += kGbThreads) {
         s_x[u] = y.atom(i0 + u);
-        s_ib[u] = y.ib[i0 + u];
-        s_b[u] = 1.0 / s_ib[u];
+        const double ib = y.ib[i0 + u];
+        s_ib[u] = -0.25 * ib;
+        s_b[u] = 1.0 / ib;
     }
+    for (int k = threadIdx.x; k < kExpTable; k += kGbThreads) s_exp[k] = exp2(k * (1.0 / kExpTable));
     __syncthreads();
     double e = 0.0;
     if (j < y.n) {
@@ -604,11 +631,11 @@ __global__ void __launch_bounds__(kGbThreads) gb_pair_kernel(const __grid_consta
             const double4 xi = s_x[u];
             const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
             const double r2 = dx * dx + dy * dy + dz * dz;
-            const double s = r2 + s_b[u] * bj * exp(-0.25 * r2 * (s_ib[u] * ibj)) + 1e-20;
+            const double s = fma(s_b[u] * bj, gb_exp(r2 * (s_ib[u] * ibj), s_exp), r2) + 1e-20;
             const double fi = rsqrt(s);
-            e += xi.w * fi * gb_prefactor(s * fi);
+            e = fma(xi.w * fi, fma(gb_exp(s * fi * -kGbKappa, s_exp), -1.0 / kGbSolvent, 1.0), e);
         }
-        e *= xj.w;
+        e *= xj.w * (0.5 * kGbCoulomb);
     }
     e = gb_lane_sum<kWarp>(e);
     if ((threadIdx.x & (kWarp - 1)) == 0) s_sum[threadIdx.x / kWarp] = e;

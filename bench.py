@@ -1043,7 +1043,7 @@ def main():
         poses = np.concatenate([all_poses[b * N_POSES:(b + 1) * N_POSES] for b in mine])
         del all_poses
     else:
-        rec, lig, box, poses = workload(seed_poses=2)
+        rec, lig, box, poses = workload(seed_poses=2, n_poses=N_POSES)
     ctx = native.Context(local)
     ctx.set_receptor(rec)
     ctx.build_grid(box, sorted(set(int(t) for t in lig.vdw_type)))

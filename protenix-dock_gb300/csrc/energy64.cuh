@@ -4,18 +4,20 @@
 // energy. The optimiser steers on the FP32 evaluation (device_eval.cuh); this evaluation
 // gives the reported number. One warp per pose, every lane returns the same value.
 //
-// The ligand's terms and the map lookups are FP32 pairs (device_pairs.cuh): a pose's
-// coordinates are FP32, so their differences are exact pairs, and every term carries ~1e-13
+// The ligand's larger terms and the map lookups are FP32 pairs (device_pairs.cuh): a pose's
+// coordinates are FP32, so their differences are exact pairs, and such a term carries ~1e-13
 // of itself. In FP64 the pair terms over 1 kcal/mol alone (present in nearly every round of
 // 32) held the FP64 pipe for 20,000 of the 25,000 cycles of a 42-atom pose:
-// score_kernel took 6.6 ms for 65,536 poses.
+// score_kernel took 6.6 ms for 65,536 poses, and takes 1.9 now.
 //
 // Precision per term, against the FP64 objective:
 //   - grid lookups (grid.cpp:197-303): an atom's place in its cell from the box's geometry in
 //     three FP32 parts, weights and sums in pairs, over map energies E = FP32 record + FP32
 //     residual of the FP64 sum (grid build);
-//   - bonds (interaction.cpp:27-47) and intra pairs (pair.h:25-60) of the ligand: pairs, FP64
-//     where atoms nearly coincide or fly apart beyond FP32's range;
+//   - bonds (interaction.cpp:27-47) of the ligand: pairs;
+//   - its intra pairs (pair.h:25-60): FP32 terms up to 1 kcal/mol (each to ~1e-7 of itself,
+//     ~1e-6 kcal/mol a pose), pairs above. Both are FP64 where atoms nearly coincide or fly apart
+//     beyond FP32's range;
 //   - angles and dihedrals (interaction.cpp:49-117): FP32 geometry, sums in pairs. These are
 //     bounded (0.5 k pi^2, 2 sum k): an FP32 angle error of ~1e-7 rad moves a term by at
 //     most k |theta - theta0| 1e-7, ~1e-5 kcal/mol;
@@ -183,9 +185,20 @@ __device__ __forceinline__ void ligand_energy(const DevTopo& t, const float* x, 
     for (int s = lane; s < t.n_pair_slots; s += kWarp) {
         const int2 ij = __ldg(&t.pair_ij[s]);
         if (ij.x < 0) continue;
-        const F2 r2 = atom_distance2(x, ij.x, ij.y);
+        const float4 p = __ldg(&t.pair_p[s]);  // A, C, S2
+        const float3 rij = sub3(pos(ij.y), pos(ij.x));
+        const float d2 = dot3(rij, rij);
+        const float d_1 = rsqrtf(d2);
+        const float v = p.z * d_1 * d_1;
+        const float v6 = v * v * v;
+        const float en = fmaf(p.y, v6 * v6 - v6, p.x * d_1);
+        if (fabsf(en) <= kPairFp64) {
+            pair_acc(e, F2{en, 0.f});
+            continue;
+        }
+        const F2 r2 = atom_distance2(x, ij.x, ij.y);  // also for an infinite or NaN term
         if (r2.h > kPairR2Min && r2.h < kPairR2Max) {
-            const float4 p = __ldg(&t.pair_p[s]), pl = __ldg(&t.pair_lo[s]);  // A, C, S2
+            const float4 pl = __ldg(&t.pair_lo[s]);
             F2 rinv, inv;
             pair_rsqrt(r2, rinv, inv);
             const F2 u = pair_mul(inv, F2{p.z, pl.z});

@@ -449,8 +449,7 @@ int upload_explicit(pxd_context* ctx, const std::vector<int>& atoms, const std::
     offs[4] = pk.put(se64);
     int rc = cuda_check(ctx, cudaMalloc(mem, pk.bytes.size()), "receptor explicit list");
     if (rc) return rc;
-    return cuda_check(ctx, cudaMemcpy(*mem, pk.bytes.data(), pk.bytes.size(), cudaMemcpyHostToDevice),
-                      "receptor explicit copy");
+    return upload(ctx, *mem, pk.bytes.data(), pk.bytes.size(), "receptor explicit copy");
 }
 
 void point_explicit(pxd_context* ctx, bool with_maps) {
@@ -505,9 +504,8 @@ int refresh_ligand_slots(pxd_context* ctx) {
                 slots[a] = s;
             }
         }
-        int rc = cuda_check(ctx, cudaMemcpy(const_cast<int*>(e.dev.map_slot), slots.data(),
-                                            sizeof(int) * e.n_atoms, cudaMemcpyHostToDevice),
-                            "map slot refresh");
+        int rc = upload(ctx, const_cast<int*>(e.dev.map_slot), slots.data(), sizeof(int) * e.n_atoms,
+                        "map slot refresh");
         if (rc) return rc;
     }
     return PXD_OK;
@@ -734,8 +732,7 @@ int pxd_set_receptor(pxd_context* ctx, const pxd_receptor_desc* r) {
     TopoOffsets to = pack_topo(pk, sub);
     int rc = cuda_check(ctx, cudaMalloc(&ctx->rec_mem, pk.bytes.size()), "receptor allocation");
     if (rc) return rc;
-    rc = cuda_check(ctx, cudaMemcpy(ctx->rec_mem, pk.bytes.data(), pk.bytes.size(), cudaMemcpyHostToDevice),
-                    "receptor copy");
+    rc = upload(ctx, ctx->rec_mem, pk.bytes.data(), pk.bytes.size(), "receptor copy");
     if (rc) return rc;
     DevReceptor& d = ctx->rec;
     d.n_rotors = r->n_rotors;
@@ -977,21 +974,18 @@ static int install_map(pxd_context* ctx, const pxd_box* box, int32_t map, const 
         for (int t = 0; t < PXD_NUM_VDW_TYPES; ++t) all.push_back(t);
         int rc = alloc_maps(ctx, box, all);
         if (rc) return rc;
-        rc = cuda_check(ctx, cudaMemset(ctx->maps, 0, (sizeof(float4) + sizeof(float)) * ctx->grid.P * ctx->n_slots),
-                        "map clear");
+        rc = clear(ctx, ctx->maps, (sizeof(float4) + sizeof(float)) * ctx->grid.P * ctx->n_slots, "map clear");
         if (rc) return rc;
     }
     const int slot = map == PXD_NUM_VDW_TYPES ? 0 : ctx->type_slot[map];
-    int rc = cuda_check(ctx, cudaMemcpy(ctx->maps + static_cast<size_t>(slot) * ctx->grid.P, host_records,
-                                        sizeof(float4) * ctx->grid.P, cudaMemcpyHostToDevice),
-                        "map write");
+    int rc = upload(ctx, ctx->maps + static_cast<size_t>(slot) * ctx->grid.P, host_records,
+                    sizeof(float4) * ctx->grid.P, "map write");
     if (rc) return rc;
     float* lo = const_cast<float*>(ctx->grid.e_lo) + static_cast<size_t>(slot) * ctx->grid.P;
     if (e_lo_host)
-        rc = cuda_check(ctx, cudaMemcpy(lo, e_lo_host, sizeof(float) * ctx->grid.P, cudaMemcpyHostToDevice),
-                        "map remainder write");
+        rc = upload(ctx, lo, e_lo_host, sizeof(float) * ctx->grid.P, "map remainder write");
     else  // an installed FP32 record set carries no FP64 remainder: its energies are the records'
-        rc = cuda_check(ctx, cudaMemset(lo, 0, sizeof(float) * ctx->grid.P), "map remainder clear");
+        rc = clear(ctx, lo, sizeof(float) * ctx->grid.P, "map remainder clear");
     if (rc) return rc;
     if (ctx->has_receptor) point_explicit(ctx, true);
     rc = refresh_ligand_slots(ctx);
@@ -1106,7 +1100,7 @@ int pxd_add_ligand(pxd_context* ctx, const pxd_ligand_desc* lig, int32_t* ligand
     LigandEntry e;
     int rc = cuda_check(ctx, cudaMalloc(&e.mem, pk.bytes.size()), "ligand allocation");
     if (rc) return rc;
-    rc = cuda_check(ctx, cudaMemcpy(e.mem, pk.bytes.data(), pk.bytes.size(), cudaMemcpyHostToDevice), "ligand copy");
+    rc = upload(ctx, e.mem, pk.bytes.data(), pk.bytes.size(), "ligand copy");
     if (rc) {
         cudaFree(e.mem);
         return rc;

@@ -341,6 +341,21 @@ inline void queue_copy(pxd_context* ctx, int* rc, void* dst, const void* src, si
     *rc = cuda_check(ctx, cudaMemcpyAsync(dst, src, bytes, kind, s), what);
 }
 
+// Copies to the device before it returns. A pageable copy on the legacy stream may return once
+// its source is staged, and the library's streams do not wait for that stream (they are
+// non-blocking), so a kernel launched next could read what was there before. The copy stays on
+// the legacy stream, behind what a caller launched there.
+inline int upload(pxd_context* ctx, void* dst, const void* src, size_t bytes, const char* what) {
+    const int rc = cuda_check(ctx, cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), what);
+    return rc ? rc : cuda_check(ctx, cudaStreamSynchronize(cudaStreamLegacy), what);
+}
+
+// Zeroes device memory before it returns, like upload.
+inline int clear(pxd_context* ctx, void* dst, size_t bytes, const char* what) {
+    const int rc = cuda_check(ctx, cudaMemset(dst, 0, bytes), what);
+    return rc ? rc : cuda_check(ctx, cudaStreamSynchronize(cudaStreamLegacy), what);
+}
+
 // Waits for the work queued on s, so that no host buffer is released while a copy into it
 // is in flight, and returns the first failure: rc (a copy that failed to queue) before the
 // stream's own.

@@ -169,8 +169,7 @@ int upload_receptor_scoring(pxd_context* ctx, const pxd_score_lists* l, const st
     if (!l) {
         int rc0 = cuda_check(ctx, cudaMalloc(&ctx->rec_score_mem, pk.bytes.size()), "receptor score lists");
         if (rc0) return rc0;
-        rc0 = cuda_check(ctx, cudaMemcpy(ctx->rec_score_mem, pk.bytes.data(), pk.bytes.size(), cudaMemcpyHostToDevice),
-                         "receptor score lists copy");
+        rc0 = upload(ctx, ctx->rec_score_mem, pk.bytes.data(), pk.bytes.size(), "receptor score lists copy");
         if (rc0) return rc0;
         d.pair_rec = at<float4>(ctx->rec_score_mem, o_pair);
         d.all_lc = at<int2>(ctx->rec_score_mem, o_lc);
@@ -231,8 +230,7 @@ int upload_receptor_scoring(pxd_context* ctx, const pxd_score_lists* l, const st
     const size_t o_pcl = pk.put(pcls);
     int rc_ = cuda_check(ctx, cudaMalloc(&ctx->rec_score_mem, pk.bytes.size()), "receptor score lists");
     if (rc_) return rc_;
-    rc_ = cuda_check(ctx, cudaMemcpy(ctx->rec_score_mem, pk.bytes.data(), pk.bytes.size(), cudaMemcpyHostToDevice),
-                     "receptor score lists copy");
+    rc_ = upload(ctx, ctx->rec_score_mem, pk.bytes.data(), pk.bytes.size(), "receptor score lists copy");
     if (rc_) return rc_;
     void* b = ctx->rec_score_mem;
     d.has = 1;
@@ -305,8 +303,7 @@ int upload_ligand_scoring(pxd_context* ctx, LigandEntry& e, const pxd_score_list
     void* b = nullptr;
     int rc = cuda_check(ctx, cudaMalloc(&b, pk.bytes.size()), "ligand score lists");
     if (rc) return rc;
-    rc = cuda_check(ctx, cudaMemcpy(b, pk.bytes.data(), pk.bytes.size(), cudaMemcpyHostToDevice),
-                    "ligand score lists copy");
+    rc = upload(ctx, b, pk.bytes.data(), pk.bytes.size(), "ligand score lists copy");
     if (rc) {
         cudaFree(b);
         return rc;
@@ -814,8 +811,7 @@ int pxd_set_scoring_function(pxd_context* ctx, int32_t which, const pxd_sf_param
         int rc = cuda_check(ctx, cudaMalloc(&ctx->d_sf[which], sizeof(DevSf)), "scoring function");
         if (rc) return rc;
     }
-    int rc = cuda_check(ctx, cudaMemcpy(ctx->d_sf[which], &h, sizeof(DevSf), cudaMemcpyHostToDevice),
-                        "scoring function copy");
+    int rc = upload(ctx, ctx->d_sf[which], &h, sizeof(DevSf), "scoring function copy");
     if (rc) return rc;
     ctx->sf_host[which] = *p;
     ctx->sf_set[which] = true;

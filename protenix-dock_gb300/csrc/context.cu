@@ -761,9 +761,11 @@ int pxd_set_receptor(pxd_context* ctx, const pxd_receptor_desc* r) {
     point_explicit(ctx, false);
     rc = upload_receptor_scoring(ctx, r->lists, local_of);
     if (rc) return rc;
+    rc = build_score_tables(ctx);
+    if (rc) return rc;
     ctx->has_receptor = true;
     ctx->ligands_dirty = true;
-    return build_score_tables(ctx);
+    return PXD_OK;
 }
 
 int pxd_decide_grid_dims(double cx, double cy, double cz, double sx, double sy, double sz,

@@ -347,20 +347,28 @@ __global__ void score_vdw_kernel(const DevSf* sf, const float2* cls, int n_cls, 
     out[k] = make_float2((ti.x + se.x) * 0.5f, sqrtf(ti.y * se.y) * 4.f);
 }
 
-// (Re)builds the tables of the installed scoring functions for the installed receptor.
+static int alloc_score_table(pxd_context* ctx, float2** out) {
+    const size_t n = static_cast<size_t>(PXD_NUM_VDW_TYPES) * ctx->rec_score.n_cls;
+    return cuda_check(ctx, cudaMalloc(out, sizeof(float2) * std::max<size_t>(n, 1)), "score tables");
+}
+
+static int fill_score_table(pxd_context* ctx, int w, float2* out) {
+    const int n = PXD_NUM_VDW_TYPES * ctx->rec_score.n_cls;
+    if (n > 0)
+        score_vdw_kernel<<<(n + 127) / 128, 128, 0, ctx->stream>>>(ctx->d_sf[w], ctx->rec_score.cls_se,
+                                                                   ctx->rec_score.n_cls, out);
+    const int rc = cuda_check(ctx, cudaGetLastError(), "score_vdw_kernel launch");
+    return rc ? rc : cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "score tables");
+}
+
+// The tables of the installed scoring functions for a receptor that is being installed (they are
+// freed with it). A context that has a receptor and a scoring function has their table: the
+// callers set either only once it stands.
 int build_score_tables(pxd_context* ctx) {
     for (int w = 0; w < 2; ++w) {
-        if (!ctx->sf_set[w] || !ctx->has_receptor) continue;
-        const int n = PXD_NUM_VDW_TYPES * ctx->rec_score.n_cls;
-        if (ctx->d_vdw[w]) cudaFree(ctx->d_vdw[w]);
-        ctx->d_vdw[w] = nullptr;
-        int rc = cuda_check(ctx, cudaMalloc(&ctx->d_vdw[w], sizeof(float2) * std::max(n, 1)), "score tables");
-        if (rc) return rc;
-        if (n > 0)
-            score_vdw_kernel<<<(n + 127) / 128, 128, 0, ctx->stream>>>(ctx->d_sf[w], ctx->rec_score.cls_se,
-                                                                       ctx->rec_score.n_cls, ctx->d_vdw[w]);
-        rc = cuda_check(ctx, cudaGetLastError(), "score_vdw_kernel launch");
-        if (!rc) rc = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "score tables");
+        if (!ctx->sf_set[w]) continue;
+        int rc = alloc_score_table(ctx, &ctx->d_vdw[w]);
+        if (!rc) rc = fill_score_table(ctx, w, ctx->d_vdw[w]);
         if (rc) return rc;
     }
     return PXD_OK;
@@ -811,11 +819,22 @@ int pxd_set_scoring_function(pxd_context* ctx, int32_t which, const pxd_sf_param
         int rc = cuda_check(ctx, cudaMalloc(&ctx->d_sf[which], sizeof(DevSf)), "scoring function");
         if (rc) return rc;
     }
-    int rc = upload(ctx, ctx->d_sf[which], &h, sizeof(DevSf), "scoring function copy");
+    // the new table's memory first: without it, the function and table that were there stay
+    float2* table = nullptr;
+    int rc = ctx->has_receptor ? alloc_score_table(ctx, &table) : PXD_OK;
     if (rc) return rc;
+    ctx->sf_set[which] = false;
+    rc = upload(ctx, ctx->d_sf[which], &h, sizeof(DevSf), "scoring function copy");
+    if (!rc && table) rc = fill_score_table(ctx, which, table);
+    if (rc) {
+        if (table) cudaFree(table);
+        return rc;
+    }
+    if (ctx->d_vdw[which]) cudaFree(ctx->d_vdw[which]);
+    ctx->d_vdw[which] = table;
     ctx->sf_host[which] = *p;
     ctx->sf_set[which] = true;
-    return build_score_tables(ctx);
+    return PXD_OK;
 }
 
 int pxd_score_dev(pxd_context* ctx, int32_t which, int32_t n_poses, int32_t max_atoms, const int32_t* ids,

@@ -247,9 +247,10 @@ extern "C" {
 int pxd_score_weight_grad_dev(pxd_context* ctx, int32_t n_poses, const double* features, const double* grad_out,
                               const double* weights, double* dweights, void* stream) {
     if (!ctx) return PXD_ERR_INVALID;
-    if (n_poses < 0 || !features || !grad_out || !weights || !dweights)
+    if (n_poses < 0) return set_error(ctx, PXD_ERR_INVALID, "bad weight gradient batch");
+    if (n_poses == 0) return PXD_OK;  // an empty batch's arrays have no address
+    if (!features || !grad_out || !weights || !dweights)
         return set_error(ctx, PXD_ERR_INVALID, "bad weight gradient batch");
-    if (n_poses == 0) return PXD_OK;
     cudaSetDevice(ctx->device);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
     const int blocks = std::min((n_poses + 7) / 8, 1024);

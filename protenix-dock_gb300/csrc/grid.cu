@@ -10,28 +10,30 @@
 // few types per walk and combines the sums into their energies.
 //
 // Precision. FP64 runs at 1/64 of FP32 here and bounded the build (84 % of the FP64 pipe busy)
-// when the Coulomb terms and the LJ terms near a point were FP64 per (point, map). The pair
-// terms of grid_moment_kernel are FP32 pairs (hi + lo, ~47 bits, products by fma, sums by
-// two-sum) instead:
-//   - atom and point coordinates are split into a hi part on a common power-of-two grid, so
-//     that the difference of two hi parts is exact, and an FP32 remainder (~2^-44 A);
-//   - 1/r comes from the FP32 rsqrt with a third-order correction in pairs;
-//   - r^-6 and r^-12 of atoms closer than 2 A are formed and summed in FP64 from the FP64
-//     coordinates (the 12th power of a clash amplifies the coordinates' rounding most);
+// when the Coulomb terms and the LJ terms near a point were FP64 per (point, map). The terms
+// of grid_moment_kernel are FP32 pairs and triples instead (device_pairs.cuh):
+//   - atom and point coordinates are split into three parts, two of them on common power-of-two
+//     grids, so that the differences of these parts are exact;
+//   - the Coulomb energy is formed and summed in triples: its q/r terms of both signs cancel to
+//     a small part of their size, and 1,900 terms of ~7 kcal/mol a unit charge in pairs left
+//     1e-12 kcal/mol. The triple sum, and the pair sums of the gradient, are folded into FP64
+//     every kMomentTile atoms;
+//   - r^-6 and r^-12 are pairs; of atoms closer than 2 A they are formed and summed in FP64 from
+//     the FP64 coordinates (the 12th power of a clash amplifies the coordinates' rounding most);
 //   - the classes' energies are combined in FP64, and kept as the FP32 record and the FP32
 //     remainder below it.
-// The Coulomb map needs the pairs throughout: its q/r terms of both signs cancel to a small
-// part of their size. Against FP64 sums over the same points the LJ energies are off by
-// 3e-15 of themselves in the median (4e-13 before) and 1e-11 kcal/mol where |E| < 10 (1e-7
-// before, when the terms under 1e-2 kcal/mol were plain FP32); the Coulomb energies of a unit
-// charge by 2e-11 kcal/mol (3e-13 before; 1e-15 of the sum of the terms' sizes).
+// Against exact sums over the same points, 1,866 atoms, points off the atoms: the Coulomb
+// energies of a unit charge are off by 1.1e-13 kcal/mol in the median and 7e-13 at most, with
+// or without an atom far away (4e-13 and 5e-12 with an FP64 loop over coordinates of two FP32
+// parts); the LJ energies by 3e-15 of themselves in the median, 1e-11 kcal/mol where |E| < 10.
 // The LJ gradients are FP32 per pair from hi + lo coordinate differences, folded into FP64
 // every kGridTile atoms. Squared distances are floored at 1e-4 A^2 (a point that sits on an
 // atom cannot overflow FP32) and records clamped to +-1e30 before the FP32 store.
 //
-// Measured, 81^3 points x 1,866 atoms: 12 maps in 11.1 ms (104 ms with FP64 terms per point and
-// map): 5.0 ms for grid_moment_kernel and 3.0 ms for each walk of grid_lj_kernel over 6 types,
-// both near the FP32 issue rate; all 99 types over 55 x 49 x 53 points in 15.9 ms (240 ms).
+// Measured, 81^3 points x 1,866 atoms: 12 maps in 15.5 ms (104 ms with FP64 terms per point and
+// map): 9.4 ms for grid_moment_kernel (5.0 with Coulomb terms in pairs) and 3.0 ms for each
+// walk of grid_lj_kernel over 6 types, both near the FP32 issue rate; all 99 types over
+// 55 x 49 x 53 points in 17.0 ms (240 ms).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -78,8 +80,9 @@ struct LjAtoms {
 };
 
 struct GridArgs {
-    const float4* hi;        // class order: coordinates on the hi grid relative to `origin`, charge
-    const float4* lo;        // remainders
+    const float4* hi;        // class order: first parts of the coordinates relative to `origin`, and charge
+    const float4* lo;        // second parts
+    const float4* rest;      // third parts of the coordinates
     const double4* x64;      // FP64 coordinates
     const GridClass* classes;
     int n_classes, n_slots;  // n_slots: classes with sums
@@ -111,31 +114,54 @@ __device__ __forceinline__ void store_record(const GridArgs& a, int slot, int p,
 }
 
 struct PointSums {
-    F2 e, x, y, z;     // Coulomb energy and gradient
+    F3 e;              // Coulomb energy
+    F2 x, y, z;        // and gradient
     F2 m6, m12;        // LJ sums of the current class
     double m6d, m12d;  // its atoms within 2 A
 };
 
 __device__ __forceinline__ double to_double(F2 a) { return static_cast<double>(a.h) + static_cast<double>(a.l); }
-
-// a.hi - p.hi and the remainder of the difference. kWide: the hi parts are not on a common
-// grid, so the difference's rounding is formed too (two-sum).
-template <bool kWide>
-__device__ __forceinline__ F2 coord_diff(float ah, float al, float ph, float pl) {
-    if (kWide) return pair_sub({ah, al}, {ph, pl});
-    return {__fsub_rn(ah, ph), __fsub_rn(al, pl)};
+__device__ __forceinline__ double to_double(F3 a) {
+    return static_cast<double>(a.h) + (static_cast<double>(a.l) + static_cast<double>(a.m));
 }
 
-// Adds one receptor atom to the sums of the point (ph + pl, FP64 p64).
+// One coordinate of an atom or a point as three parts. The first two on the grids of `step` and
+// 2^-24 step, so that the differences of two of them are exact; kWide: each the rounding of
+// what is left.
+template <bool kWide>
+__host__ __device__ __forceinline__ F3 coord_parts(double r, double step, double step_inv) {
+    constexpr double k24 = 16777216.0;
+    const double h = kWide ? static_cast<double>(static_cast<float>(r)) : rint(r * step_inv) * step;
+    const double d = r - h;
+    const double l = kWide ? static_cast<double>(static_cast<float>(d)) : rint(d * step_inv * k24) * (step / k24);
+    return {static_cast<float>(h), static_cast<float>(l), static_cast<float>(d - l)};
+}
+
+// a - p, its first part carrying the leading bits.
+template <bool kWide>
+__device__ __forceinline__ F3 coord_diff(float ah, float al, float am, F3 p) {
+    float h = __fsub_rn(ah, p.h), l = __fsub_rn(al, p.l), m = __fsub_rn(am, p.m);
+    if (kWide) {
+        const F2 e = two_diff(ah, p.h), g = two_diff(al, p.l);
+        const F2 k = two_sum(e.l, g.h);
+        h = e.h;
+        l = k.h;
+        m = __fadd_rn(m, __fadd_rn(k.l, g.l));
+    }
+    const float s = __fadd_rn(h, l);
+    return {s, __fsub_rn(l, __fsub_rn(s, h)), m};
+}
+
+// Adds one receptor atom to the sums of the point (px, py, pz; FP64 p64).
 template <bool kLj, bool kWide>
-__device__ __forceinline__ void grid_pair(const float4 ah, const float4 al, const double4* x64, float3 ph, float3 pl,
-                                          double3 p64, PointSums& s) {
-    const F2 dx = coord_diff<kWide>(ah.x, al.x, ph.x, pl.x), dy = coord_diff<kWide>(ah.y, al.y, ph.y, pl.y),
-             dz = coord_diff<kWide>(ah.z, al.z, ph.z, pl.z);
-    F2 r2 = pair_norm2(dx, dy, dz);
+__device__ __forceinline__ void grid_pair(const float4 ah, const float4 al, const float4 am, const double4* x64, F3 px,
+                                          F3 py, F3 pz, double3 p64, PointSums& s) {
+    const F3 dx = coord_diff<kWide>(ah.x, al.x, am.x, px), dy = coord_diff<kWide>(ah.y, al.y, am.y, py),
+             dz = coord_diff<kWide>(ah.z, al.z, am.z, pz);
+    F3 r2 = triple_norm2(dx, dy, dz);
     const bool near = r2.h < kNearR2;
     if (near) {
-        if (r2.h < kR2Floor) r2 = {kR2Floor, 0.f};
+        if (r2.h < kR2Floor) r2 = {kR2Floor, 0.f, 0.f};
         if (kLj) {
             const double4 x = *x64;
             const double ux = x.x - p64.x, uy = x.y - p64.y, uz = x.z - p64.z;
@@ -145,15 +171,15 @@ __device__ __forceinline__ void grid_pair(const float4 ah, const float4 al, cons
             s.m12d += n6 * n6;
         }
     }
-    F2 rinv, inv;
-    pair_rsqrt(r2, rinv, inv);
+    F3 rinv;
+    F2 inv;
+    triple_rsqrt(r2, rinv, inv);
     // Coulomb: q/r and q (x - p)/r^3
-    const F2 q = pair_mul({ah.w, al.w}, rinv);
-    pair_acc(s.e, q);
+    const F2 q = triple_acc(s.e, {ah.w, al.w}, rinv);
     const F2 w = pair_mul(q, inv);
-    pair_acc(s.x, pair_mul(dx, w));
-    pair_acc(s.y, pair_mul(dy, w));
-    pair_acc(s.z, pair_mul(dz, w));
+    pair_acc(s.x, pair_mul(F2{dx.h, dx.l}, w));
+    pair_acc(s.y, pair_mul(F2{dy.h, dy.l}, w));
+    pair_acc(s.z, pair_mul(F2{dz.h, dz.l}, w));
     if (kLj) {
         F2 i6 = pair_mul(pair_square(inv), inv);
         F2 i12 = pair_square(i6);
@@ -164,12 +190,13 @@ __device__ __forceinline__ void grid_pair(const float4 ah, const float4 al, cons
 }
 
 // One thread per point, 128 consecutive points (k fastest) per block, so that every thread
-// reads the same atom of a shared-memory tile (broadcast). About 150 FP32 operations a pair:
+// reads the same atom of a shared-memory tile (broadcast). About 280 FP32 operations a pair:
 // bound by FP32 issue.
 template <bool kWide>
 __global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_constant__ GridArgs a) {
     __shared__ float4 s_hi[kMomentTile];
     __shared__ float4 s_lo[kMomentTile];
+    __shared__ float4 s_rest[kMomentTile];
     const int t = blockIdx.x * kGridThreads + threadIdx.x;
     const int p = a.p0 + t;
     const int nz = a.npts.z, ny = a.npts.y;
@@ -178,13 +205,11 @@ __global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_
     const int i = p / (nz * ny);
     // grid.cpp:159-163: point = init + spacing * index, formed in FP64
     const double3 p64 = make_double3(a.init.x + a.spacing * i, a.init.y + a.spacing * j, a.init.z + a.spacing * k);
-    const double rx = p64.x - a.origin.x, ry = p64.y - a.origin.y, rz = p64.z - a.origin.z;
-    auto hi_part = [&a](double r) { return kWide ? static_cast<double>(static_cast<float>(r)) : rint(r * a.step_inv) * a.step; };
-    const double hx = hi_part(rx), hy = hi_part(ry), hz = hi_part(rz);
-    const float3 ph = make_float3(static_cast<float>(hx), static_cast<float>(hy), static_cast<float>(hz));
-    const float3 pl = make_float3(static_cast<float>(rx - hx), static_cast<float>(ry - hy), static_cast<float>(rz - hz));
+    const F3 px = coord_parts<kWide>(p64.x - a.origin.x, a.step, a.step_inv);
+    const F3 py = coord_parts<kWide>(p64.y - a.origin.y, a.step, a.step_inv);
+    const F3 pz = coord_parts<kWide>(p64.z - a.origin.z, a.step, a.step_inv);
     PointSums s{};
-    double E = 0.0;
+    double E = 0.0, GX = 0.0, GY = 0.0, GZ = 0.0;
     for (int c = 0; c < a.n_classes; ++c) {
         const GridClass gc = a.classes[c];
         for (int t0 = 0; t0 < gc.count; t0 += kMomentTile) {
@@ -194,16 +219,23 @@ __global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_
             for (int u = threadIdx.x; u < n; u += kGridThreads) {
                 s_hi[u] = a.hi[base + u];
                 s_lo[u] = a.lo[base + u];
+                s_rest[u] = a.rest[base + u];
             }
             __syncthreads();
             if (gc.slot >= 0) {
-                for (int u = 0; u < n; ++u) grid_pair<true, kWide>(s_hi[u], s_lo[u], a.x64 + base + u, ph, pl, p64, s);
+                for (int u = 0; u < n; ++u)
+                    grid_pair<true, kWide>(s_hi[u], s_lo[u], s_rest[u], a.x64 + base + u, px, py, pz, p64, s);
             } else {
-                for (int u = 0; u < n; ++u) grid_pair<false, kWide>(s_hi[u], s_lo[u], nullptr, ph, pl, p64, s);
+                for (int u = 0; u < n; ++u)
+                    grid_pair<false, kWide>(s_hi[u], s_lo[u], s_rest[u], nullptr, px, py, pz, p64, s);
             }
-            // the low part of a long sum would round at ~1e-11 kcal/mol
+            // the low part of a long sum would round by more than its terms do
             E += to_double(s.e);
-            s.e = {0.f, 0.f};
+            GX += to_double(s.x);
+            GY += to_double(s.y);
+            GZ += to_double(s.z);
+            s.e = {0.f, 0.f, 0.f};
+            s.x = s.y = s.z = {0.f, 0.f};
         }
         if (gc.slot >= 0) {
             if (t < a.n_points) {
@@ -216,8 +248,8 @@ __global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_
         }
     }
     if (t < a.n_points) {
-        store_record(a, 0, p, E * kCoulombD, clampf_rec(to_double(s.x) * kCoulombD), clampf_rec(to_double(s.y) * kCoulombD),
-                     clampf_rec(to_double(s.z) * kCoulombD));
+        store_record(a, 0, p, E * kCoulombD, clampf_rec(GX * kCoulombD), clampf_rec(GY * kCoulombD),
+                     clampf_rec(GZ * kCoulombD));
     }
 }
 
@@ -352,7 +384,7 @@ int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
     const bool wide = reach >= kGridReach;
     a.step = std::ldexp(1.0, std::ilogb(std::max(reach, 1.0)) + 1 - 24);
     a.step_inv = 1.0 / a.step;
-    std::vector<float4> hi, lo;
+    std::vector<float4> hi, lo, rest;
     std::vector<double4> x64;
     std::vector<GridClass> classes;
     std::vector<int> order;  // receptor atoms in class order
@@ -364,17 +396,15 @@ int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
         if (lj) kinds.push_back(kind);
         for (int i : atoms) {
             order.push_back(i);
-            float h[4], l[4];
+            F3 x[3];
             for (int d = 0; d < 3; ++d) {
                 const double r = ctx->rec_xyz[3 * i + d] - (&a.origin.x)[d];
-                const double g = wide ? static_cast<double>(static_cast<float>(r)) : std::rint(r * a.step_inv) * a.step;
-                h[d] = static_cast<float>(g);
-                l[d] = static_cast<float>(r - g);
+                x[d] = wide ? coord_parts<true>(r, a.step, a.step_inv) : coord_parts<false>(r, a.step, a.step_inv);
             }
-            h[3] = static_cast<float>(ctx->rec_charge[i]);
-            l[3] = static_cast<float>(ctx->rec_charge[i] - h[3]);
-            hi.push_back(make_float4(h[0], h[1], h[2], h[3]));
-            lo.push_back(make_float4(l[0], l[1], l[2], l[3]));
+            const float q = static_cast<float>(ctx->rec_charge[i]);
+            hi.push_back(make_float4(x[0].h, x[1].h, x[2].h, q));
+            lo.push_back(make_float4(x[0].l, x[1].l, x[2].l, static_cast<float>(ctx->rec_charge[i] - q)));
+            rest.push_back(make_float4(x[0].m, x[1].m, x[2].m, 0.f));
             x64.push_back(make_double4(ctx->rec_xyz[3 * i], ctx->rec_xyz[3 * i + 1], ctx->rec_xyz[3 * i + 2], 0.0));
         }
     }
@@ -423,7 +453,7 @@ int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
         if (bytes) std::memcpy(in.data() + off, v.data(), bytes);
         return off;
     };
-    const size_t o_hi = put(hi), o_lo = put(lo), o_x = put(x64), o_cls = put(classes), o_coef = put(coef);
+    const size_t o_hi = put(hi), o_lo = put(lo), o_rest = put(rest), o_x = put(x64), o_cls = put(classes), o_coef = put(coef);
     const size_t o_lh = put(lj_hi), o_ll = put(lj_lo), o_tile = put(tiles), o_kind = put(kind_se), o_type = put(type_se);
     cudaStream_t s = ctx->stream;
     char* mem = nullptr;
@@ -433,6 +463,7 @@ int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
     queue_copy(ctx, &rc, mem, in.data(), in.size(), cudaMemcpyHostToDevice, s, "map build inputs");
     a.hi = reinterpret_cast<const float4*>(mem + o_hi);
     a.lo = reinterpret_cast<const float4*>(mem + o_lo);
+    a.rest = reinterpret_cast<const float4*>(mem + o_rest);
     a.x64 = reinterpret_cast<const double4*>(mem + o_x);
     a.classes = reinterpret_cast<const GridClass*>(mem + o_cls);
     a.coef = reinterpret_cast<const FoldCoef*>(mem + o_coef);

@@ -831,7 +831,10 @@ static int alloc_maps(pxd_context* ctx, const pxd_box* box, const std::vector<in
     for (int d = 0; d < 3; ++d) split_parts(box->init_xyz[d], g.init_p[d], 3);
     split_parts(box->spacing, g.spacing_p, 3);
     split_parts(1.0 / box->spacing, g.spacing_inv_p, 2);
-    split_parts(ctx->slope, g.slope_p, 2);
+    g.init64 = make_double3(box->init_xyz[0], box->init_xyz[1], box->init_xyz[2]);
+    g.spacing64 = box->spacing;
+    g.spacing_inv64 = 1.0 / box->spacing;
+    g.slope64 = ctx->slope;
     return PXD_OK;
 }
 
@@ -881,7 +884,7 @@ int pxd_grid_set_slope(pxd_context* ctx, double slope) {
     if (!ctx) return PXD_ERR_INVALID;
     ctx->slope = slope;
     ctx->grid.slope = static_cast<float>(slope);
-    split_parts(slope, ctx->grid.slope_p, 2);
+    ctx->grid.slope64 = slope;
     return PXD_OK;
 }
 

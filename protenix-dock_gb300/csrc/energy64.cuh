@@ -4,20 +4,24 @@
 // energy. The optimiser steers on the FP32 evaluation (device_eval.cuh); this evaluation
 // gives the reported number. One warp per pose, every lane returns the same value.
 //
-// The ligand's larger terms and the map lookups are FP32 pairs (device_pairs.cuh): a pose's
-// coordinates are FP32, so their differences are exact pairs, and such a term carries ~1e-13
-// of itself. In FP64 the pair terms over 1 kcal/mol alone (present in nearly every round of
-// 32) held the FP64 pipe for 20,000 of the 25,000 cycles of a 42-atom pose:
-// score_kernel took 6.6 ms for 65,536 poses, and takes 1.9 now.
+// The ligand's moderate terms and the map lookups are FP32 pairs (device_pairs.cuh): a pose's
+// coordinates are FP32, so their differences are exact pairs. In FP64 the pair terms over
+// 1 kcal/mol alone (present in nearly every round of 32) held the FP64 pipe for 20,000 of
+// the 25,000 cycles of a 42-atom pose: score_kernel took 6.6 ms for 65,536 poses, and takes 2.2.
 //
 // Precision per term, against the FP64 objective:
 //   - grid lookups (grid.cpp:197-303): an atom's place in its cell from the box's geometry in
-//     three FP32 parts, weights and sums in pairs, over map energies E = FP32 record + FP32
-//     residual of the FP64 sum (grid build);
+//     three FP32 parts, weights and the cell's sum in pairs, over map energies E = FP32
+//     record + FP32 residual of the FP64 sum (grid build): 6e-16 of the cell's largest energy
+//     in the median (1.2e-15 with weights from an FP64 place in the box, whose fraction of a
+//     cell rounds at 1e-14). The penalty of an atom outside is FP64;
 //   - bonds (interaction.cpp:27-47) of the ligand: pairs;
-//   - its intra pairs (pair.h:25-60): FP32 terms up to 1 kcal/mol (each to ~1e-7 of itself,
-//     ~1e-6 kcal/mol a pose), pairs above. Both are FP64 where atoms nearly coincide or fly apart
-//     beyond FP32's range;
+//   - its intra pairs (pair.h:25-60): FP32 terms up to 1 kcal/mol, with ~1e-6 of their larger
+//     part (Coulomb or LJ; the 12th power multiplies the rounding of 1/r twelvefold), pairs
+//     above, with ~2e-13 of themselves;
+//   - terms and lookups over kPairTop, of coincident atoms or of atoms flung apart: FP64, and
+//     summed in FP64, so that what pairs round off stays below 1e-8 kcal/mol, a hundredth of
+//     what FP32 angles leave;
 //   - angles and dihedrals (interaction.cpp:49-117): FP32 geometry, sums in pairs. These are
 //     bounded (0.5 k pi^2, 2 sum k): an FP32 angle error of ~1e-7 rad moves a term by at
 //     most k |theta - theta0| 1e-7, ~1e-5 kcal/mol;
@@ -52,7 +56,8 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 }
 
 constexpr double kCoulombD64 = 332.0637141491396;  // kCoulombFactor, system.h:83
-constexpr float kPairFp64 = 1.f;                   // kcal/mol: larger pair terms go FP64
+constexpr float kPairFp64 = 1.f;                   // kcal/mol: larger FP32 terms are recomputed
+constexpr float kPairTop = 1e4f;                   // kcal/mol: larger terms in pairs are FP64
 
 // Pair energy A/r + C((S2/r^2)^6 - (S2/r^2)^3) from FP64 parameters and coordinates.
 __device__ __forceinline__ double pair_energy64(double4 p, D3 xi, D3 xj) {
@@ -122,8 +127,8 @@ __device__ double topo_energy64(const DevTopo& t, const P32& pos32, const P64& p
     return e;
 }
 
-// Squared distances for which a bond or pair term stays in pairs; outside (coincident atoms,
-// whose 12th power leaves FP32's range, or atoms flung apart) it is FP64.
+// Squared distances for which a bond or pair term stays in pairs; outside (coincident atoms, or
+// atoms flung apart) it is FP64.
 constexpr float kPairR2Min = 1e-2f, kPairR2Max = 1e30f;
 
 __device__ __forceinline__ F2 atom_distance2(const float* x, int i, int j) {
@@ -131,8 +136,8 @@ __device__ __forceinline__ F2 atom_distance2(const float* x, int i, int j) {
                       two_diff(x[3 * j + 2], x[3 * i + 2]));
 }
 
-// Energy of the ligand's terms at FP32 coordinates x, added to `e` in pairs; terms out of the
-// pairs' range to `e64`.
+// Energy of the ligand's terms at FP32 coordinates x: terms in pairs added to `e`, FP64 terms to
+// `e64`.
 __device__ __forceinline__ void ligand_energy(const DevTopo& t, const float* x, F2& e, double& e64, int lane) {
     auto pos = [x](int i) { return make_float3(x[3 * i], x[3 * i + 1], x[3 * i + 2]); };
     auto pos64 = [x](int i) {
@@ -147,13 +152,16 @@ __device__ __forceinline__ void ligand_energy(const DevTopo& t, const float* x, 
             F2 rinv, inv;
             pair_rsqrt(r2, rinv, inv);
             const F2 dr = pair_sub(pair_norm(pair_mul(r2, rinv)), {p.y, pl.y});
-            pair_acc(e, pair_mul({0.5f * p.x, 0.5f * pl.x}, pair_square(pair_norm(dr))));
-        } else {
-            const double2 p = __ldg(&t.bond_p64[s]);
-            const D3 d = d3_sub(pos64(ij.y), pos64(ij.x));
-            const double dr = sqrt(d3_dot(d, d)) - p.y;
-            e64 += 0.5 * p.x * (dr * dr);
+            const F2 en = pair_mul({0.5f * p.x, 0.5f * pl.x}, pair_square(pair_norm(dr)));
+            if (en.h <= kPairTop) {
+                pair_acc(e, en);
+                continue;
+            }
         }
+        const double2 p = __ldg(&t.bond_p64[s]);
+        const D3 d = d3_sub(pos64(ij.y), pos64(ij.x));
+        const double dr = sqrt(d3_dot(d, d)) - p.y;
+        e64 += 0.5 * p.x * (dr * dr);
     }
     for (int s = lane; s < t.n_angle_slots; s += kWarp) {
         const int4 ijk = __ldg(&t.angle_ijk[s]);
@@ -196,8 +204,8 @@ __device__ __forceinline__ void ligand_energy(const DevTopo& t, const float* x, 
             pair_acc(e, F2{en, 0.f});
             continue;
         }
-        const F2 r2 = atom_distance2(x, ij.x, ij.y);  // also for an infinite or NaN term
-        if (r2.h > kPairR2Min && r2.h < kPairR2Max) {
+        const F2 r2 = atom_distance2(x, ij.x, ij.y);
+        if (fabsf(en) <= kPairTop && r2.h > kPairR2Min && r2.h < kPairR2Max) {  // not for an infinite or NaN term
             const float4 pl = __ldg(&t.pair_lo[s]);
             F2 rinv, inv;
             pair_rsqrt(r2, rinv, inv);
@@ -211,11 +219,12 @@ __device__ __forceinline__ void ligand_energy(const DevTopo& t, const float* x, 
     }
 }
 
-// One axis of an atom's place in the maps (receptor_cache::get, grid.cpp:211-262): its cell,
-// its fraction of the cell as a pair, and how far beyond the box it is (A, 0 inside).
-__device__ __forceinline__ void grid_place(const float* init, const DevGrid& g, int npts, float p, int& cell, F2& frac,
-                                           F2& beyond) {
+// One axis of an atom's place in the maps (receptor_cache::get, grid.cpp:211-262): its cell and
+// its fraction of the cell as a pair; -1 or 1 if it is below or above the box (the fraction is
+// the face's), also for a coordinate that is not finite.
+__device__ __forceinline__ int grid_place(const float* init, const DevGrid& g, int npts, float at, int& cell, F2& frac) {
     const int last = npts - 2;  // the last cell
+    const float p = fmaxf(fminf(at, 1e9f), -1e9f);
     int c = static_cast<int>(floorf((p - init[0]) * g.spacing_inv));
     c = min(max(c, 0), last);
     // r = p - init - c spacing: the leading parts exactly, the small ones in a pair
@@ -242,31 +251,37 @@ __device__ __forceinline__ void grid_place(const float* init, const DevGrid& g, 
     r = pair_norm(r);
     const F2 over = pair_norm(pair_sub(r, sp));
     cell = c;
-    beyond = {0.f, 0.f};
     if (c == 0 && r.h < 0.f) {
-        beyond = {-r.h, -r.l};
         frac = {0.f, 0.f};
-    } else if (c == last && over.h >= 0.f) {
-        beyond = over;
-        frac = {1.f, 0.f};
-    } else {
-        frac = pair_norm(pair_mul(r, F2{g.spacing_inv_p[0], g.spacing_inv_p[1]}));
+        return -1;
     }
+    if (c == last && over.h >= 0.f) {
+        frac = {1.f, 0.f};
+        return 1;
+    }
+    frac = pair_norm(pair_mul(r, F2{g.spacing_inv_p[0], g.spacing_inv_p[1]}));
+    return 0;
 }
 
-// receptor_cache::get (grid.cpp:197-262) energy in pairs for an atom of charge q at p.
+// How far a coordinate lies outside the box on the given side, in cells.
+__device__ __forceinline__ double grid_beyond(const DevGrid& g, double from_init, int side, int npts) {
+    const double f = from_init * g.spacing_inv64;
+    return side < 0 ? -f : f - (npts - 1);
+}
+
+// receptor_cache::get (grid.cpp:197-262) energy for an atom of charge q at p.
 __device__ __forceinline__ void grid_energy(const DevGrid& g, int slot, F2 q, float3 p, F2& e, double& e64) {
     int cx, cy, cz;
-    F2 x, y, z, bx, by, bz;
-    grid_place(g.init_p[0], g, g.npts.x, p.x, cx, x, bx);
-    grid_place(g.init_p[1], g, g.npts.y, p.y, cy, y, by);
-    grid_place(g.init_p[2], g, g.npts.z, p.z, cz, z, bz);
-    pair_acc(bx, by);
-    pair_acc(bx, bz);
-    if (bx.h > 0.f && bx.h < 1e25f)
-        pair_acc(e, pair_mul(pair_norm(bx), F2{g.slope_p[0], g.slope_p[1]}));
-    else if (bx.h > 0.f)  // an atom flung so far that the penalty could leave FP32's range
-        e64 += static_cast<double>(bx.h) * (static_cast<double>(g.slope_p[0]) + static_cast<double>(g.slope_p[1]));
+    F2 x, y, z;
+    const int ox = grid_place(g.init_p[0], g, g.npts.x, p.x, cx, x), oy = grid_place(g.init_p[1], g, g.npts.y, p.y, cy, y),
+              oz = grid_place(g.init_p[2], g, g.npts.z, p.z, cz, z);
+    if (ox | oy | oz) {
+        double out = 0.0;
+        if (ox) out += grid_beyond(g, p.x - g.init64.x, ox, g.npts.x);
+        if (oy) out += grid_beyond(g, p.y - g.init64.y, oy, g.npts.y);
+        if (oz) out += grid_beyond(g, p.z - g.init64.z, oz, g.npts.z);
+        if (out > 0.0) e64 += out * g.spacing64 * g.slope64;
+    }
     const F2 one{1.f, 0.f};
     const F2 mx = pair_norm(pair_sub(one, x)), my = pair_norm(pair_sub(one, y)), mz = pair_norm(pair_sub(one, z));
     const F2 xy[4] = {pair_mul(mx, my), pair_mul(x, my), pair_mul(mx, y), pair_mul(x, y)};
@@ -281,11 +296,14 @@ __device__ __forceinline__ void grid_energy(const DevGrid& g, int slot, F2 q, fl
         pair_acc(ec, pair_mul(w, F2{__ldg(&g.maps[off].x), __ldg(&g.e_lo[off])}));
         if (slot > 0) pair_acc(ev, pair_mul(w, F2{__ldg(&g.maps[slot * P + off].x), __ldg(&g.e_lo[slot * P + off])}));
     }
-    pair_acc(e, pair_mul(pair_norm(ec), q));
-    pair_acc(e, ev);
+    pair_acc(ev, pair_mul(pair_norm(ec), q));
+    if (fabsf(ev.h) <= kPairTop)
+        pair_acc(e, ev);
+    else
+        e64 += static_cast<double>(ev.h) + static_cast<double>(ev.l);
 }
 
-// FP64 energy of the pose x = [ligand xyz (3N) | receptor torsions] (shared memory, the
+// Reported energy of the pose x = [ligand xyz (3N) | receptor torsions] (shared memory, the
 // optimiser's flat layout). b.loc_grad serves as scratch for the FP64 positions of the
 // receptor's local atoms (24 of its 64 bytes per atom); the next evaluation clears it.
 static __device__ __noinline__ double energy64(const EvalEnv& env, const DevLigand& L, const float* x,

@@ -165,11 +165,13 @@ struct DevGrid {
     float slope;
     int P;
     const float4* maps;
-    // the reported energy: box geometry and slope as sums of FP32 parts (init and spacing in
-    // three, 1/spacing and slope in two), and per map point the FP64 energy's residual below
-    // its FP32 record, E = maps[.].x + e_lo[.]
+    // the reported energy: box geometry and slope in FP64 and as sums of FP32 parts (init and
+    // spacing in three, 1/spacing in two), and per map point the FP64 energy's residual
+    // below its FP32 record, E = maps[.].x + e_lo[.]
+    double3 init64;
+    double spacing64, spacing_inv64, slope64;
     float init_p[3][3];       // [axis][part]
-    float spacing_p[3], spacing_inv_p[2], slope_p[2];
+    float spacing_p[3], spacing_inv_p[2];
     const float* e_lo;        // [n_slots][P]
 };
 

@@ -51,6 +51,7 @@ constexpr int kMomentTile = 128;
 constexpr int kGridTile = 256;  // atoms per FP32 partial sum of the LJ gradients
 constexpr float kR2Floor = 1e-4f;
 constexpr float kNearR2 = 4.f;  // A^2: closer atoms' LJ powers are FP64
+constexpr float kFarR2 = 1e30f;  // A^2: farther atoms, whose squares FP32 does not hold, are FP64
 // Systems that reach further than this from an atom to a point (A) give up the common hi
 // grid, whose step would grow with them (an outlying atom would cost every point precision),
 // for two-sum differences: 15 operations a pair more.
@@ -83,7 +84,7 @@ struct GridArgs {
     const float4* hi;        // class order: first parts of the coordinates relative to `origin`, and charge
     const float4* lo;        // second parts
     const float4* rest;      // third parts of the coordinates
-    const double4* x64;      // FP64 coordinates
+    const double4* x64;      // FP64 coordinates, charge
     const GridClass* classes;
     int n_classes, n_slots;  // n_slots: classes with sums
     int3 npts;
@@ -114,10 +115,11 @@ __device__ __forceinline__ void store_record(const GridArgs& a, int slot, int p,
 }
 
 struct PointSums {
-    F3 e;              // Coulomb energy
-    F2 x, y, z;        // and gradient
-    F2 m6, m12;        // LJ sums of the current class
-    double m6d, m12d;  // its atoms within 2 A
+    F3 e;                   // Coulomb energy
+    F2 x, y, z;             // and gradient
+    double E, GX, GY, GZ;   // of the tiles before
+    F2 m6, m12;             // LJ sums of the current class
+    double m6d, m12d;       // its FP64 atoms
 };
 
 __device__ __forceinline__ double to_double(F2 a) { return static_cast<double>(a.h) + static_cast<double>(a.l); }
@@ -152,6 +154,18 @@ __device__ __forceinline__ F3 coord_diff(float ah, float al, float am, F3 p) {
     return {s, __fsub_rn(l, __fsub_rn(s, h)), m};
 }
 
+// The vector from the point to the atom, its squared length in w.
+__device__ __forceinline__ double4 vector64(double4 x, double3 p) {
+    const double vx = x.x - p.x, vy = x.y - p.y, vz = x.z - p.z;
+    return make_double4(vx, vy, vz, fmax(vx * vx + vy * vy + vz * vz, static_cast<double>(kR2Floor)));
+}
+
+__device__ __forceinline__ void add_powers64(double r2, PointSums& s) {
+    const double inv = 1.0 / r2, n6 = inv * inv * inv;
+    s.m6d += n6;
+    s.m12d += n6 * n6;
+}
+
 // Adds one receptor atom to the sums of the point (px, py, pz; FP64 p64).
 template <bool kLj, bool kWide>
 __device__ __forceinline__ void grid_pair(const float4 ah, const float4 al, const float4 am, const double4* x64, F3 px,
@@ -159,17 +173,20 @@ __device__ __forceinline__ void grid_pair(const float4 ah, const float4 al, cons
     const F3 dx = coord_diff<kWide>(ah.x, al.x, am.x, px), dy = coord_diff<kWide>(ah.y, al.y, am.y, py),
              dz = coord_diff<kWide>(ah.z, al.z, am.z, pz);
     F3 r2 = triple_norm2(dx, dy, dz);
+    if (kWide && !(r2.h < kFarR2)) {  // also a coordinate that is not finite
+        const double4 x = *x64, v = vector64(x, p64);
+        const double rinv = rsqrt(v.w), qr = x.w * rinv, w = qr * rinv * rinv;
+        s.E += qr;
+        s.GX = fma(v.x, w, s.GX);
+        s.GY = fma(v.y, w, s.GY);
+        s.GZ = fma(v.z, w, s.GZ);
+        if (kLj) add_powers64(v.w, s);
+        return;
+    }
     const bool near = r2.h < kNearR2;
     if (near) {
         if (r2.h < kR2Floor) r2 = {kR2Floor, 0.f, 0.f};
-        if (kLj) {
-            const double4 x = *x64;
-            const double ux = x.x - p64.x, uy = x.y - p64.y, uz = x.z - p64.z;
-            const double inv = 1.0 / fmax(ux * ux + uy * uy + uz * uz, static_cast<double>(kR2Floor));
-            const double n6 = inv * inv * inv;
-            s.m6d += n6;
-            s.m12d += n6 * n6;
-        }
+        if (kLj) add_powers64(vector64(*x64, p64).w, s);
     }
     F3 rinv;
     F2 inv;
@@ -209,7 +226,6 @@ __global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_
     const F3 py = coord_parts<kWide>(p64.y - a.origin.y, a.step, a.step_inv);
     const F3 pz = coord_parts<kWide>(p64.z - a.origin.z, a.step, a.step_inv);
     PointSums s{};
-    double E = 0.0, GX = 0.0, GY = 0.0, GZ = 0.0;
     for (int c = 0; c < a.n_classes; ++c) {
         const GridClass gc = a.classes[c];
         for (int t0 = 0; t0 < gc.count; t0 += kMomentTile) {
@@ -227,13 +243,13 @@ __global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_
                     grid_pair<true, kWide>(s_hi[u], s_lo[u], s_rest[u], a.x64 + base + u, px, py, pz, p64, s);
             } else {
                 for (int u = 0; u < n; ++u)
-                    grid_pair<false, kWide>(s_hi[u], s_lo[u], s_rest[u], nullptr, px, py, pz, p64, s);
+                    grid_pair<false, kWide>(s_hi[u], s_lo[u], s_rest[u], a.x64 + base + u, px, py, pz, p64, s);
             }
             // the low part of a long sum would round by more than its terms do
-            E += to_double(s.e);
-            GX += to_double(s.x);
-            GY += to_double(s.y);
-            GZ += to_double(s.z);
+            s.E += to_double(s.e);
+            s.GX += to_double(s.x);
+            s.GY += to_double(s.y);
+            s.GZ += to_double(s.z);
             s.e = {0.f, 0.f, 0.f};
             s.x = s.y = s.z = {0.f, 0.f};
         }
@@ -248,8 +264,8 @@ __global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_
         }
     }
     if (t < a.n_points) {
-        store_record(a, 0, p, E * kCoulombD, clampf_rec(GX * kCoulombD), clampf_rec(GY * kCoulombD),
-                     clampf_rec(GZ * kCoulombD));
+        store_record(a, 0, p, s.E * kCoulombD, clampf_rec(s.GX * kCoulombD), clampf_rec(s.GY * kCoulombD),
+                     clampf_rec(s.GZ * kCoulombD));
     }
 }
 
@@ -375,13 +391,16 @@ int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
         (&a.origin.x)[d] = ctx->box.init_xyz[d] + half[d];
         reach = std::max(reach, half[d]);
     }
+    bool wide = !(reach < kGridReach);
     for (const auto& [kind, atoms] : by_kind)
         for (int i : atoms)
             for (int d = 0; d < 3; ++d) {
                 const double r = std::fabs(ctx->rec_xyz[3 * i + d] - (&a.origin.x)[d]) + half[d];
-                if (std::isfinite(r)) reach = std::max(reach, r);
+                if (r < kGridReach)
+                    reach = std::max(reach, r);
+                else  // also where r is not a number
+                    wide = true;
             }
-    const bool wide = reach >= kGridReach;
     a.step = std::ldexp(1.0, std::ilogb(std::max(reach, 1.0)) + 1 - 24);
     a.step_inv = 1.0 / a.step;
     std::vector<float4> hi, lo, rest;
@@ -405,7 +424,8 @@ int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
             hi.push_back(make_float4(x[0].h, x[1].h, x[2].h, q));
             lo.push_back(make_float4(x[0].l, x[1].l, x[2].l, static_cast<float>(ctx->rec_charge[i] - q)));
             rest.push_back(make_float4(x[0].m, x[1].m, x[2].m, 0.f));
-            x64.push_back(make_double4(ctx->rec_xyz[3 * i], ctx->rec_xyz[3 * i + 1], ctx->rec_xyz[3 * i + 2], 0.0));
+            x64.push_back(make_double4(ctx->rec_xyz[3 * i], ctx->rec_xyz[3 * i + 1], ctx->rec_xyz[3 * i + 2],
+                                       ctx->rec_charge[i]));
         }
     }
     a.n_classes = static_cast<int>(classes.size());

@@ -45,3 +45,25 @@ def test_coulomb_energies(far):
     # the gradient: FP32 roundings of sums in pairs
     g = (q[..., None] * d / (r * r)[..., None]).sum(1)
     np.testing.assert_allclose(got[at, 1:], g.astype(np.float64), rtol=2.0 ** -23, atol=1e-9)
+
+
+@pytest.mark.parametrize("where", [1e16, 1e22])
+def test_atom_out_of_fp32(where):
+    """An atom so far that FP32 does not hold its squared distance adds next to nothing: the maps
+    are those of the receptor with its charge and well depth at zero (q / r <= 2e-14 kcal/mol)."""
+    native.load(auto_build=True)
+    js = synth.make_receptor(seed=5, n_heavy=120, cube=14.0, cavity=3.0)
+    js["xyz"][0] = [where, -0.5 * where, 0.25 * where]
+    box = model.make_box((0.0, 0.0, 0.0), (5.0, 4.0, 3.0), 0.375)
+    maps = []
+    for off in (False, True):
+        rec = model.Receptor.from_json(js)
+        if off:
+            rec.ff.charge[0] = rec.ff.epsilon[0] = 0.0
+        with native.Context(0) as ctx:
+            ctx.set_receptor(rec)
+            ctx.build_grid(box, [3, 7])
+            maps.append([ctx.read_map(m) for m in (abi.COULOMB_MAP, 3, 7)])
+    for got, want in zip(*maps):
+        assert np.isfinite(want).all()
+        np.testing.assert_allclose(got, want, rtol=2.0 ** -23, atol=1e-12)

@@ -373,9 +373,10 @@ static void launch_lj(const GridArgs& a, int blocks, cudaStream_t s) {
 // Builds the Coulomb map (slot 0) and the maps of `types` (slots 1..) over the context's
 // box from every non-rotor receptor atom (grid.cpp:119-123, 173). Synchronous.
 int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
-    std::map<std::pair<double, double>, std::vector<int>> by_kind;  // (epsilon, sigma) -> atoms
+    // (epsilon, sigma) -> atoms, by the numbers' bits: a NaN has no place among numbers
+    std::map<std::pair<int64_t, int64_t>, std::vector<int>> by_kind;
     for (int i = 0; i < ctx->n_rec; ++i)
-        if (!ctx->is_mov[i]) by_kind[{ctx->rec_epsilon[i], ctx->rec_sigma[i]}].push_back(i);
+        if (!ctx->is_mov[i]) by_kind[{number_bits(ctx->rec_epsilon[i]), number_bits(ctx->rec_sigma[i])}].push_back(i);
     GridArgs a{};
     a.npts = make_int3(ctx->box.npoints[0], ctx->box.npoints[1], ctx->box.npoints[2]);
     a.init = make_double3(ctx->box.init_xyz[0], ctx->box.init_xyz[1], ctx->box.init_xyz[2]);
@@ -392,7 +393,7 @@ int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
         reach = std::max(reach, half[d]);
     }
     bool wide = !(reach < kGridReach);
-    for (const auto& [kind, atoms] : by_kind)
+    for (const auto& [bits, atoms] : by_kind)
         for (int i : atoms)
             for (int d = 0; d < 3; ++d) {
                 const double r = std::fabs(ctx->rec_xyz[3 * i + d] - (&a.origin.x)[d]) + half[d];
@@ -408,7 +409,8 @@ int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
     std::vector<GridClass> classes;
     std::vector<int> order;  // receptor atoms in class order
     std::vector<std::pair<double, double>> kinds;  // of the classes with sums
-    for (const auto& [kind, atoms] : by_kind) {
+    for (const auto& [bits, atoms] : by_kind) {
+        const std::pair<double, double> kind(ctx->rec_epsilon[atoms[0]], ctx->rec_sigma[atoms[0]]);
         const bool lj = kind.first != 0.0;
         classes.push_back({static_cast<int>(hi.size()), static_cast<int>(atoms.size()),
                            lj ? static_cast<int>(kinds.size()) : -1});

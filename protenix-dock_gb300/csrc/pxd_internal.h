@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cstring>
 #include <map>
 #include <string>
 #include <utility>
@@ -301,6 +302,13 @@ cudaError_t launch_with_map_window(const pxd_context* ctx, void (*kern)(KArgs...
     cfg.attrs = on ? &attr : nullptr;
     cfg.numAttrs = on ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
+// A number's bits, as a key: equal numbers of one bit pattern, and every NaN apart from numbers.
+inline int64_t number_bits(double v) {
+    int64_t b;
+    std::memcpy(&b, &v, sizeof(b));
+    return b;
 }
 
 // kernels (launchers), one per translation unit

@@ -155,10 +155,11 @@ int upload_receptor_scoring(pxd_context* ctx, const pxd_score_lists* l, const st
     std::vector<float2> cls;
     std::vector<int2> lc(M);
     {
-        std::map<std::pair<float, float>, int> seen;
+        std::map<std::pair<int64_t, int64_t>, int> seen;
         for (int a = 0; a < M; ++a) {
             const float2 se = make_float2(static_cast<float>(ctx->rec_sigma[a]), static_cast<float>(ctx->rec_epsilon[a]));
-            const auto it = seen.emplace(std::make_pair(se.x, se.y), static_cast<int>(cls.size())).first;
+            const auto it =
+                seen.emplace(std::make_pair(number_bits(se.x), number_bits(se.y)), static_cast<int>(cls.size())).first;
             if (it->second == static_cast<int>(cls.size())) cls.push_back(se);
             lc[a] = make_int2(ctx->is_mov[a] ? local_of[a] : -1, it->second);
         }

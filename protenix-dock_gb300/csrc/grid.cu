@@ -17,7 +17,7 @@
 //   - the Coulomb energy is formed and summed in triples: its q/r terms of both signs cancel to
 //     a small part of their size, and 1,900 terms of ~7 kcal/mol a unit charge in pairs left
 //     1e-12 kcal/mol. The triple sum, and the pair sums of the gradient, are folded into FP64
-//     every kMomentTile atoms;
+//     every kMomentTile atoms or so;
 //   - r^-6 and r^-12 are pairs; of atoms closer than 2 A they are formed and summed in FP64 from
 //     the FP64 coordinates (the 12th power of a clash amplifies the coordinates' rounding most);
 //   - the classes' energies are combined in FP64, and kept as the FP32 record and the FP32
@@ -59,7 +59,10 @@ constexpr double kGridReach = 256.0;
 constexpr double kRecordCeil = 1e30;
 constexpr double kCoulombD = 332.0637141491396;  // kCoulombFactor, system.h:83
 constexpr size_t kMomentBytes = 2 * sizeof(double);  // per point and class
-constexpr size_t kMomentLimit = size_t(96) << 20;  // workspace of the sums; larger boxes run in chunks
+// Workspace of the sums; larger boxes run in chunks of points. A chunk is at least four blocks per
+// SM: a receptor whose atoms all have parameters of their own (1,866 classes) would get 26
+// blocks in 96 MB, and 160 launches for 81^3 points.
+constexpr size_t kMomentLimit = size_t(96) << 20, kMomentMost = size_t(2) << 30;
 
 struct GridClass {
     int first, count;  // atoms [first, first + count) of the class-ordered list
@@ -114,18 +117,27 @@ __device__ __forceinline__ void store_record(const GridArgs& a, int slot, int p,
         fabs(E) < kRecordCeil ? static_cast<float>(E - static_cast<double>(hi)) : 0.f;
 }
 
-struct PointSums {
-    F3 e;                   // Coulomb energy
-    F2 x, y, z;             // and gradient
-    double E, GX, GY, GZ;   // of the tiles before
-    F2 m6, m12;             // LJ sums of the current class
-    double m6d, m12d;       // its FP64 atoms
-};
-
 __device__ __forceinline__ double to_double(F2 a) { return static_cast<double>(a.h) + static_cast<double>(a.l); }
 __device__ __forceinline__ double to_double(F3 a) {
     return static_cast<double>(a.h) + (static_cast<double>(a.l) + static_cast<double>(a.m));
 }
+
+struct PointSums {
+    F3 e;                   // Coulomb energy
+    F2 x, y, z;             // and gradient
+    double E, GX, GY, GZ;   // folded before
+    F2 m6, m12;             // LJ sums of the current class
+    double m6d, m12d;       // its FP64 atoms
+
+    __device__ __forceinline__ void fold() {
+        E += to_double(e);
+        GX += to_double(x);
+        GY += to_double(y);
+        GZ += to_double(z);
+        e = {0.f, 0.f, 0.f};
+        x = y = z = {0.f, 0.f};
+    }
+};
 
 // One coordinate of an atom or a point as three parts. The first two on the grids of `step` and
 // 2^-24 step, so that the differences of two of them are exact; kWide: each the rounding of
@@ -226,6 +238,7 @@ __global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_
     const F3 py = coord_parts<kWide>(p64.y - a.origin.y, a.step, a.step_inv);
     const F3 pz = coord_parts<kWide>(p64.z - a.origin.z, a.step, a.step_inv);
     PointSums s{};
+    int since = 0;  // atoms since the last fold
     for (int c = 0; c < a.n_classes; ++c) {
         const GridClass gc = a.classes[c];
         for (int t0 = 0; t0 < gc.count; t0 += kMomentTile) {
@@ -246,12 +259,11 @@ __global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_
                     grid_pair<false, kWide>(s_hi[u], s_lo[u], s_rest[u], a.x64 + base + u, px, py, pz, p64, s);
             }
             // the low part of a long sum would round by more than its terms do
-            s.E += to_double(s.e);
-            s.GX += to_double(s.x);
-            s.GY += to_double(s.y);
-            s.GZ += to_double(s.z);
-            s.e = {0.f, 0.f, 0.f};
-            s.x = s.y = s.z = {0.f, 0.f};
+            since += n;
+            if (since >= kMomentTile) {
+                s.fold();
+                since = 0;
+            }
         }
         if (gc.slot >= 0) {
             if (t < a.n_points) {
@@ -263,6 +275,7 @@ __global__ void __launch_bounds__(kGridThreads) grid_moment_kernel(const __grid_
             s.m6d = s.m12d = 0.0;
         }
     }
+    s.fold();
     if (t < a.n_points) {
         store_record(a, 0, p, s.E * kCoulombD, clampf_rec(s.GX * kCoulombD), clampf_rec(s.GY * kCoulombD),
                      clampf_rec(s.GZ * kCoulombD));
@@ -466,8 +479,9 @@ int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
     a.lj.n_tiles = static_cast<int>(tiles.size());
     // one allocation: inputs, then the sums of a chunk of points
     const size_t n_slots = std::max(1, a.n_slots);
-    const size_t fit = kMomentLimit / (kMomentBytes * n_slots) / kGridThreads * kGridThreads;
-    const int chunk = static_cast<int>(std::min<size_t>(a.P, std::max<size_t>(fit, kGridThreads)));
+    const size_t per_point = kMomentBytes * n_slots, fill = size_t(4) * ctx->n_sm * kGridThreads;
+    const size_t fit = std::max(kMomentLimit / per_point, std::min(fill, kMomentMost / per_point));
+    size_t chunk = std::min<size_t>(a.P, std::max<size_t>(fit / kGridThreads, 1) * kGridThreads);
     std::vector<unsigned char> in;
     auto put = [&in](const auto& v) {
         const size_t off = in.size(), bytes = v.size() * sizeof(v[0]);
@@ -479,8 +493,13 @@ int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
     const size_t o_lh = put(lj_hi), o_ll = put(lj_lo), o_tile = put(tiles), o_kind = put(kind_se), o_type = put(type_se);
     cudaStream_t s = ctx->stream;
     char* mem = nullptr;
-    int rc = cuda_check(ctx, cudaMallocAsync(reinterpret_cast<void**>(&mem), in.size() + kMomentBytes * n_slots * chunk, s),
+    int rc;
+    for (;; chunk = (chunk / 2 + kGridThreads - 1) / kGridThreads * kGridThreads) {  // smaller where memory is short
+        rc = cuda_check(ctx, cudaMallocAsync(reinterpret_cast<void**>(&mem), in.size() + per_point * chunk, s),
                         "map build workspace");
+        if (rc != PXD_ERR_NOMEM || chunk <= kGridThreads) break;
+        cudaGetLastError();
+    }
     if (rc) return rc;
     queue_copy(ctx, &rc, mem, in.data(), in.size(), cudaMemcpyHostToDevice, s, "map build inputs");
     a.hi = reinterpret_cast<const float4*>(mem + o_hi);
@@ -496,9 +515,9 @@ int launch_grid_build(pxd_context* ctx, const std::vector<int>& types) {
     a.lj.types = reinterpret_cast<const float2*>(mem + o_type);
     a.m6 = reinterpret_cast<double*>(mem + in.size());
     a.m12 = a.m6 + n_slots * chunk;
-    for (int p0 = 0; p0 < a.P && !rc; p0 += chunk) {
+    for (int p0 = 0; p0 < a.P && !rc; p0 += static_cast<int>(chunk)) {
         a.p0 = p0;
-        a.n_points = std::min(chunk, a.P - p0);
+        a.n_points = std::min(static_cast<int>(chunk), a.P - p0);
         const int blocks = (a.n_points + kGridThreads - 1) / kGridThreads;
         if (wide)
             grid_moment_kernel<true><<<blocks, kGridThreads, 0, s>>>(a);

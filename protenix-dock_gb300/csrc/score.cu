@@ -461,7 +461,8 @@ constexpr double kGbOffset = 0.09;
 constexpr int kGbTile = 64;
 constexpr int kGbThreads = 128;
 constexpr int kGbLanes = 8;       // lanes that share a receptor atom's sum over the ligand
-constexpr int kGbPoses = 512;     // poses per batch of launches (bounds the workspace)
+constexpr int kGbPoses = 512;     // poses per batch of launches
+constexpr size_t kGbBytes = size_t(64) << 20;  // workspace of a batch, or one pose's if that is more
 
 struct GbArgs {
     int n_lig, n_rec, n_poses, n_conf;  // n_conf: receptor conformations, 1 or n_poses
@@ -707,6 +708,16 @@ static std::vector<double> receptor_coords(pxd_context* ctx, const double* t) {
     return x;
 }
 
+// Poses per batch of gbsa_batch: a pose's tile sums grow with the square of its atoms (1.2 MB at
+// 20,000), and with rotors each has a receptor of its own.
+static int gb_batch_poses(const pxd_context* ctx, const LigandEntry& e) {
+    const size_t nr = ctx->n_rec, nl = e.n_atoms, nb = (nl + nr + kGbTile - 1) / kGbTile;
+    const bool own = ctx->rec.n_rotors > 0;
+    const size_t pose = sizeof(double) * ((own ? 3 : 2) * (nb * (nb + 1) / 2) + nr + 2 * nl + (own ? 2 * nr : 0)) +
+                        sizeof(double4) * (nl + (own ? nr : 0));
+    return static_cast<int>(std::min<size_t>(std::max<size_t>(kGbBytes / pose, 1), kGbPoses));
+}
+
 // GB/SA energies of n poses of one ligand (lig_xyz [n][N][3], rec_tors [n][R]):
 // complex, ligand and receptor energies of pose k in parts[3 k .. 3 k + 2].
 static int gbsa_batch(pxd_context* ctx, const LigandEntry& e, int n, const double* lig_xyz, const double* rec_tors,
@@ -931,11 +942,16 @@ int pxd_score(pxd_context* ctx, int32_t which, int32_t lig, int32_t n_poses, con
     const double gcoef = ctx->sf_host[which].coef[PXD_TERM_GBSA];
     if (gcoef > 1e-5 || gcoef < -1e-5) {
         if (R > 0 && !tors) return set_error(ctx, PXD_ERR_INVALID, "receptor torsions required");
-        std::vector<double> parts(3 * static_cast<size_t>(std::min(n_poses, kGbPoses)));
-        for (int p0 = 0; p0 < n_poses; p0 += kGbPoses) {
-            const int n = std::min(kGbPoses, n_poses - p0);
-            rc = gbsa_batch(ctx, ctx->ligands[lig], n, xyz + 3 * static_cast<size_t>(N) * p0,
-                            R > 0 ? tors + static_cast<size_t>(R) * p0 : nullptr, parts.data());
+        int batch = std::min(n_poses, gb_batch_poses(ctx, ctx->ligands[lig]));
+        std::vector<double> parts(3 * static_cast<size_t>(batch));
+        for (int p0 = 0, n; p0 < n_poses; p0 += n) {
+            for (;; batch = n / 2) {  // smaller where the device is short of memory
+                n = std::min(batch, n_poses - p0);
+                rc = gbsa_batch(ctx, ctx->ligands[lig], n, xyz + 3 * static_cast<size_t>(N) * p0,
+                                R > 0 ? tors + static_cast<size_t>(R) * p0 : nullptr, parts.data());
+                if (rc != PXD_ERR_NOMEM || n <= 1) break;
+                cudaGetLastError();
+            }
             if (rc) return rc;
             for (int p = 0; p < n; ++p) {
                 const double g = parts[3 * p] - parts[3 * p + 1] - parts[3 * p + 2];

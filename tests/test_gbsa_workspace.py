@@ -21,6 +21,7 @@ def test_batches(tmp_path, heavy, rotors, poses):
         ctx.set_receptor(rec)
         lid = ctx.add_ligand(lig)
         xyz, tors = np.repeat(lig.poses[:1], poses, axis=0), np.zeros((poses, rec.n_rotors))
+        ctx.score(1, lid, xyz[:1], tors[:1])  # the ligand table, once
         fake.reset()
         ctx.score(1, lid, xyz, tors)
         last = fake.lib.fake_mallocs() - 1  # the last batch's workspace

@@ -93,72 +93,82 @@ __device__ __forceinline__ float signed_dihedral(float3 pi, float3 pj, float3 pk
     return dot3(rij, n) < 0.f ? phi : -phi;
 }
 
-// This warp's share (w of nw) of the terms of the pose in X (ligand, smem) with receptor
-// rotor atoms in loc_xyz (smem), added up per lane into acc. The warps split the Coulomb / LJ
-// pairs by receptor atom and the hydrophobic contacts by ligand atom, whose partial sums are
-// compensated; the other terms are FP32 sums of one warp each. The terms read the receptor
-// lists by value, one record per atom: through index lists a contact was a chain of four
-// loads, and a pose of 55 atoms in a pocket of 1,866 took one warp 460,000 cycles.
-static __device__ __forceinline__ void score_terms(const ScoreEnv& env, const DevLigand& L, const DevLigScore& ls,
-                                                   const float4* X, const float4* loc_xyz, int lane, int w, int nw,
-                                                   DS* acc) {
+// The Coulomb and LJ pairs and the hydrophobic contacts of the pose in X (ligand, smem) with
+// receptor rotor atoms in loc_xyz (smem) are split into parts, the pairs by receptor atom, the
+// contacts by ligand atom; a part's sums are compensated, per lane. The other terms are FP32
+// sums of one warp each. The terms read the receptor lists by value, one record per atom:
+// through index lists a contact was a chain of four loads, and a pose of 55 atoms in a pocket
+// of 1,866 took one warp 460,000 cycles.
+
+// Part `part` of `parts` of the Coulomb and clamped LJ terms over every ligand x receptor pair
+// (scorer.cpp:222-276). Each lane takes receptor atoms and walks the ligand atoms (shared
+// memory and L1-resident records, read by every lane at once): a receptor atom's records are
+// loaded once per call instead of once per ligand atom. Mean sigma and 4 sqrt(eps eps) of a
+// (type, class) come from a table; their square root per pair was a quarter of the loop.
+static __device__ __forceinline__ void score_pairs(const ScoreEnv& env, const DevLigand& L, const float4* X,
+                                                   const float4* loc_xyz, int lane, int part, int parts, DS& coul,
+                                                   DS& vdw) {
     const DevRecScore& rs = env.rs;
     const DevSf& sf = *env.sf;
+    if (sf.coef[PXD_TERM_COULOMB] == 0.f && sf.coef[PXD_TERM_VDW] == 0.f) return;
     const int N = L.n_atoms;
-    const bool own_hb = w == nw - 1, own_ion = w == max(nw - 2, 0);
-    const int hyd_warps = nw > 2 ? nw - 2 : nw;  // the warps that share the hydrophobic contacts
-#pragma unroll
-    for (int k = 0; k < PXD_NUM_TERMS - 1; ++k) acc[k] = DS{0.f, 0.f};
-    const bool coul = sf.coef[PXD_TERM_COULOMB] != 0.f, vdw = sf.coef[PXD_TERM_VDW] != 0.f;
-    // Coulomb and clamped LJ over every ligand x receptor pair (scorer.cpp:222-276). Each
-    // lane takes receptor atoms and walks the ligand atoms (shared memory and L1-resident
-    // records, read by every lane at once): a receptor atom's records are loaded once per
-    // call instead of once per ligand atom. Mean sigma and 4 sqrt(eps eps) of a (type, class)
-    // come from a table; their square root per pair was a quarter of the loop.
-    if (coul || vdw) {
-        const float cutoff = sf.vdw_cutoff;
-        const float* const charge = L.charge;
-        const int* const type = L.type;
-        for (int j = lane + w * kWarp; j < rs.n_all; j += nw * kWarp) {
-            const float4 rj = __ldg(&rs.all_xyzq[j]);
-            const int2 lc = __ldg(&rs.all_lc[j]);
-            const float3 xj = lc.x >= 0 ? xyz(loc_xyz[lc.x]) : xyz(rj);
-            const float2* const row = env.vdw + lc.y;
-            float ec = 0.f, ev = 0.f;
+    const float cutoff = sf.vdw_cutoff;
+    const float* const charge = L.charge;
+    const int* const type = L.type;
+    for (int j = lane + part * kWarp; j < rs.n_all; j += parts * kWarp) {
+        const float4 rj = __ldg(&rs.all_xyzq[j]);
+        const int2 lc = __ldg(&rs.all_lc[j]);
+        const float3 xj = lc.x >= 0 ? xyz(loc_xyz[lc.x]) : xyz(rj);
+        const float2* const row = env.vdw + lc.y;
+        float ec = 0.f, ev = 0.f;
 #pragma unroll 4
-            for (int i = 0; i < N; ++i) {
-                const float3 xi = xyz(X[i]);
-                const float qi = __ldg(&charge[i]);
-                const float2 sc = __ldg(&row[__ldg(&type[i]) * rs.n_cls]);
-                const float d = dist3(xi, xj);
-                const float rinv = 1.f / (d + kEpsF);
-                ec = fmaf(qi * rj.w, rinv, ec);
-                const float s = sc.x * rinv;
-                const float s2 = s * s;
-                const float u6 = s2 * s2 * s2;
-                const float v = (u6 * u6 - u6) * sc.y;
-                ev += fminf(fmaxf(v, -cutoff), cutoff);
-            }
-            ds_add(acc[PXD_TERM_COULOMB], ec * kCoulombF);
-            ds_add(acc[PXD_TERM_VDW], ev);
-        }
-    }
-    // hydrophobic contacts (scorer.cpp:278-311)
-    if (sf.coef[PXD_TERM_HYDROPHOBIC] != 0.f && w < hyd_warps) {
-        const float hydro_factor = sf.hydro_factor, hydro_min = sf.hydro_min, hydro_max = sf.hydro_max;
-        for (int a = w; a < ls.n_hyd; a += hyd_warps) {
-            const int i = __ldg(&ls.hyd[a]);
+        for (int i = 0; i < N; ++i) {
             const float3 xi = xyz(X[i]);
-            const float s1 = sf.vdw_sigma_raw[__ldg(&L.type[i])];
-            float e = 0.f;
-#pragma unroll 4
-            for (int b = lane; b < rs.n_hyd; b += kWarp) {
-                const float r1 = (s1 + __ldg(&rs.hyd_sigma[b])) * hydro_factor + hydro_min;
-                e -= ramp_down(dist3(xi, rec_pos(__ldg(&rs.hyd[b]), loc_xyz)), r1, r1 + hydro_max);
-            }
-            ds_add(acc[PXD_TERM_HYDROPHOBIC], e);
+            const float qi = __ldg(&charge[i]);
+            const float2 sc = __ldg(&row[__ldg(&type[i]) * rs.n_cls]);
+            const float d = dist3(xi, xj);
+            const float rinv = 1.f / (d + kEpsF);
+            ec = fmaf(qi * rj.w, rinv, ec);
+            const float s = sc.x * rinv;
+            const float s2 = s * s;
+            const float u6 = s2 * s2 * s2;
+            const float v = (u6 * u6 - u6) * sc.y;
+            ev += fminf(fmaxf(v, -cutoff), cutoff);
         }
+        ds_add(coul, ec * kCoulombF);
+        ds_add(vdw, ev);
     }
+}
+
+// Part `part` of `parts` of the hydrophobic contacts (scorer.cpp:278-311).
+static __device__ __forceinline__ void score_hydrophobic(const ScoreEnv& env, const DevLigand& L, const DevLigScore& ls,
+                                                         const float4* X, const float4* loc_xyz, int lane, int part,
+                                                         int parts, DS& acc) {
+    const DevRecScore& rs = env.rs;
+    const DevSf& sf = *env.sf;
+    if (sf.coef[PXD_TERM_HYDROPHOBIC] == 0.f) return;
+    const float hydro_factor = sf.hydro_factor, hydro_min = sf.hydro_min, hydro_max = sf.hydro_max;
+    for (int a = part; a < ls.n_hyd; a += parts) {
+        const int i = __ldg(&ls.hyd[a]);
+        const float3 xi = xyz(X[i]);
+        const float s1 = sf.vdw_sigma_raw[__ldg(&L.type[i])];
+        float e = 0.f;
+#pragma unroll 4
+        for (int b = lane; b < rs.n_hyd; b += kWarp) {
+            const float r1 = (s1 + __ldg(&rs.hyd_sigma[b])) * hydro_factor + hydro_min;
+            e -= ramp_down(dist3(xi, rec_pos(__ldg(&rs.hyd[b]), loc_xyz)), r1, r1 + hydro_max);
+        }
+        ds_add(acc, e);
+    }
+}
+
+// The other terms: the ionic, pi-cation and stacking terms (own_ion), hydrogen bonds and torsion
+// strain (own_hb), added to acc.
+static __device__ __forceinline__ void score_few(const ScoreEnv& env, const DevLigand& L, const DevLigScore& ls,
+                                                 const float4* X, const float4* loc_xyz, int lane, bool own_ion,
+                                                 bool own_hb, DS* acc) {
+    const DevRecScore& rs = env.rs;
+    const DevSf& sf = *env.sf;
     // ionic (scorer.cpp:313-368): ligand cations x receptor anions, receptor cations x ligand anions
     if (own_ion && sf.coef[PXD_TERM_IONIC] != 0.f) {
         float e = 0.f;
@@ -293,7 +303,13 @@ static __device__ __forceinline__ double score_total(const DevSf& sf, const DevL
 static __device__ __noinline__ double score_pose(const ScoreEnv& env, const DevLigand& L, const float4* X,
                                                  const float4* loc_xyz, int lane, int tw, int tn, TeamShared* ts) {
     DS acc[PXD_NUM_TERMS - 1];
-    score_terms(env, L, L.score, X, loc_xyz, lane, tw, tn, acc);
+#pragma unroll
+    for (int k = 0; k < PXD_NUM_TERMS - 1; ++k) acc[k] = DS{0.f, 0.f};
+    score_pairs(env, L, X, loc_xyz, lane, tw, tn, acc[PXD_TERM_COULOMB], acc[PXD_TERM_VDW]);
+    const int hyd_warps = tn > 2 ? tn - 2 : tn;
+    if (tw < hyd_warps)
+        score_hydrophobic(env, L, L.score, X, loc_xyz, lane, tw, hyd_warps, acc[PXD_TERM_HYDROPHOBIC]);
+    score_few(env, L, L.score, X, loc_xyz, lane, tw == max(tn - 2, 0), tw == tn - 1, acc);
     double vals[PXD_NUM_TERMS];
     if (tn > 1) {
 #pragma unroll

@@ -1,5 +1,5 @@
-// Empirical scores on the GPU: the pose-selection / affinity score kernel (one warp per
-// pose) and the FP64 generalised-Born / surface-area term, with their C ABI.
+// Empirical scores on the GPU: the pose-selection / affinity score kernel (a block per pose)
+// and the FP64 generalised-Born / surface-area term, with their C ABI.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -391,10 +391,15 @@ struct EsArgs {
     double* terms;
 };
 
-// One block per pose, its warps sharing the terms (score_terms).
+// One block per pose, its warps sharing the terms. The parts that a term is split into, and the
+// order that they are added in, are the same for any number of warps (4 to 16), so a pose's
+// score does not depend on its batch, bit for bit.
+constexpr int kHydParts = kMaxScoreWarps - 2;
+
 __global__ void __launch_bounds__(kMaxScoreWarps * kWarp) empirical_score_kernel(const __grid_constant__ EsArgs a) {
     extern __shared__ __align__(16) float smem[];
-    __shared__ float2 s_part[kMaxScoreWarps][PXD_NUM_TERMS - 1];
+    __shared__ float2 s_part[3][kMaxScoreWarps][kWarp];  // Coulomb, LJ, hydrophobic
+    __shared__ float2 s_term[PXD_NUM_TERMS - 1];
     const int lane = threadIdx.x & (kWarp - 1);
     const int w = threadIdx.x / kWarp, nw = blockDim.x / kWarp;
     float4* X = reinterpret_cast<float4*>(smem);
@@ -421,27 +426,52 @@ __global__ void __launch_bounds__(kMaxScoreWarps * kWarp) empirical_score_kernel
             loc[l] = make_float4(p.x, p.y, p.z, 0.f);
         }
         __syncthreads();
-        DS acc[PXD_NUM_TERMS - 1];
-        score_terms(a.env, L, L.score, X, loc, lane, w, nw, acc);
+        for (int v = w; v < kMaxScoreWarps; v += nw) {
+            DS c{0.f, 0.f}, e{0.f, 0.f};
+            score_pairs(a.env, L, X, loc, lane, v, kMaxScoreWarps, c, e);
+            s_part[0][v][lane] = make_float2(c.hi, c.lo);
+            s_part[1][v][lane] = make_float2(e.hi, e.lo);
+        }
+        if (w < nw - 2) {
+            for (int v = w; v < kHydParts; v += nw - 2) {
+                DS h{0.f, 0.f};
+                score_hydrophobic(a.env, L, L.score, X, loc, lane, v, kHydParts, h);
+                s_part[2][v][lane] = make_float2(h.hi, h.lo);
+            }
+        } else {
+            DS acc[PXD_NUM_TERMS - 1];
 #pragma unroll
-        for (int k = 0; k < PXD_NUM_TERMS - 1; ++k) {
-            const DS r = ds_warp_reduce(acc[k]);
-            if (lane == 0) s_part[w][k] = make_float2(r.hi, r.lo);
+            for (int k = 0; k < PXD_NUM_TERMS - 1; ++k) acc[k] = DS{0.f, 0.f};
+            const bool ion = w == nw - 2;
+            score_few(a.env, L, L.score, X, loc, lane, ion, !ion, acc);
+#pragma unroll
+            for (int k = 0; k < PXD_NUM_TERMS - 1; ++k) {
+                if (k == PXD_TERM_COULOMB || k == PXD_TERM_VDW || k == PXD_TERM_HYDROPHOBIC) continue;
+                if ((k == PXD_TERM_HBOND || k == PXD_TERM_TSTRAIN || k == PXD_TERM_ROTATABLE) == ion) continue;
+                const DS r = ds_warp_reduce(acc[k]);
+                if (lane == 0) s_term[k] = make_float2(r.hi, r.lo);
+            }
+        }
+        __syncthreads();
+        if (w < 3) {
+            DS t{s_part[w][0][lane].x, s_part[w][0][lane].y};
+            const int n = w < 2 ? kMaxScoreWarps : kHydParts;
+            for (int v = 1; v < n; ++v) ds_add_ds(t, DS{s_part[w][v][lane].x, s_part[w][v][lane].y});
+            t = ds_warp_reduce(t);
+            const int k = w == 0 ? PXD_TERM_COULOMB : w == 1 ? PXD_TERM_VDW : PXD_TERM_HYDROPHOBIC;
+            if (lane == 0) s_term[k] = make_float2(t.hi, t.lo);
         }
         __syncthreads();
         if (threadIdx.x == 0) {
             double vals[PXD_NUM_TERMS];
 #pragma unroll
-            for (int k = 0; k < PXD_NUM_TERMS - 1; ++k) {
-                DS t{s_part[0][k].x, s_part[0][k].y};
-                for (int u = 1; u < nw; ++u) ds_add_ds(t, DS{s_part[u][k].x, s_part[u][k].y});
-                vals[k] = static_cast<double>(t.hi) + static_cast<double>(t.lo);
-            }
+            for (int k = 0; k < PXD_NUM_TERMS - 1; ++k)
+                vals[k] = static_cast<double>(s_term[k].x) + static_cast<double>(s_term[k].y);
             a.score[pose] = score_total(*a.env.sf, L.score, vals);
             if (a.terms)
                 for (int k = 0; k < PXD_NUM_TERMS; ++k) a.terms[static_cast<size_t>(pose) * PXD_NUM_TERMS + k] = vals[k];
         }
-        // s_part and X are rewritten only after the next pose's first barrier has seen thread 0
+        // s_term, s_part and X are rewritten only after the next pose's first barrier has seen thread 0
         __syncthreads();
     }
 }
@@ -876,11 +906,12 @@ int pxd_score_dev(pxd_context* ctx, int32_t which, int32_t n_poses, int32_t max_
     a.score = score;
     a.terms = terms;
     const size_t smem = sizeof(float4) * (max_atoms + ctx->rec.n_mov + 1);
-    if (smem > 48 * 1024) {
+    if (smem > 32 * 1024) {  // with the kernel's own 12.1 KB, towards the 48 KB of an unasked launch
         rc = raise_smem_limit(ctx, reinterpret_cast<const void*>(empirical_score_kernel), smem, "score smem");
         if (rc) return rc;
     }
-    // enough warps to fill the chip: four per pose once the poses do, up to 16 for a few poses
+    // enough warps to fill the chip: four per pose (the kernel's least) once the poses do, up to 16
+    // for a few poses
     int warps = 4;
     while (warps < kMaxScoreWarps && static_cast<long long>(n_poses) * warps < 16LL * ctx->n_sm) warps *= 2;
     const int blocks = std::min(n_poses, ctx->n_sm * 64);

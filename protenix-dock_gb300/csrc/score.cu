@@ -9,6 +9,7 @@
 
 #include "../../include/pxdock_gb300_vdw.h"
 #include "device_score.cuh"
+#include "gb_exp.cuh"
 
 namespace pxd {
 
@@ -507,6 +508,7 @@ struct GbArgs {
     double* partial;         // [systems][n_tiles]
     int n_tiles;             // of the complex
     double* energy;          // [systems]: n_poses complexes, n_conf receptors, n_poses ligands
+    GbExpTable exp2;
 };
 
 // One pair term of atom j's Born sum (scorer.cpp:806-821).
@@ -616,26 +618,6 @@ __device__ __forceinline__ double gb_prefactor(double f) {
     return 0.5 * kGbCoulomb * (1.0 - exp(-kGbKappa * f) / kGbSolvent);
 }
 
-// exp(y) by Tang's table-driven method (ACM Trans. Math. Softw. 15, 144, 1989): y = n ln2 / 128 + r,
-// exp(y) = 2^(n / 128) (1 + p(r)), |r| <= 0.0028, p to r^5 (the next term is 6e-19). table[k] =
-// 2^(k / 128). Ten FP64 operations, within 1 ulp of exp. Beyond |y| = 690, and for NaN, the
-// library's exp.
-constexpr int kExpTable = 128;
-__device__ __forceinline__ double gb_exp(double y, const double* table) {
-    const int top = __double2hiint(y) & 0x7fffffff;
-    if (top > 0x40859000) return exp(y);
-    const double round = 6755399441055744.0;  // 1.5 * 2^52: the sum's low bits are the nearest integer
-    const double t = fma(y, 184.6649652337873, round);
-    const int n = __double2loint(t);
-    const double nd = t - round;
-    const double r = fma(nd, -1.2655086083325438e-13, fma(nd, -0.005415212347998022, y));
-    const double q = fma(r, fma(r, fma(r, 1.0 / 120.0, 1.0 / 24.0), 1.0 / 6.0), 0.5);
-    const double p = fma(q, r * r, r);
-    const double v = table[n & (kExpTable - 1)];
-    const double e = fma(v, p, v);
-    return __hiloint2double(__double2hiint(e) + ((n >> 7) << 20), __double2loint(e));
-}
-
 // Pair energies of one 64 x 64 tile (rows bi <= columns bj of the triangle i < j). The FP64 pipe
 // bounds it (86 % busy), so the operations per pair are what counts: 66 with the library's exp
 // and a division per pair, 45 with gb_exp, the division as a multiplication and the constant
@@ -657,7 +639,7 @@ __global__ void __launch_bounds__(kGbThreads) gb_pair_kernel(const __grid_consta
         s_ib[u] = -0.25 * ib;
         s_b[u] = 1.0 / ib;
     }
-    for (int k = threadIdx.x; k < kExpTable; k += kGbThreads) s_exp[k] = exp2(k * (1.0 / kExpTable));
+    for (int k = threadIdx.x; k < kExpTable; k += kGbThreads) s_exp[k] = a.exp2.v[k];
     __syncthreads();
     double e = 0.0;
     if (j < y.n) {
@@ -770,6 +752,8 @@ static int gbsa_batch(pxd_context* ctx, const LigandEntry& e, int n, const doubl
     const size_t o_lp = pk.put(gb_properties4(e.gb_radius, e.gb_screen));
     const int nb = (nl + nr + kGbTile - 1) / kGbTile, systems = 2 * n + nc;
     GbArgs a{};
+    static const GbExpTable exp2 = gb_exp_table();
+    a.exp2 = exp2;
     a.n_lig = nl;
     a.n_rec = nr;
     a.n_poses = n;

@@ -421,7 +421,29 @@ void free_receptor(pxd_context* ctx) {
     ctx->has_receptor = false;
 }
 
-// Explicit-pair atom list: (position, charge), (sigma, epsilon), local rotor index.
+// The sorted list `atoms` with no atom twice among kWarp consecutive entries (from multiples of
+// kWarp on): the evaluation adds the gradients of so many receptor atoms at once, one lane
+// each. An atom that rotors list more than once goes to a later run, and -1 fills the runs
+// before.
+std::vector<int> spread_repeats(const std::vector<int>& atoms) {
+    std::vector<std::vector<int>> runs(1);
+    for (int a : atoms) {
+        size_t r = 0;
+        while (runs[r].size() == static_cast<size_t>(kWarp) ||
+               std::find(runs[r].begin(), runs[r].end(), a) != runs[r].end())
+            if (++r == runs.size()) runs.emplace_back();
+        runs[r].push_back(a);
+    }
+    std::vector<int> out;
+    for (const auto& run : runs) {
+        out.resize((out.size() + kWarp - 1) / kWarp * kWarp, -1);
+        out.insert(out.end(), run.begin(), run.end());
+    }
+    return out;
+}
+
+// Explicit-pair atom list: (position, charge), (sigma, epsilon), local rotor index; -1 stands for
+// an atom without charge and well depth, far from everything.
 int upload_explicit(pxd_context* ctx, const std::vector<int>& atoms, const std::vector<int>& local_of,
                     void** mem, size_t* offs) {
     Packer pk;
@@ -431,6 +453,14 @@ int upload_explicit(pxd_context* ctx, const std::vector<int>& atoms, const std::
     std::vector<double4> xq64;
     std::vector<double2> se64;
     for (int a : atoms) {
+        if (a < 0) {
+            xq64.push_back(make_double4(1e18, 0.0, 0.0, 0.0));
+            se64.push_back(make_double2(0.0, 0.0));
+            xq.push_back(make_float4(1e18f, 0.f, 0.f, 0.f));
+            se.push_back(make_float2(0.f, 0.f));
+            loc.push_back(-1);
+            continue;
+        }
         xq64.push_back(make_double4(ctx->rec_xyz[3 * a], ctx->rec_xyz[3 * a + 1], ctx->rec_xyz[3 * a + 2],
                                     ctx->rec_charge[a]));
         se64.push_back(make_double2(ctx->rec_sigma[a], ctx->rec_epsilon[a]));
@@ -754,6 +784,7 @@ int pxd_set_receptor(pxd_context* ctx, const pxd_receptor_desc* r) {
     if (rc) return rc;
     std::vector<int> movs(ctx->mov_atoms.begin(), ctx->mov_atoms.end());
     std::sort(movs.begin(), movs.end());  // grid.cpp:118-123 keeps them in a set
+    movs = spread_repeats(movs);
     rc = upload_explicit(ctx, movs, local_of, &ctx->rec_ex_mov, ctx->ex_mov_off);
     if (rc) return rc;
     ctx->n_ex_all = M;

@@ -71,8 +71,8 @@ __device__ void adj_receptor_rotors(const DevReceptor& R, const float* t, float4
 // Bound by FP32 issue and its latencies: about 100 instructions per pair of a ligand and a
 // receptor atom, at 8 to 16 warps per SM. The table gradient's additions go to global memory,
 // where they return nothing: in shared memory a float addition is a compare-and-swap loop that
-// the warp waits for, and the table's 32 KB took L1 from the receptor. A training step of 4,096
-// poses in 16 pockets: 4.56 -> 3.85 ms, with the loads taken out of the pair loop. A tangent
+// the warp waits for, and the table's 32 KB took L1 from the receptor: with the loads taken out
+// of the pair loop, 0.7 ms of a training step of 4,096 poses in 16 pockets (3.3 ms now). A tangent
 // launch keeps its table in shared memory: its dual numbers bound it, and it measures the same.
 template <bool kGrad, bool kMulti, class S>
 __global__ void __launch_bounds__(kAdjWarps * kWarp, 2) score_adjoint_kernel(const __grid_constant__ AdjArgs a) {
@@ -242,7 +242,7 @@ using namespace pxd;
 extern "C" {
 
 // Two launches in place of the ~150 of the same sums written with one tensor operation per
-// weight: a training step of 4,096 poses 3.87 -> 3.50 ms. 8 poses per block and pass, so that a
+// weight, which took 0.4 ms more of a training step of 4,096 poses. 8 poses per block and pass, so that a
 // few thousand poses fill the chip once; at most 1,024 blocks, 32 partials per run below.
 int pxd_score_weight_grad_dev(pxd_context* ctx, int32_t n_poses, const double* features, const double* grad_out,
                               const double* weights, double* dweights, void* stream) {

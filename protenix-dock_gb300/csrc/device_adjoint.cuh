@@ -291,8 +291,8 @@ __device__ void score_adjoint_pose(const ScoreEnv& env, const DevLigand& L, cons
     const bool table = ap.tab && ls.pclass;  // receptor atoms without a class carry -1
     // Coulomb, clamped LJ and the pair table over every ligand x receptor pair. What the loop
     // reads through pointers is taken out of it: the table gradient's additions to global memory
-    // would have it read again for every pair (4.15 -> 3.85 ms for a training step of 4,096
-    // poses in 16 pockets).
+    // would have it read again for every pair (0.3 ms more of a training step of 4,096 poses in
+    // 16 pockets).
     const float4* const atoms = rs.all_xyzq;
     const float4* const recs = rs.pair_rec;
     const int n_all = rs.n_all;

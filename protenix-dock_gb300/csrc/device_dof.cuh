@@ -211,7 +211,7 @@ __device__ __forceinline__ double closure_eval(DofClosure& c, double t, const fl
     return dof_eval(c, t, d, g, gdot);
 }
 
-// FP64 objective at the pose the variables x place; leaves that pose in c.xc.
+// The reported energy of the pose that the variables x place; leaves that pose in c.xc.
 __device__ __forceinline__ double closure_energy64(DofClosure& c, const float* x) {
     dof_place(c, x);
     return energy64(*c.env, *c.L, c.xc, *c.b, c.lane);

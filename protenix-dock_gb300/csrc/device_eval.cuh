@@ -198,7 +198,7 @@ __device__ __forceinline__ void add_lanes(float4* rec, float3 g, int n, int lane
 // Squared pair distances are floored at 1e-4 A^2 (r = 0.01 A) in the FP32 pair terms: below
 // r ~ 3e-3 A the 12th power overflows FP32 (the FP64 reference stays finite down to 1e-25 A),
 // and the inf energy / NaN gradient would end the optimisation as a NaN. Only such near-
-// coincident atoms see the floor; the reported FP64 energy (energy64.cuh) has none.
+// coincident atoms see the floor; the reported energy (energy64.cuh) has none.
 constexpr float kPairR2Floor = 1e-4f;
 
 // One pre-combined pair (p = A, C, S2) at d = x_j - x_i: energy into `en`, returns the factor of

@@ -84,7 +84,7 @@ __device__ __forceinline__ double closure_eval(Closure& c, double t, const float
     return eval_pose(*c.env, *c.L, c.x0, d, static_cast<float>(t), g, *c.b, c.lane, gdot);
 }
 
-// FP64 objective at the optimiser's variables x (the reported energy).
+// The reported energy (energy64.cuh) at the optimiser's variables x.
 __device__ __forceinline__ double closure_energy64(Closure& c, const float* x) {
     return energy64(*c.env, *c.L, x, *c.b, c.lane);
 }
@@ -270,7 +270,7 @@ static __device__ void strong_wolfe(Cl& c, const LbfgsConsts& p, const float* d,
 // (loss, step, H_diag, the history ring) live with the line search's in the lane-private
 // LsState.
 //
-// energy receives the FP64 objective at the returned pose (energy64), or, with
+// energy receives the reported energy of the returned pose (energy64), or, with
 // final_energy false (a caller that does not use it), the last FP32 loss.
 // The two-loop recursion for (E - 1) * 32 < D <= E * 32, the direction held in registers (E
 // elements per lane, only the last of them tested against D) instead of the shared vectors q
@@ -763,7 +763,7 @@ static __device__ int lbfgs_pose(Cl& c, const LbfgsConsts& p, const Vecs& v, int
             break;
         }
     }
-    // the reported energy: the FP64 objective at the returned pose; an optimisation that
+    // the reported energy, of the returned pose; an optimisation that
     // moved counts it as its final evaluation, as the reference does (optimizer.cpp:552-556)
     if (updated) ++c.nevals;
     energy = final_energy ? closure_energy64(c, v.x) : S.loss;

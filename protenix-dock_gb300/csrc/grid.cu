@@ -25,15 +25,16 @@
 // Against exact sums over the same points, 1,866 atoms, points off the atoms: the Coulomb
 // energies of a unit charge are off by 1.1e-13 kcal/mol in the median and 7e-13 at most, with
 // or without an atom far away (4e-13 and 5e-12 with an FP64 loop over coordinates of two FP32
-// parts); the LJ energies by 3e-15 of themselves in the median, 1e-11 kcal/mol where |E| < 10.
+// parts); the LJ energies by 1e-15 of themselves in the median, and where |E| < 10 by 2e-13 kcal/mol
+// in the median and 2e-11 at most (4e-8 and 2e-7 with FP32 terms under 1e-2 kcal/mol).
 // The LJ gradients are FP32 per pair from hi + lo coordinate differences, folded into FP64
 // every kGridTile atoms. Squared distances are floored at 1e-4 A^2 (a point that sits on an
 // atom cannot overflow FP32) and records clamped to +-1e30 before the FP32 store.
 //
-// Measured, 81^3 points x 1,866 atoms: 12 maps in 15.5 ms (104 ms with FP64 terms per point and
-// map): 9.4 ms for grid_moment_kernel (5.0 with Coulomb terms in pairs) and 3.0 ms for each
+// Measured, 81^3 points x 1,866 atoms: 12 maps in 14.9 ms (104 ms with FP64 terms per point and
+// map): 8.4 ms for grid_moment_kernel (4.4 with Coulomb terms in pairs) and 3.0 ms for each
 // walk of grid_lj_kernel over 6 types, both near the FP32 issue rate; all 99 types over
-// 55 x 49 x 53 points in 17.0 ms (240 ms).
+// 55 x 49 x 53 points in 16.7 ms (239 ms).
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -37,8 +37,8 @@ struct LbfgsArgs {
 };
 
 constexpr int kWarpsPerBlock = 4;
-// Poses/s of 4 blocks of 128 registers against 5 of 96 (65,536 poses of a 43-atom ligand: 180
-// against 187 ms; 16,384 of 60 and 80 atoms: 71 against 77, 109 against 109; 2,000 poses: 12.7
+// 4 blocks of 128 registers against 5 of 96 (ms of 65,536 poses of a 43-atom ligand: 180
+// against 187; 16,384 of 60 and 80 atoms: 71 against 77, 109 against 109; 2,000 poses: 12.7
 // against 13.0; 28,800 poses of 24 ligands of 10 to 47 heavy atoms: 151 against 151) and 3 (187,
 // 75, 113, 12.1, 149): fewer spills, and fewer warps that take each other's instructions out of
 // the cache.
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, kMinBlocks > 0 ? kMinB
             for (int r = lane; r < R; r += kWarp)
                 a.tors_grad[static_cast<size_t>(pose) * R + r] = g[3 * N + r];
         }
-        // the energy is the FP64 objective, the gradient the FP32 one
+        // the energy is the reported one (energy64.cuh), the gradient the FP32 objective's
         if (reported) {
             const double e = energy64(a.env, a.ligands[lid], x, b, lane);
             if (lane == 0) a.energy[pose] = e;
@@ -287,11 +287,16 @@ static size_t lbfgs_block_smem(const pxd_context* ctx, int cap, int history, boo
 }
 
 // The register budget of a score launch. A warp waits for map gathers most of the time, so more
-// of them help, as long as their shared memory leaves L1 for the maps. 65,536 poses of a
-// 43-atom ligand (19 KB per block): 2.39 ms uncapped (4 blocks), 2.22 / 1.89 / 2.33 ms with 6 /
-// 8 / 10 blocks; 32,768 of 65 atoms (27 KB): 1.73, 1.61 / 1.89 with 6 / 8; of 73 atoms (30 KB):
-// 2.55, 2.38 / 3.45. A batch that is resident at once without a cap keeps it: 1,000 poses take
-// 94 us, and 104 with 8 blocks.
+// of them help, as long as their shared memory leaves L1 for the maps. 32,768 poses, ms
+// uncapped (4 blocks) / with 6 / with 8:
+//   31 atoms 0.89 / 0.73 / 0.74, 43: 1.17 / 0.97 / 1.02, 45: 1.29 / 1.04 / 1.05,
+//   53: 1.45 / 1.21 / 1.26, 60: 1.70 / 1.41 / 1.60, 66: 2.00 / 1.67 / 2.13, 78: 2.58 / 2.46 / 2.62;
+// 4,096 poses, which one wave holds with 8 blocks but not with 6:
+//   43 atoms 0.19 / 0.20 / 0.15, 53: 0.23 / 0.24 / 0.19, 66: 0.30 / 0.34 / 0.29, 78: 0.39 / 0.48 / 0.56.
+// So 8 blocks while their shared memory leaves a third of the SM's to L1 (44 atoms without
+// rotors), where large batches are within 5 % of the best, then 6, and no cap from 184 KB on (74
+// atoms). A batch that is resident at once without a cap keeps it: 1,000 poses take 94 us, and
+// 104 with 8 blocks.
 using ScoreKernelFn = void (*)(ScoreArgs);
 static ScoreKernelFn score_variant(const pxd_context* ctx, int n_poses, size_t block_smem) {
     if (n_poses <= 4 * kWarpsPerBlock * ctx->n_sm) return score_kernel<0>;
@@ -396,7 +401,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * kWarp) score_multi_kernel(con
         for (int k = lane; k < 3 * a.max_atoms; k += kWarp) og[k] = k < 3 * N ? g[k] : 0.f;
         for (int r = lane; r < R; r += kWarp)
             a.tors_grad[static_cast<size_t>(pose) * a.tors_stride + r] = g[3 * N + r];
-        // the energy is the FP64 objective, the gradient the FP32 one (as score_kernel)
+        // the energy is the reported one, the gradient the FP32 objective's (as score_kernel)
         const double e = energy64(env, a.tabs[c][lid], x, b, lane);
         if (lane == 0) a.energy[pose] = e;
         __syncwarp();

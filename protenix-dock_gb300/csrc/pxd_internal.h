@@ -121,7 +121,7 @@ struct DevLigand {
     const int* map_slot;      // [N] vdW map slot of the atom's type (-1: no map)
     const float2* se;         // [N] sigma, epsilon (explicit inter pairs)
     const float* charge_lo;   // [N] charge64 - charge
-    const double* charge64;   // [N] FP64 copies for the final FP64 energy
+    const double* charge64;   // [N] FP64 copies for the reported energy
     const double2* se64;      // [N]
     const int* type;          // [N] ligand vdW type
     // torsion tree (forward kinematics, data.cpp:592-641)
@@ -145,7 +145,7 @@ struct DevReceptor {
     const float4* rotor_axis;     // [R] unit
     const int* rotor_mov;         // [R+1] rotor atoms are local [rotor_mov[r], rotor_mov[r+1])
     const float4* local_xyz0;     // [n_local] input coordinates (rotor atoms: x0 - origin)
-    // FP64 copies for the final FP64 energy
+    // FP64 copies for the reported energy
     const double4* ex_xyzq64;
     const double2* ex_se64;
     const double4* rotor_origin64;
